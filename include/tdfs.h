@@ -37,12 +37,19 @@ typedef struct tdfs_graph tdfs_graph; /* device-resident data graph */
 typedef struct tdfs_plan tdfs_plan;   /* compiled pattern plan */
 typedef struct tdfs_csr tdfs_csr;     /* host CSR (generators, file reader) */
 
-/* Launch knobs.  Zero means "choose automatically". */
+/* Launch knobs.  Zero means "choose automatically".  Two kernels count: the
+ * flat kernel, which extends 32 partial embeddings per warp at once, and the
+ * DFS kernel.  The library takes the flat one where the plan has its form;
+ * stealing off, a work budget, or a value for one of the DFS kernel's own
+ * knobs (steal_min, steal_first, merge_window, merge_ratio, fixed_stage,
+ * lane_list, split_rush_us, leaf_steal_min, level_hoist, tail_count,
+ * dead_prune) asks for the DFS kernel.  The counts are the same. */
 typedef struct {
   int warps_per_block;  /* warps per CTA */
   int blocks_per_sm;    /* resident CTAs per SM */
-  int chunk_cap;        /* candidate slots per DFS level (multiple of 32; 0 auto: 128 for patterns
-                           of at most 4 vertices, 512 for 5, 256 for 6 and 7, per launch) */
+  int chunk_cap;        /* candidate slots per level (multiple of 32; 0 auto: DFS kernel 128 for patterns
+                           of at most 4 vertices, 512 for 5, 256 for 6 and 7, per launch; flat kernel
+                           what 32 warps per SM leave room for) */
   int steal;            /* 1: intra-block work stealing + global split queue; 0: off; -1 auto */
   int merge_window;     /* merge-window size in ints (0 auto, -1 = binary search only) */
   int64_t edge_begin;   /* level-0 directed-edge range [edge_begin, edge_end) */
@@ -60,8 +67,9 @@ typedef struct {
   int fixed_stage;      /* last vertex: stage the intersection of its backward neighbours
                            other than the parent once per parent in shared memory
                            (0 auto = on, -1 off) */
-  int split_after_us;   /* a warp's subtree becomes stealable after this many microseconds
-                           on it, donatable to the HBM ring after 4x (0 auto = 150, -1 = at once) */
+  int split_after_us;   /* DFS kernel: a warp's subtree becomes stealable after this many microseconds
+                           on it, donatable to the HBM ring after 4x (0 auto = 150, -1 = at once);
+                           flat kernel: a warp gives work to idle ones after this long (0 auto = 30) */
   int steal_first;      /* an idle warp first takes a level with >= steal_first items from a warp
                            of its CTA, then a unit of the split ring, and only then a level
                            with >= steal_min items (0 auto = 8) */

@@ -25,8 +25,8 @@ CXX = os.environ.get("CXX", "g++")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-O3,-Wall", "--expt-relaxed-constexpr"]
 
-SOURCES = ["error.cpp", "plan.cpp", "csr.cpp", "capi.cpp", "serve.cpp", "graph.cu", "match.cu", "static_count.cu", "estimate.cpp"]
-HEADERS = ["common.h", "plan.h", "csr.h", "graph.h", "match.cuh", "serve.h"]
+SOURCES = ["error.cpp", "plan.cpp", "csr.cpp", "capi.cpp", "serve.cpp", "graph.cu", "match.cu", "flat.cu", "flat_plan.cpp", "static_count.cu", "estimate.cpp"]
+HEADERS = ["common.h", "plan.h", "csr.h", "graph.h", "match.cuh", "flat.cuh", "serve.h"]
 
 
 def _newer(src_paths, out):

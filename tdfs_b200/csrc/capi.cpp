@@ -23,6 +23,8 @@
 struct tdfs_plan {
   tdfs::HostPlan host;
   tdfs::DevPlan dev;
+  tdfs::FlatPlan flat;
+  bool has_flat;
 };
 
 namespace tdfs {
@@ -140,6 +142,49 @@ int launch_shape(const tdfs_graph *g, int kmax, bool labeled, const tdfs_options
   return TDFS_OK;
 }
 
+bool flat_options(const tdfs_options &o) {
+  return o.work_budget == 0 && o.steal != 0 && o.merge_window == 0 && o.merge_ratio == 0 && o.fixed_stage == 0 &&
+         o.steal_min == 0 && o.steal_first == 0 && o.lane_list == 0 && o.split_rush_us == 0 &&
+         o.leaf_steal_min == 0 && o.level_hoist == 0 && o.tail_count == 0 && o.dead_prune == 0;
+}
+
+int flat_shape(int device, int smax, bool labeled, const tdfs_options &o, FlatShape *out) {
+  static int sms[64] = {};
+  static std::map<std::tuple<int, bool, int, size_t>, int> occ;  // CTAs per SM, as launch_shape caches them
+  static std::mutex mu;
+  FlatShape s;
+  std::memset(&s, 0, sizeof s);
+  s.warps_per_block = o.warps_per_block > 0 ? o.warps_per_block : 8;
+  // entries per warp: as many as let 4 CTAs share an SM; chunk_cap asks for
+  // that many (at least 64) per level
+  const int levels = std::max(1, smax - 1);
+  s.cfg.entries = o.chunk_cap > 0 ? std::max(64, (o.chunk_cap + 31) & ~31) * levels : smax > 1 ? flat_auto_entries() : 0;
+  // (launch_shape accepts depths whose buffers fit the DFS kernel's layout)
+  s.cfg.entries = std::min(s.cfg.entries, flat_max_entries(s.warps_per_block));
+  s.cfg.warp_bytes = (int)flat_warp_bytes(s.cfg.entries);
+  s.cfg.idle_ms = o.wait_limit_ms > 0 ? o.wait_limit_ms : 30000;
+  s.cfg.split_ns = o.split_after_us > 0 ? o.split_after_us * 1000 : (o.split_after_us < 0 ? 0 : 30000);
+  s.cfg.segments = o.label_rows < 0 ? 0 : 1;
+  const size_t smem = (size_t)s.cfg.warp_bytes * s.warps_per_block;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!sms[device]) {
+    const cudaError_t e = cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return cuda_err(e, "cudaDeviceGetAttribute");
+  }
+  const auto key = std::make_tuple(device, labeled, s.warps_per_block, smem);
+  auto it = occ.find(key);
+  if (it == occ.end()) {
+    const int fit = flat_blocks_per_sm(labeled, s.warps_per_block, smem);
+    if (fit < 0) return fail(TDFS_ERR_CUDA, "occupancy query failed: %s", cudaGetErrorString(cudaGetLastError()));
+    it = occ.emplace(key, fit).first;
+  }
+  if (it->second == 0) return fail(TDFS_ERR_CAPACITY, "the flat kernel does not fit on an SM with this shape");
+  s.blocks = std::min(sms[device] * (o.blocks_per_sm > 0 ? std::min(o.blocks_per_sm, it->second) : it->second),
+                      flat_max_blocks(s.warps_per_block));
+  *out = s;
+  return TDFS_OK;
+}
+
 // The level-0 range of a slot: the edge ids [eb, ee), or -- for a labeled
 // plan on a graph with a label index -- the positions of the index group of
 // the plan's first two labels that hold those ids.
@@ -165,6 +210,14 @@ int64_t ticket_count(int64_t b, int64_t e, int stride, int phase, int chunk) {
   return (chunks - phase + stride - 1) / stride;
 }
 
+// One launch of either kernel.
+struct Launch {
+  bool flat;
+  LaunchShape dfs;  // !flat
+  FlatShape fl;     // flat
+  int warps() const { return flat ? fl.blocks * fl.warps_per_block : dfs.blocks * dfs.warps_per_block; }
+};
+
 // Captured launches: one CUDA graph per (batch size, mode, launch shape)
 // holding the slot-table upload from the pinned staging copy, the control
 // reset, the kernel and the read-back; replays read the staging copy as it is
@@ -172,8 +225,7 @@ int64_t ticket_count(int64_t b, int64_t e, int stride, int phase, int chunk) {
 struct GraphEntry {
   int n;
   bool labeled;
-  int blocks, warps;
-  KernelCfg cfg;
+  Launch launch;
   cudaGraphExec_t exec;
   cudaEvent_t k0, k1;  // recorded inside the graph around the match kernel
 };
@@ -199,7 +251,20 @@ std::vector<GraphEntry> &graph_cache(tdfs_graph *g) {
   return *static_cast<std::vector<GraphEntry> *>(g->graphs);
 }
 
-int enqueue_launch(tdfs_graph *g, const LaunchShape &s, bool labeled, int n, cudaStream_t st, cudaEvent_t k0,
+void reset_launch(tdfs_graph *g, const Launch &L, cudaStream_t st) {
+  if (L.flat) init_flat(g->ctl, g->queue, st);
+  else init_launch(g->ctl, queue_hdr(g), st);
+}
+
+int enqueue_kernel(tdfs_graph *g, const Launch &L, bool labeled, cudaStream_t st) {
+  if (L.flat)
+    return launch_flat(labeled, graph_view(g), g->ctl, g->tab, g->queue, L.fl.cfg, L.fl.blocks,
+                       L.fl.warps_per_block, st);
+  return launch_match(labeled, graph_view(g), g->ctl, g->tab, g->queue, queue_hdr(g), L.dfs.cfg, L.dfs.blocks,
+                      L.dfs.warps_per_block, st);
+}
+
+int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStream_t st, cudaEvent_t k0,
                    cudaEvent_t k1) {
   SlotTable *h = g->htab, *d = g->tab;
   cudaError_t e = cudaMemcpyAsync(&d->ctl, &h->ctl, sizeof h->ctl, cudaMemcpyHostToDevice, st);
@@ -207,13 +272,12 @@ int enqueue_launch(tdfs_graph *g, const LaunchShape &s, bool labeled, int n, cud
   if (e == cudaSuccess) e = cudaMemcpyAsync(d->info, h->info, sizeof(SlotInfo) * n, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d->plan, h->plan, sizeof(DevPlan) * n, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_err(e, "slot table upload");
-  init_launch(g->ctl, queue_hdr(g), st);
+  reset_launch(g, L, st);
   // external records: captured as event-record nodes, so they time the
   // kernel when the graph replays (a plain record is only a join point)
   e = cudaEventRecordWithFlags(k0, st, cudaEventRecordExternal);
   if (e != cudaSuccess) return cuda_err(e, "kernel start event");
-  int rc = launch_match(labeled, graph_view(g), g->ctl, d, g->queue, queue_hdr(g), s.cfg, s.blocks,
-                        s.warps_per_block, st);
+  int rc = enqueue_kernel(g, L, labeled, st);
   if (rc) return rc;
   e = cudaEventRecordWithFlags(k1, st, cudaEventRecordExternal);
   if (e != cudaSuccess) return cuda_err(e, "kernel end event");
@@ -226,12 +290,13 @@ int enqueue_launch(tdfs_graph *g, const LaunchShape &s, bool labeled, int n, cud
 // Counts of a finished launch from the read-back slot lines.  A slot that ran
 // out of its work budget gets status TDFS_ERR_TIMEOUT and count 0; without a
 // status array that fails the call.
-int collect(const RunCtl &hc, const SlotHot *hot, int n, unsigned long long *raw, int *status) {
+int collect(const RunCtl &hc, const SlotHot *hot, int n, bool flat, unsigned long long *raw, int *status) {
   if (hc.error == TDFS_ERR_TIMEOUT) return fail(TDFS_ERR_TIMEOUT, "a bounded device wait ran out");
   if (hc.error) return fail(hc.error, "device error %d", hc.error);
+  if (flat && !hc.finished) return fail(TDFS_ERR_TIMEOUT, "the launch did not complete");
   int first_abort = -1;
   for (int i = 0; i < n; ++i) {
-    if (hot[i].state != kSlotDone) return fail(TDFS_ERR_TIMEOUT, "slot %d did not complete", i);
+    if (!flat && hot[i].state != kSlotDone) return fail(TDFS_ERR_TIMEOUT, "slot %d did not complete", i);
     const bool ab = hot[i].aborted != 0;
     raw[i] = ab ? 0 : hot[i].count;
     if (status) status[i] = ab ? TDFS_ERR_TIMEOUT : TDFS_OK;
@@ -242,7 +307,7 @@ int collect(const RunCtl &hc, const SlotHot *hot, int n, unsigned long long *raw
   return TDFS_OK;
 }
 
-int run_captured(tdfs_graph *g, const LaunchShape &s, bool labeled, int n, float *ms, unsigned long long *raw,
+int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms, unsigned long long *raw,
                  int *status) {
   cudaError_t e;
   if (!g->ws->gstream) {
@@ -255,18 +320,17 @@ int run_captured(tdfs_graph *g, const LaunchShape &s, bool labeled, int n, float
   auto &cache = graph_cache(g);
   const GraphEntry *hit = nullptr;
   for (auto &c : cache)
-    if (c.n == n && c.labeled == labeled && c.blocks == s.blocks && c.warps == s.warps_per_block &&
-        !std::memcmp(&c.cfg, &s.cfg, sizeof c.cfg))
+    if (c.n == n && c.labeled == labeled && !std::memcmp(&c.launch, &L, sizeof L))
       hit = &c;
   if (!hit) {
-    GraphEntry ent{n, labeled, s.blocks, s.warps_per_block, s.cfg, nullptr, nullptr, nullptr};
+    GraphEntry ent{n, labeled, L, nullptr, nullptr, nullptr};
     e = cudaEventCreate(&ent.k0);
     if (e == cudaSuccess) e = cudaEventCreate(&ent.k1);
     if (e != cudaSuccess) return cuda_err(e, "cudaEventCreate");
     cudaGraph_t graph;
     e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_err(e, "cudaStreamBeginCapture");
-    int rc = enqueue_launch(g, s, labeled, n, st, ent.k0, ent.k1);
+    int rc = enqueue_launch(g, L, labeled, n, st, ent.k0, ent.k1);
     e = cudaStreamEndCapture(st, &graph);
     if (!rc && e == cudaSuccess) {
       e = cudaGraphInstantiate(&ent.exec, graph, 0);
@@ -285,27 +349,37 @@ int run_captured(tdfs_graph *g, const LaunchShape &s, bool labeled, int n, float
   // the match kernel's own time, from the event nodes around it in the graph
   if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, hit->k0, hit->k1);
   if (e != cudaSuccess) return cuda_err(e, "graph launch");
-  return collect(*g->hctl, g->htab->hot, n, raw, status);
+  return collect(*g->hctl, g->htab->hot, n, L.flat, raw, status);
 }
 
 // One launch over n plans of the same mode: slot i counts plans[i] on the
 // option's edge range; raw[i] receives the count before the |Aut| multiplier.
-int run_batch(tdfs_graph *g, const DevPlan *const *plans, int n, const tdfs_options &o, unsigned long long *raw,
-              int *status, float *ms) {
+// flat: on the flat kernel (every plan has that form), else on the DFS kernel.
+int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, const tdfs_options &o,
+              unsigned long long *raw, int *status, float *ms) {
   if (n <= 0) return TDFS_OK;
   if (n > kMaxSlots) return fail(TDFS_ERR_CAPACITY, "at most %d plans per launch", kMaxSlots);
-  const bool labeled = plans[0]->labeled != 0;
-  int kmax = 3;
+  const bool labeled = plans[0]->dev.labeled != 0;
+  int kmax = 3, smax = 1;
   for (int i = 0; i < n; ++i) {
-    if ((plans[i]->labeled != 0) != labeled) return fail(TDFS_ERR_ARG, "a launch mixes labeled and unlabeled plans");
-    kmax = std::max(kmax, (int)plans[i]->k);
+    if ((plans[i]->dev.labeled != 0) != labeled) return fail(TDFS_ERR_ARG, "a launch mixes labeled and unlabeled plans");
+    kmax = std::max(kmax, (int)plans[i]->dev.k);
+    if (flat) smax = std::max(smax, (int)plans[i]->flat.s);
   }
   if (labeled && !g->labeled) return fail(TDFS_ERR_ARG, "labeled pattern on a graph opened without labels");
   cudaError_t e = cudaSetDevice(g->device);
   if (e != cudaSuccess) return cuda_err(e, "cudaSetDevice");
-  LaunchShape s;
-  int rc = launch_shape(g, kmax, labeled, o, &s);
+  Launch L;
+  std::memset(static_cast<void *>(&L), 0, sizeof L);
+  L.flat = flat;
+  LaunchShape shape;
+  int rc = launch_shape(g, kmax, labeled, o, &shape);  // checks the options for either kernel
   if (rc) return rc;
+  if (flat) {
+    if ((rc = flat_shape(g->device, smax, labeled, o, &L.fl))) return rc;
+  } else {
+    L.dfs = shape;
+  }
   if ((rc = acquire_workspace(g))) return rc;
   const int64_t eb = std::max<int64_t>(0, o.edge_begin);
   const int64_t ee = (o.edge_end < 0 || o.edge_end > g->nedges) ? g->nedges : o.edge_end;
@@ -315,10 +389,10 @@ int run_batch(tdfs_graph *g, const DevPlan *const *plans, int n, const tdfs_opti
   std::memset(&h->ctl, 0, sizeof h->ctl);
   h->ctl.admitted = (unsigned long long)n;
   h->ctl.shutdown = 1;
-  const int warps = s.blocks * s.warps_per_block;
+  const int warps = L.warps();
   for (int i = 0; i < n; ++i) {
     SlotInfo &in = h->info[i];
-    level0_range(g, *plans[i], eb, ee, o.label_index >= 0, &in);
+    level0_range(g, plans[i]->dev, eb, ee, o.label_index >= 0, &in);
     in.stride = stride;
     in.phase = o.edge_phase;
     in.chunk = auto_chunk(in.e_end - in.e_begin, stride, warps, o.edge_chunk);
@@ -327,10 +401,22 @@ int run_batch(tdfs_graph *g, const DevPlan *const *plans, int n, const tdfs_opti
     std::memset(&h->hot[i], 0, sizeof h->hot[i]);
     h->hot[i].state = in.ntickets > 0 ? kSlotActive : kSlotDone;  // an empty range is done at once
     if (in.ntickets == 0) ++h->ctl.completed;
-    h->plan[i] = *plans[i];
+    if (flat) std::memcpy(&h->plan[i], &plans[i]->flat, sizeof plans[i]->flat);
+    else h->plan[i] = plans[i]->dev;
   }
-  g->last_warps = (int64_t)s.blocks * s.warps_per_block;
-  if (o.graph_capture) return run_captured(g, s, labeled, n, ms, raw, status);
+  if (flat) {
+    // tickets run over all slots in order; the first ones are dealt one per
+    // warp, so the warps do not queue for them on one counter
+    for (int i = 0; i < n; ++i) {
+      h->info[i].ticket0 = h->ctl.tickets;
+      h->ctl.tickets += h->info[i].ntickets;
+    }
+    h->ctl.slots = n;
+    h->ctl.ticket = (unsigned long long)warps;
+    h->ctl.pending = L.fl.blocks;
+  }
+  g->last_warps = warps;
+  if (o.graph_capture) return run_captured(g, L, labeled, n, ms, raw, status);
   cudaStream_t st = static_cast<cudaStream_t>(o.stream);
   SlotTable *d = g->tab;
   e = cudaMemcpyAsync(&d->ctl, &h->ctl, sizeof h->ctl, cudaMemcpyHostToDevice, st);
@@ -343,9 +429,9 @@ int run_batch(tdfs_graph *g, const DevPlan *const *plans, int n, const tdfs_opti
     cudaEventCreate(&ev0);
     cudaEventCreate(&ev1);
   }
-  init_launch(g->ctl, queue_hdr(g), st);
+  reset_launch(g, L, st);
   if (ms) cudaEventRecord(ev0, st);
-  rc = launch_match(labeled, graph_view(g), g->ctl, d, g->queue, queue_hdr(g), s.cfg, s.blocks, s.warps_per_block, st);
+  rc = enqueue_kernel(g, L, labeled, st);
   if (ms) cudaEventRecord(ev1, st);
   if (!rc) {
     e = cudaMemcpyAsync(h->hot, d->hot, sizeof(SlotHot) * n, cudaMemcpyDeviceToHost, st);
@@ -360,7 +446,7 @@ int run_batch(tdfs_graph *g, const DevPlan *const *plans, int n, const tdfs_opti
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (rc) return rc;
-  return collect(*g->hctl, h->hot, n, raw, status);
+  return collect(*g->hctl, h->hot, n, flat, raw, status);
 }
 
 }  // namespace
@@ -368,6 +454,7 @@ int run_batch(tdfs_graph *g, const DevPlan *const *plans, int n, const tdfs_opti
 
 namespace tdfs {
 const DevPlan &plan_device_table(const tdfs_plan *p) { return p->dev; }
+const FlatPlan *plan_flat_table(const tdfs_plan *p) { return p->has_flat ? &p->flat : nullptr; }
 }  // namespace tdfs
 
 using namespace tdfs;
@@ -426,6 +513,7 @@ int tdfs_plan_from_text(const char *text, int labeled, tdfs_plan **out) {
   int rc = compile_pattern(text, labeled != 0, &p->host);
   if (rc) return rc;
   p->dev = p->host.to_device();
+  p->has_flat = flat_plan(p->dev, &p->flat);
   *out = p.release();
   return TDFS_OK;
 }
@@ -470,8 +558,7 @@ int tdfs_count(tdfs_graph *g, const tdfs_plan *p, const tdfs_options *opt, uint6
   tdfs_options o;
   if (opt) o = *opt; else tdfs_options_default(&o);
   unsigned long long raw = 0;
-  const DevPlan *dp = &p->dev;
-  int rc = run_batch(g, &dp, 1, o, &raw, nullptr, kernel_ms);
+  int rc = run_batch(g, &p, 1, g->hash && p->has_flat && flat_options(o), o, &raw, nullptr, kernel_ms);
   if (rc) return rc;
   // cu_test.cu:100-105: the unlabeled total is multiplied by |Aut|
   *count = (uint64_t)(raw * (unsigned long long)p->dev.multiplicity);
@@ -489,14 +576,17 @@ int tdfs_count_batch_status(tdfs_graph *g, const tdfs_plan *const *plans, int np
   tdfs_options o;
   if (opt) o = *opt; else tdfs_options_default(&o);
   float total = 0.f;
-  // one launch per mode (a launch runs either the labeled or the unlabeled kernel)
-  for (int mode = 0; mode < 2; ++mode) {
-    std::vector<const DevPlan *> dp;
+  for (int i = 0; i < nplans; ++i)
+    if (!plans[i]) return fail(TDFS_ERR_ARG, "null plan %d", i);
+  const bool flat_here = g->hash && flat_options(o);
+  // one launch per mode (labeled or unlabeled) and kernel
+  for (int launch = 0; launch < 4; ++launch) {
+    const bool labeled = launch >= 2, flat = (launch & 1) == 0;
+    std::vector<const tdfs_plan *> dp;
     std::vector<int> idx;
     for (int i = 0; i < nplans; ++i) {
-      if (!plans[i]) return fail(TDFS_ERR_ARG, "null plan %d", i);
-      if ((plans[i]->dev.labeled != 0) == (mode == 1)) {
-        dp.push_back(&plans[i]->dev);
+      if ((plans[i]->dev.labeled != 0) == labeled && (flat_here && plans[i]->has_flat) == flat) {
+        dp.push_back(plans[i]);
         idx.push_back(i);
       }
     }
@@ -505,11 +595,12 @@ int tdfs_count_batch_status(tdfs_graph *g, const tdfs_plan *const *plans, int np
       std::vector<unsigned long long> raw(n);
       std::vector<int> st(n, TDFS_OK);
       float ms = 0.f;
-      int rc = run_batch(g, dp.data() + b, n, o, raw.data(), status ? st.data() : nullptr, kernel_ms ? &ms : nullptr);
+      int rc = run_batch(g, dp.data() + b, n, flat, o, raw.data(), status ? st.data() : nullptr,
+                         kernel_ms ? &ms : nullptr);
       if (rc) return rc;
       total += ms;
       for (int j = 0; j < n; ++j) {
-        counts[idx[b + j]] = (uint64_t)(raw[j] * (unsigned long long)dp[b + j]->multiplicity);
+        counts[idx[b + j]] = (uint64_t)(raw[j] * (unsigned long long)dp[b + j]->dev.multiplicity);
         if (status) status[idx[b + j]] = st[j];
       }
     }
@@ -524,19 +615,15 @@ int tdfs_autotune(tdfs_graph *g, const tdfs_plan *const *plans, int nplans, cons
   tdfs_options b;
   if (base) b = *base; else tdfs_options_default(&b);
   if (sample_stride < 1) sample_stride = 1;
-  // resolve the automatic values so every knob has a concrete start
+  // The descent starts from the caller's options, in general the automatic
+  // choice of the kernel; a value for one of the DFS kernel's own knobs tries
+  // that kernel (flat_options) and is kept when it wins.  chunk_cap stays
+  // automatic (0) unless a fixed depth wins: the automatic depth is chosen
+  // per launch, so a batch that mixes modes gets each launch's own.
   tdfs_options cur = b;
   if (cur.warps_per_block <= 0) cur.warps_per_block = 8;
-  // chunk_cap stays automatic (0) unless a fixed depth wins: the automatic
-  // depth is chosen per launch, so a batch that mixes modes gets each
-  // launch's own
   cur.chunk_cap = std::max(0, cur.chunk_cap);
-  if (cur.merge_window == 0) cur.merge_window = 128;
   if (cur.steal < 0) cur.steal = 1;
-  if (cur.steal_min <= 0) cur.steal_min = 2;
-  if (cur.merge_ratio <= 0) cur.merge_ratio = 4;
-  if (cur.tail_count == 0) cur.tail_count = 1;
-  if (cur.dead_prune == 0) cur.dead_prune = 1;
   cur.edge_stride = sample_stride;
   cur.edge_phase = 0;
   std::vector<uint64_t> counts(nplans);

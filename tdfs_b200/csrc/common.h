@@ -37,6 +37,42 @@ struct DevPlan {
   uint64_t multiplicity;      // |Aut| multiplier (unlabeled)
 };
 
+// ---- flat plans (flat.cu) ---------------------------------------------------
+// One candidate set as the flat kernel produces or counts it: the backward
+// neighbours whose lists are intersected, the label, and bit masks over the
+// earlier vertices j of the conditions x > phi(j), x < phi(j), x != phi(j).
+// With dep != 0 the set is also the candidate set of the earlier vertex dep
+// intersected with the lists of bnsh (the plan's reuse level).
+struct FlatStep {
+  uint8_t nbn;
+  uint8_t bn[kMaxK - 1];
+  uint8_t label;
+  uint8_t larger, less, neq;
+  uint8_t dep, nsh;
+  uint8_t bnsh[3];
+};
+
+// How the flat kernel runs a plan: vertices 2..s are enumerated (step[i - 2]);
+// the t = k - 1 - s vertices after s are counted below each level-s node from
+// the sizes of the candidate sets term[]: term_of[m] is the set shared by the
+// tail vertices in bit mask m (kNoTerm: empty).  form 0: tuples of distinct
+// vertices by inclusion-exclusion; form 1: the tail vertices have one and the
+// same set and a total order among them, so the tuples are its t-subsets.
+constexpr uint8_t kNoTerm = 255;
+struct FlatPlan {
+  int32_t k, orient;
+  int32_t deg[3];
+  int32_t label[2];     // of pattern vertices 0 and 1
+  uint8_t s, t, form, nterm;
+  uint8_t term_of[8];
+  FlatStep step[4];
+  FlatStep term[7];
+};
+static_assert(sizeof(FlatPlan) <= sizeof(DevPlan), "a slot's plan record holds either plan");
+
+// The flat form of a plan; false when it has none (flat_plan.cpp).
+bool flat_plan(const DevPlan &d, FlatPlan *out);
+
 // Device view of a resident data graph.
 struct DevGraph {
   const int64_t *rowptr;   // n + 1
@@ -47,11 +83,24 @@ struct DevGraph {
   const int32_t *lperm;    // level-0 label index (labeled graphs), or nullptr
   const int32_t *colidx_l; // labeled graphs with few labels: every row re-sorted by (label, id), or nullptr
   const int32_t *loff;     // its segment starts: loff[v * (nlab + 1) + l], relative to rowptr[v]
+  const int32_t *hash;     // row membership tables (see row_table_buckets), or nullptr
   int32_t nlab;            // labels 0..nlab-1 have segments
   int64_t nedges;
   int32_t n;
   int32_t max_degree;
 };
+
+// ---- row membership tables ---------------------------------------------------
+// Every adjacency row again as a hash table of 8-entry buckets (32 bytes: one
+// load, one sector): "is y in row v?" costs one load, whatever the row's
+// length, where a binary search costs log2(degree) dependent ones.  Row v owns
+// the buckets [first, first + count) with first = rowptr[v] / 3 + v, so no
+// offset array is needed and a bucket holds 3 entries on average.  Entries
+// fill a bucket in order, -1 is empty; a full bucket (about one in a hundred)
+// overflows into the next one, cyclically within the row.
+constexpr int kBucket = 8;
+inline int64_t row_table_buckets(int64_t n, int64_t nedges) { return nedges / 3 + n + 1; }
+constexpr uint32_t kRowHash = 0x9E3779B1u;  // 2^32 / golden ratio: neighbouring ids spread over the buckets
 
 // Per-launch control block in device memory.  Counters that many warps touch
 // sit on their own 128-byte lines so ticket atomics, idle polling and the
@@ -65,7 +114,8 @@ struct alignas(128) RunCtl {
   int32_t pad_;
   unsigned long long idle_ns;    // diagnostics: summed time warps spent without work
   unsigned long long warp_ns;    // diagnostics: summed time warps ran
-  char pad1_[88];
+  int32_t finished;              // flat kernel: 1 = no work was left anywhere
+  char pad1_[84];
 };
 
 // Error reporting shared by the C ABI implementation files.

@@ -1,0 +1,905 @@
+// flat.cu -- the flattened subgraph-counting kernel (design notes in flat.cuh).
+// Count semantics follow src/gpu_match.cu:260-1080 as in match.cu; plans come
+// in the form flat_plan.cpp derives.
+#include <cuda_runtime.h>
+
+#include <climits>
+#include <mutex>
+
+#include "flat.cuh"
+
+namespace tdfs {
+
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kTupleMax = kMaxK - 1;   // phi(0..5): the deepest enumerated level is 5
+constexpr int kProbeMax = kMaxK - 2;   // lists tested per candidate besides its source
+constexpr int kScanSteps = 64;         // 64-position steps of a leaf scan between two looks at the idle count
+constexpr int kCheckCycles = 16384;    // clocks between those looks
+constexpr int kUnitInts = 156;         // vertices one mailbox carries
+constexpr int kBoxes = 8192;           // mailboxes, one per warp of the grid
+constexpr int kIdleWords = kBoxes / 32;
+
+// Work given away goes straight to an idle warp: each warp has a mailbox and
+// a bit in a grid-wide mask of idle warps.  A busy warp reads 32 words of the
+// mask with one load, each lane claims one idle warp by clearing its bit, and
+// the entries are spread over all of them.  No two warps meet on a counter,
+// as they would on a shared ring (which passed 1.2 units per microsecond
+// whatever the demand and left 60-90% of the warps of a power-law launch
+// idle), and an idle warp reads its own line only.
+// A mailbox holds up to 32 partial embeddings (tuples of level + 1 vertices).
+struct FlatBox {
+  int32_t full;  // 0 empty, 1 filled by the warp that cleared the idle bit
+  int32_t level, n, slot;
+  int32_t v[kUnitInts];
+};
+struct FlatShared {
+  FlatBox box[kBoxes];
+  unsigned idle[kIdleWords];
+};
+static_assert(sizeof(FlatShared) <= sizeof(SplitUnit) * kQueueCap, "the mailboxes use the split ring's memory");
+
+struct FlatLevel {
+  int32_t next;      // first entry of the block being extended (blocks of 32 entries)
+  int32_t end;       // entries [next, end) are left to extend
+  int32_t n;         // entries in the buffer (>= end: some may have been given away)
+  uint32_t pos;      // positions of the block already done
+  int32_t started;   // first entry not yet touched
+  int32_t cutp;      // entry whose list the position pos lies inside, or -1
+  int32_t hcut, tcut;  // parents whose children here are incomplete at the front / at the end, or -1
+  int32_t groups;    // 0: entries came from elsewhere; siblings are not together
+};
+
+// Shared by a CTA's warps.
+struct FlatCta {
+  int32_t poll;    // 1: some idle warp of the CTA is watching SlotCtl::pending
+  int32_t done;    // 1: no work is left anywhere
+  int32_t active;  // busy warps; the CTA counts in SlotCtl::pending while there are any
+  int32_t left;    // warps still in the kernel
+  int32_t slot;    // slot whose counts are summed here first, -1 none
+  unsigned long long sum, idle_ns, warp_ns;
+};
+
+struct alignas(16) FlatSmem {
+  FlatPlan plan;
+  int32_t slot;                     // slot of `plan`, -1 none
+  int32_t cap;                      // entries per level
+  FlatLevel lev[kMaxK];             // levels 1..s
+  int64_t base[32];                 // per lane: source list start minus its first position
+  int32_t phi[kTupleMax][32];       // per lane: the partial embedding being extended
+  uint32_t hb[kProbeMax][32];       // per lane: row tables to test (first bucket, bucket count; 0 = no test)
+  uint32_t nb[kProbeMax][32];
+  uint32_t cnt[7][32];              // per lane: sizes of the tail's sets
+  int32_t er[32], ec[32];           // level-1 entries: edges (phi(0), phi(1))
+  uint8_t map[32];                  // rank among the lanes with a list -> lane
+  uint8_t kind[32];                 // per lane: 1 = the source is a range of sibling entries
+  unsigned long long t_work;        // globaltimer when the current base work was taken
+  unsigned long long idle_total, t_start;  // diagnostics
+};
+
+__device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
+__device__ __forceinline__ unsigned lanemask_lt() {
+  unsigned m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+template <bool LAB>
+struct Flat {
+  const DevGraph &G;
+  const FlatCfg &cfg;
+  RunCtl *ctl;
+  SlotTable *tab;
+  FlatShared *sh;
+  FlatBox &box;  // this warp's
+  const int gid;
+  FlatSmem &W;
+  FlatCta &C;
+  int32_t *X;   // entries: the vertex of the level ...
+  uint16_t *P;  // ... and the parent's entry one level up
+  unsigned long long count = 0;  // per lane; summed at release
+  int lane;
+
+  __device__ Flat(const DevGraph &g, const FlatCfg &c, RunCtl *ct, SlotTable *tb, FlatShared *s, int warp,
+                  FlatSmem &w, FlatCta &cta, unsigned char *bufs)
+      : G(g), cfg(c), ctl(ct), tab(tb), sh(s), box(s->box[warp]), gid(warp), W(w), C(cta), X(reinterpret_cast<int32_t *>(bufs)),
+        P(reinterpret_cast<uint16_t *>(bufs + (size_t)c.entries * 4)), lane(lane_id()) {}
+
+  __device__ __forceinline__ int32_t *xs(int l) const { return X + (l - 2) * W.cap; }
+  __device__ __forceinline__ uint16_t *ps(int l) const { return P + (l - 2) * W.cap; }
+  __device__ __forceinline__ bool segmented() const { return LAB && cfg.segments && G.colidx_l != nullptr; }
+  __device__ __forceinline__ const int32_t *lists() const { return segmented() ? G.colidx_l : G.colidx; }
+
+  // Adjacency row of v as candidates of label `lab` are drawn from it: its
+  // label segment when the graph has them, else the whole row.
+  __device__ __forceinline__ void row(int32_t v, int lab, int64_t &b, uint32_t &len) const {
+    const int64_t r = G.rowptr[v];
+    if (segmented()) {
+      b = r;
+      len = 0;
+      if (lab < G.nlab) {
+        const int32_t *o = G.loff + (int64_t)v * (G.nlab + 1) + lab;
+        const int32_t o0 = o[0];
+        b = r + o0;
+        len = (uint32_t)(o[1] - o0);
+      }
+    } else {
+      b = r;
+      len = (uint32_t)(G.rowptr[v + 1] - r);
+    }
+  }
+
+  // Row v's membership table: false when the row is empty.
+  __device__ __forceinline__ bool table(int32_t v, uint32_t &hb, uint32_t &nb) const {
+    const int64_t r = G.rowptr[v], e = G.rowptr[v + 1];
+    hb = (uint32_t)(r / 3 + v);
+    nb = (uint32_t)(e / 3 - r / 3) + 1;
+    return e > r;
+  }
+  // First half of bucket i (the second half shares its sector).
+  __device__ __forceinline__ int4 bucket(uint32_t i) const {
+    return __ldg(reinterpret_cast<const int4 *>(G.hash) + 2 * (size_t)i);
+  }
+  // Is x in the table, given the first half q of its bucket (offset b)?
+  __device__ __forceinline__ bool found(int4 q, uint32_t hb, uint32_t nb, uint32_t b, int32_t x) const {
+    if (q.x == x || q.y == x || q.z == x || q.w == x) return true;
+    if (q.w < 0) return false;  // entries fill a bucket in order
+    const int4 *h = reinterpret_cast<const int4 *>(G.hash);
+    uint32_t half = 2 * b + 1;  // 16-byte halves, cyclically within the row
+    for (uint32_t t = 1; t < 2 * nb; ++t) {
+      q = __ldg(h + 2 * (size_t)hb + half);
+      if (q.x == x || q.y == x || q.z == x || q.w == x) return true;
+      if (q.w < 0) return false;
+      half = half + 1 == 2 * nb ? 0 : half + 1;
+    }
+    return false;
+  }
+  __device__ __forceinline__ bool member(int32_t v, int32_t x) const {
+    uint32_t hb, nb;
+    if (!table(v, hb, nb)) return false;
+    const uint32_t b = __umulhi((uint32_t)x * kRowHash, nb);
+    return found(bucket(hb + b), hb, nb, b, x);
+  }
+
+  // This lane's partial embedding: entry p of level L and its ancestors, into
+  // W.phi.  Returns its ancestor entry at level `dep` (-1 when dep is 0).
+  __device__ __forceinline__ int load_tuple(int L, int p, int dep) {
+    int e = -1, q = p;
+    for (int l = L; l >= 2; --l) {
+      if (l == dep) e = q;
+      W.phi[l][lane] = xs(l)[q];
+      q = ps(l)[q];
+    }
+    W.phi[0][lane] = W.er[q];
+    W.phi[1][lane] = W.ec[q];
+    return e;
+  }
+
+  // Bounds of the order conditions of st under this lane's embedding.
+  __device__ __forceinline__ void bounds(const FlatStep &st, int32_t &lo, int32_t &hi) const {
+    lo = -1;
+    hi = INT_MAX;
+    if (!LAB) {
+      for (unsigned m = st.larger; m; m &= m - 1) lo = max(lo, W.phi[__ffs(m) - 1][lane]);
+      for (unsigned m = st.less; m; m &= m - 1) hi = min(hi, W.phi[__ffs(m) - 1][lane]);
+    }
+  }
+
+  // Narrow the ascending range a[b, b + len) to the values in (lo, hi).
+  template <typename T>
+  __device__ __forceinline__ void trim(const int32_t *a, T &b, int &len, int32_t lo, int32_t hi) const {
+    if (len > 0 && a[b] <= lo) {
+      int s = 1, e = len;  // a[b + s - 1] <= lo
+      while (s < e) {
+        const int m = (s + e) >> 1;
+        if (a[b + m] <= lo) s = m + 1; else e = m;
+      }
+      b += s;
+      len -= s;
+    }
+    if (hi < INT_MAX && len > 0 && a[b + len - 1] >= hi) {
+      int s = 0, e = len - 1;  // a[b + e] >= hi
+      while (s < e) {
+        const int m = (s + e) >> 1;
+        if (a[b + m] < hi) s = m + 1; else e = m;
+      }
+      len = s;
+    }
+  }
+
+  // Set up this lane's candidate scan for st (its embedding: entry p of level
+  // L).  Writes the source start (W.base, W.kind) and the row tables to test
+  // (W.hb, W.nb); returns the number of source positions.
+  __device__ int setup_lane(const FlatStep &st, int L, int p) {
+    const int e = load_tuple(L, p, st.dep);
+    // the shortest list is scanned, the others are tested
+    uint32_t best = UINT_MAX;
+    int64_t gb = 0;
+    int tb = 0;
+    for (int t = 0; t < st.nbn; ++t) {
+      int64_t b;
+      uint32_t len;
+      row(W.phi[st.bn[t]][lane], st.label, b, len);
+      if (len < best) {
+        best = len;
+        gb = b;
+        tb = t;
+      }
+    }
+    int len = (int)best;
+    if (len == 0) return 0;
+    // or, under reuse, the siblings of the ancestor at level dep, when they
+    // are all in its buffer
+    bool sib = false;
+    int sb = 0;
+    const int dep = st.dep;
+    if (dep && W.lev[dep].groups) {
+      const uint16_t *pp = ps(dep);
+      const int me = pp[e];
+      const bool later = !LAB && (st.larger >> dep & 1);  // only siblings after e can pass
+      if (me != W.lev[dep].tcut && (later || me != W.lev[dep].hcut)) {
+        int s = e + 1, t = W.lev[dep].n;
+        while (s < t) {
+          const int m = (s + t) >> 1;
+          if (pp[m] <= me) s = m + 1; else t = m;
+        }
+        sb = e + 1;
+        if (!later) {
+          int a = 0, z = e;
+          while (a < z) {
+            const int m = (a + z) >> 1;
+            if (pp[m] < me) a = m + 1; else z = m;
+          }
+          sb = a;
+        }
+        if (s - sb <= len) {
+          sib = true;
+          len = s - sb;
+        }
+      }
+    }
+    if (!LAB) {
+      int32_t lo, hi;
+      bounds(st, lo, hi);
+      if (sib) trim(xs(dep), sb, len, lo, hi);
+      else trim(lists(), gb, len, lo, hi);
+    }
+    if (len <= 0) return 0;
+    const int M = st.nbn - 1;
+    int u = 0;
+    const int nt = sib ? st.nsh : st.nbn;
+    for (int t = 0; t < nt; ++t) {
+      if (!sib && t == tb) continue;
+      uint32_t hb, nb;
+      if (!table(W.phi[sib ? st.bnsh[t] : st.bn[t]][lane], hb, nb)) return 0;
+      W.hb[u][lane] = hb;
+      W.nb[u][lane] = nb;
+      ++u;
+    }
+    for (; u < M; ++u) W.nb[u][lane] = 0;
+    W.base[lane] = sib ? (int64_t)sb : gb;
+    W.kind[lane] = sib;
+    return len;
+  }
+
+  // The candidates of st for the block of up to 32 entries at W.lev[L].next.
+  // mode 0: stored as entries of level L + 1 (until that buffer is full);
+  // mode 1: counted into `count`; mode 2: counted per entry into cnt[].
+  // Modes 0 and 1 resume at, and leave, the block's position in W.lev[L]; they
+  // return false when they stopped after kScanSteps steps, so that the caller
+  // can look for idle warps.
+  template <int mode>
+  __device__ __forceinline__ bool scan(const FlatStep &st, int L, uint32_t *cnt) {
+    FlatLevel &H = W.lev[L];
+    const int first = H.next;
+    int len = 0;
+    if (first + lane < H.end) len = setup_lane(st, L, first + lane);
+    uint32_t incl = (uint32_t)len;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, incl, s);
+      if (lane >= s) incl += t;
+    }
+    const uint32_t off = incl - (uint32_t)len;
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    const unsigned act = __ballot_sync(kFull, len > 0);
+    if (len > 0) {
+      W.map[__popc(act & lanemask_lt())] = (uint8_t)lane;
+      W.base[lane] -= (int64_t)off;
+    }
+    __syncwarp();
+    uint32_t pos = mode < 2 ? H.pos : 0u;
+    int cur = __popc(__ballot_sync(kFull, len > 0 && off < pos));  // lists that start before pos
+    const unsigned le = lanemask_lt() | (1u << lane);
+    const int M = st.nbn - 1;
+    const unsigned neq = st.neq;
+    const bool lab = LAB && !segmented();
+    const int32_t *L0 = lists();
+    const int32_t *Ls = st.dep ? xs(st.dep) : nullptr;
+    int32_t *ox = nullptr;
+    uint16_t *op = nullptr;
+    int n = 0;
+    if (mode == 0) {
+      ox = xs(L + 1);
+      op = ps(L + 1);
+      n = W.lev[L + 1].n;
+    }
+    const int room = W.cap - 64;
+    int step = 0;
+    for (; pos < total; ++step, pos += 64) {
+      if (mode < 2 && step >= kScanSteps) break;
+      if (mode == 0 && n > room) break;
+      int o[2];
+      int32_t x[2];
+      bool ok[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t b = pos + 32 * u;
+        // the lists that start inside these 32 positions, as a bit mask: a
+        // lane's owner is the last one that starts at or before it
+        const unsigned m = __reduce_or_sync(kFull, len > 0 && off - b < 32u ? 1u << (off - b) : 0u);
+        const int r = cur + __popc(m & le) - 1;
+        cur += __popc(m);
+        ok[u] = b + (uint32_t)lane < total;
+        o[u] = ok[u] ? W.map[r] : 0;
+        x[u] = 0;
+        if (ok[u]) {
+          const int64_t i = W.base[o[u]] + (int64_t)(b + (uint32_t)lane);
+          x[u] = W.kind[o[u]] ? Ls[i] : L0[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (lab && ok[u]) ok[u] = G.label[x[u]] == st.label;
+        for (unsigned m = neq; m; m &= m - 1) ok[u] &= W.phi[__ffs(m) - 1][o[u]] != x[u];
+      }
+      for (int m = 0; m < M; ++m) {
+        uint32_t nb[2], hb[2], b[2];
+        int4 q[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          nb[u] = ok[u] ? W.nb[m][o[u]] : 0u;
+          hb[u] = W.hb[m][o[u]];
+          b[u] = __umulhi((uint32_t)x[u] * kRowHash, nb[u]);
+          if (nb[u]) q[u] = bucket(hb[u] + b[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (nb[u]) ok[u] = found(q[u], hb[u], nb[u], b[u], x[u]);
+      }
+      if (mode == 0) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const unsigned m = __ballot_sync(kFull, ok[u]);
+          if (ok[u]) {
+            const int at = n + __popc(m & lanemask_lt());
+            ox[at] = x[u];
+            op[at] = (uint16_t)(first + o[u]);
+          }
+          n += __popc(m);
+        }
+      } else if (mode == 1) {
+        count += (unsigned)ok[0] + (unsigned)ok[1];
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (ok[u]) atomicAdd(&cnt[o[u]], 1u);
+      }
+    }
+    __syncwarp();
+    if (mode == 2) return true;
+    const bool done = pos >= total;
+    const unsigned in = __ballot_sync(kFull, len > 0 && off < pos && off + (uint32_t)len > pos);
+    const unsigned before = __ballot_sync(kFull, len > 0 && off < pos);
+    if (lane == 0) {
+      if (mode == 0) W.lev[L + 1].n = n;
+      if (done) {
+        H.next = min(first + 32, H.end);
+        H.pos = 0;
+        H.started = H.next;
+        H.cutp = -1;
+      } else {
+        H.pos = pos;
+        H.started = before ? first + 32 - __clz(before) : first;
+        H.cutp = in ? first + __ffs(in) - 1 : -1;
+      }
+    }
+    __syncwarp();
+    return done || step < kScanSteps;
+  }
+
+  // Fill level L + 1 from the entries of level L; `more`: go on filling.
+  // Returns true when it stopped early (kScanSteps).
+  __device__ bool expand(int L, bool more) {
+    FlatLevel &H = W.lev[L], &D = W.lev[L + 1];
+    if (lane == 0 && !more) {
+      D.next = D.end = D.n = 0;
+      D.pos = 0;
+      D.started = 0;
+      D.cutp = -1;
+      D.hcut = H.pos ? H.cutp : -1;
+      D.groups = 1;
+    }
+    __syncwarp();
+    while (H.next < H.end && D.n <= W.cap - 64)
+      if (!scan<0>(W.plan.step[L - 1], L, nullptr)) return true;
+    if (lane == 0) {
+      D.end = D.n;
+      D.tcut = H.pos ? H.cutp : -1;
+    }
+    __syncwarp();
+    return false;
+  }
+
+  // Size of the set st of this lane's embedding (in W.phi), st having a single
+  // list: the list's part inside the bounds, less the earlier vertices found
+  // in it (on labeled plans those of the set's label).
+  __device__ uint32_t closed_count(const FlatStep &st) {
+    const int32_t v = W.phi[st.bn[0]][lane];
+    int64_t b;
+    uint32_t ulen;
+    row(v, st.label, b, ulen);
+    int len = (int)ulen;
+    int32_t lo, hi;
+    bounds(st, lo, hi);
+    if (!LAB) trim(lists(), b, len, lo, hi);
+    if (len <= 0) return 0;
+    int c = len;
+    for (unsigned m = st.neq; m; m &= m - 1) {
+      const int j = __ffs(m) - 1;
+      const int32_t y = W.phi[j][lane];
+      if (j == 1 && (st.neq & 1) && y == W.phi[0][lane]) continue;  // a self-loop edge: one value
+      if (y > lo && y < hi && member(v, y)) --c;
+    }
+    return (uint32_t)c;
+  }
+
+  // Count below a block of level-s entries.
+  __device__ void leaf(int L) {
+    FlatLevel &H = W.lev[L];
+    const FlatPlan &F = W.plan;
+    const bool single = !LAB || segmented();  // single lists are counted in closed form
+    if (F.t == 1 && !(F.term[0].nbn == 1 && single)) {
+      scan<1>(F.term[0], L, nullptr);
+      return;
+    }
+    const int p = H.next + lane;
+    const bool mine = p < H.end;
+    for (int u = 0; u < F.nterm; ++u) {
+      const FlatStep &st = F.term[u];
+      uint32_t c = 0;
+      if (st.nbn == 1 && single) {
+        if (mine) {
+          load_tuple(L, p, 0);
+          c = closed_count(st);
+        }
+        W.cnt[u][lane] = c;
+      } else {
+        W.cnt[u][lane] = 0;
+        __syncwarp();
+        scan<2>(st, L, W.cnt[u]);
+      }
+      __syncwarp();
+    }
+    if (mine) {
+      auto at = [&](int m) -> unsigned long long {
+        const int u = F.term_of[m];
+        return u == kNoTerm ? 0ull : (unsigned long long)W.cnt[u][lane];
+      };
+      const unsigned long long a = at(1);
+      if (F.t == 1) {
+        count += a;
+      } else if (F.form == 1) {
+        count += F.t == 2 ? a * (a - 1) / 2 : a * (a - 1) / 2 * (a - 2) / 3;
+      } else if (F.t == 2) {
+        count += a * at(2) - at(3);
+      } else {
+        const unsigned long long b = at(2), c = at(4);
+        count += a * b * c - at(3) * c - at(5) * b - at(6) * a + 2 * at(7);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) {
+      H.next = min(H.next + 32, H.end);
+      H.started = H.next;
+    }
+    __syncwarp();
+  }
+
+  // ---- query slots -------------------------------------------------------------
+
+  __device__ void load_plan(int s) {
+    if (W.slot == s) return;
+    flush();
+    const int32_t *srcw = reinterpret_cast<const int32_t *>(&tab->plan[s]);
+    int32_t *dstw = reinterpret_cast<int32_t *>(&W.plan);
+    for (int t = lane; t < (int)(sizeof(FlatPlan) / 4); t += 32) dstw[t] = __ldcg(srcw + t);
+    __syncwarp();
+    if (lane == 0) {
+      W.slot = s;
+      const int levels = max(1, (int)W.plan.s - 1);  // levels 2..s
+      W.cap = (cfg.entries / levels) & ~31;
+    }
+    __syncwarp();
+  }
+
+  // Add this warp's count to its slot's: through shared memory for the slot
+  // most warps of the CTA started with, so a launch of one slot does one
+  // atomic per CTA and not per warp on it.
+  __device__ void flush() {
+    unsigned long long c = count;
+    count = 0;
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) c += __shfl_xor_sync(kFull, c, d);
+    if (lane == 0 && c) {
+      if (W.slot == C.slot) atomicAdd(&C.sum, c);
+      else atomicAdd(&tab->hot[W.slot].count, c);
+    }
+    __syncwarp();
+  }
+
+  // Ticket t of slot s: its edges that pass get_job's filter
+  // (src/gpu_match.cu:531-556) become level-1 entries.
+  __device__ bool fetch_chunk(int s, long long t) {
+    const SlotInfo &in = tab->info[s];
+    const FlatPlan &F = W.plan;
+    const int chunk = __ldcg(&in.chunk);
+    const int64_t e = __ldcg(&in.e_begin) + (t * __ldcg(&in.stride) + __ldcg(&in.phase)) * (int64_t)chunk + lane;
+    bool ok = lane < chunk && e < __ldcg(&in.e_end);
+    int32_t r = 0, c = 0;
+    if (ok) {
+      const int64_t ed = __ldcg(&in.perm) ? (int64_t)G.lperm[e] : e;
+      r = G.src[ed];
+      c = G.colidx[ed];
+      if (!LAB && F.orient && !(r < c)) ok = false;
+      if (LAB && ok && ((int32_t)G.label[r] != F.label[0] || (int32_t)G.label[c] != F.label[1])) ok = false;
+      if (ok && (G.rowptr[r + 1] - G.rowptr[r] < F.deg[0] || G.rowptr[c + 1] - G.rowptr[c] < F.deg[1] ||
+                 G.maxnd[c] < F.deg[2]))
+        ok = false;
+    }
+    const unsigned mask = __ballot_sync(kFull, ok);
+    if (!mask) return false;
+    if (ok) {
+      const int at = __popc(mask & lanemask_lt());
+      W.er[at] = r;
+      W.ec[at] = c;
+    }
+    install(1, __popc(mask));
+    return true;
+  }
+
+  // Entries [0, n) of level l become this warp's base work.
+  __device__ void install(int l, int n) {
+    if (lane == 0) {
+      for (int j = 1; j <= l; ++j) {
+        FlatLevel &H = W.lev[j];
+        H.next = H.end = H.started = 0;
+        H.pos = 0;
+        H.cutp = -1;
+        H.groups = 0;
+      }
+      W.lev[l].end = W.lev[l].n = n;
+      W.t_work = now_ns();
+    }
+    __syncwarp();
+  }
+
+  // Take over ticket t of the launch: find its slot and fetch its edges.
+  // Tickets ascend, so the search starts at the slot of the last one.
+  __device__ bool start_ticket(long long t, int &hint) {
+    const int n = tab->ctl.slots;
+    int s = hint;
+    for (;; s += 31) {
+      // the last slot that starts at or before t; slots in [s, s + 32) at a time
+      const bool le = s + lane < n && __ldcg(&tab->info[s + lane].ticket0) <= t;
+      const int c = __popc(__ballot_sync(kFull, le));
+      if (c < 32) {
+        s += c - 1;
+        break;
+      }
+    }
+    hint = s;
+    load_plan(s);
+    return fetch_chunk(s, t - __ldcg(&tab->info[s].ticket0));
+  }
+
+  // The next ticket that yields edges; false when none is left.
+  __device__ bool next_ticket(int &hint) {
+    for (;;) {
+      long long t = 0;
+      if (lane == 0) t = (long long)atomicAdd(&tab->ctl.ticket, 1ull);
+      t = __shfl_sync(kFull, t, 0);
+      if (t >= tab->ctl.tickets) return false;
+      if (start_ticket(t, hint)) return true;
+    }
+  }
+
+  // ---- giving work away -------------------------------------------------------
+
+  // Give up to half of the untouched entries of the shallowest level that has
+  // some to idle warps, if there are any.
+  __device__ void donate(int base, int level) {
+    const int words = ((int)gridDim.x * (int)(blockDim.x >> 5) + 31) >> 5;
+    int l = base, take = 0;
+    for (; l <= level; ++l) {
+      const FlatLevel &H = W.lev[l];
+      const int avail = H.end - (H.pos ? H.started : H.next);
+      const bool other = l < level || H.pos;  // work stays here besides these entries
+      take = other ? (avail + 1) >> 1 : avail >> 1;
+      if (take > 0) break;
+    }
+    if (l > level) return;
+    // 32 words of the idle mask, another part of it each time
+    const int w = (int)(((unsigned)(clock64() >> 6) + (unsigned)(gid * 7 + lane)) % (unsigned)words);
+    const unsigned idle = *(volatile unsigned *)&sh->idle[w];
+    unsigned have = __ballot_sync(kFull, idle != 0 && lane < words);
+    if (!have) return;
+    bool mine = idle != 0 && lane < words && __popc(have & lanemask_lt()) < take;
+    int target = 0;
+    if (mine) {
+      const int r = (gid + lane) & 31;  // start at another bit than other warps
+      const unsigned rot = __funnelshift_r(idle, idle, r);
+      const unsigned bit = 1u << ((__ffs(rot) - 1 + r) & 31);
+      mine = (atomicAnd(&sh->idle[w], ~bit) & bit) != 0;
+      target = w * 32 + __ffs(bit) - 1;
+    }
+    have = __ballot_sync(kFull, mine);
+    const int boxes = __popc(have);
+    if (!boxes) return;
+    // entries [from, end) of level l, `per` to a box
+    const int per = min(min(32, kUnitInts / (l + 1)), (take + boxes - 1) / boxes);
+    take = min(take, per * boxes);
+    const int used = (take + per - 1) / per;
+    const int rank = __popc(have & lanemask_lt());
+    if (mine) W.cnt[0][rank] = (uint32_t)target;
+    if (lane == 0) atomicAdd(&tab->ctl.pending, used);
+    __syncwarp();
+    const int from = W.lev[l].end - take;
+    for (int t = lane; t < take; t += 32) {
+      int32_t *v = sh->box[W.cnt[0][t / per]].v + (t % per) * (l + 1);
+      int q = from + t;
+      for (int j = l; j >= 2; --j) {
+        v[j] = xs(j)[q];
+        q = ps(j)[q];
+      }
+      v[0] = W.er[q];
+      v[1] = W.ec[q];
+    }
+    const bool fill = mine && rank < used;
+    if (fill) {
+      FlatBox &b = sh->box[target];
+      b.level = l;
+      b.n = min(per, take - rank * per);
+      b.slot = W.slot;
+    }
+    __threadfence();
+    __syncwarp();
+    if (fill) *(volatile int32_t *)&sh->box[target].full = 1;
+    else if (mine) atomicOr(&sh->idle[target >> 5], 1u << (target & 31));  // claimed but not needed
+    if (lane == 0) {
+      W.lev[l].end = from;
+      atomicAdd(&ctl->splits, (unsigned long long)used);
+    }
+    __syncwarp();
+  }
+
+  // Take over the entries in this warp's mailbox; returns their level.
+  __device__ int open_box() {
+    __threadfence();
+    const int l = __ldcg(&box.level), n = __ldcg(&box.n);
+    load_plan(__ldcg(&box.slot));
+    if (lane < n) {
+      const int32_t *v = box.v + lane * (l + 1);
+      W.er[lane] = __ldcg(v);
+      W.ec[lane] = __ldcg(v + 1);
+      for (int j = 2; j <= l; ++j) {
+        xs(j)[lane] = __ldcg(v + j);
+        ps(j)[lane] = (uint16_t)lane;
+      }
+    }
+    install(l, n);
+    return l;
+  }
+
+  // Wait until this warp is given work (returns its level, installed) or none
+  // will come (0).  A waiting warp reads its own mailbox; one per CTA also
+  // reads the count of what is pending.  Bounded: after cfg.idle_ms the
+  // launch reports a timeout.
+  __device__ int wait_for_work() {
+    int st = 0;  // 1: the mailbox is full, 2: stop
+    const unsigned long long t0 = now_ns();
+    flush();
+    if (lane == 0) {
+      *(volatile int32_t *)&box.full = 0;
+      __threadfence();
+      atomicOr(&sh->idle[gid >> 5], 1u << (gid & 31));
+      if (atomicSub(&C.active, 1) == 1 && atomicSub(&tab->ctl.pending, 1) == 1) {
+        ctl->finished = 1;
+        *(volatile int32_t *)&C.done = 1;
+      }
+    }
+    bool poller = false;
+    unsigned nap = 200;
+    for (;;) {
+      if (lane == 0) {
+        if (*(volatile int32_t *)&box.full) st = 1;
+        else if (*(volatile int32_t *)&C.done) st = 2;
+        else if (poller || (poller = atomicCAS(&C.poll, 0, 1) == 0)) {
+          if (*(volatile int32_t *)&tab->ctl.pending <= 0) {
+            *(volatile int32_t *)&C.done = 1;
+            st = 2;
+          }
+        }
+        if (!st && now_ns() - t0 > (unsigned long long)cfg.idle_ms * 1000000ull) {
+          atomicCAS(&ctl->error, 0, TDFS_ERR_TIMEOUT);
+          st = 2;
+        }
+      }
+      st = __shfl_sync(kFull, st, 0);
+      if (st) break;
+      __nanosleep(nap);
+      nap = min(2 * nap, 1600u);
+    }
+    if (lane == 0) {
+      if (poller) atomicExch(&C.poll, 0);
+      // the mailbox's place in `pending` becomes the CTA's when it had no busy warp
+      if (st == 1 && atomicAdd(&C.active, 1) > 0) atomicSub(&tab->ctl.pending, 1);
+      W.idle_total += now_ns() - t0;
+    }
+    __syncwarp();
+    return st == 1 ? open_box() : 0;
+  }
+
+  // Level l extends its entries into level l + 1, the level s counts.  `base`
+  // is the level whose entries this warp was given; below it the warp takes
+  // the next ticket or waits to be given some.
+  __device__ void run() {
+    if (lane == 0) {
+      W.t_start = now_ns();
+      W.slot = -1;
+      W.idle_total = 0;
+    }
+    __syncwarp();
+    int level = 0, base = 1, hint = 0;
+    bool dry = false, more = false;
+    long long checked = clock64();
+    // the host dealt the first tickets, one per warp
+    if (gid < tab->ctl.tickets && start_ticket(gid, hint)) level = 1;
+    for (;;) {
+      if (level < base) {
+        level = 0;
+        if (!dry) {
+          if (next_ticket(hint)) level = base = 1;
+          else dry = true;
+        }
+        if (!level) {
+          level = base = wait_for_work();
+          if (!level) break;
+        }
+        continue;
+      }
+      const FlatLevel &H = W.lev[level];
+      if (H.next >= H.end && !more) {
+        --level;
+        continue;
+      }
+      if (level == W.plan.s) {
+        leaf(level);
+      } else {
+        more = expand(level, more);
+        if (!more && W.lev[level + 1].n > 0) ++level;
+      }
+      const long long c = clock64();
+      int due = 0;
+      if (c - checked > kCheckCycles) {
+        checked = c;
+        due = now_ns() - W.t_work >= (unsigned long long)cfg.split_ns;
+      }
+      if (__shfl_sync(kFull, due, 0)) donate(base, level);
+    }
+    // the CTA's sums, by its last warp
+    if (lane == 0) {
+      atomicAdd(&C.idle_ns, W.idle_total);
+      atomicAdd(&C.warp_ns, now_ns() - W.t_start);
+      __threadfence_block();
+      if (atomicSub(&C.left, 1) == 1) {
+        __threadfence_block();
+        if (C.sum) atomicAdd(&tab->hot[C.slot].count, C.sum);
+        atomicAdd(&ctl->idle_ns, C.idle_ns);
+        atomicAdd(&ctl->warp_ns, C.warp_ns);
+      }
+    }
+  }
+};
+
+template <bool LAB>
+__global__ void __launch_bounds__(256, 4) flat_kernel(const __grid_constant__ DevGraph G,
+                                                      const __grid_constant__ FlatCfg cfg, RunCtl *ctl,
+                                                      SlotTable *tab, FlatShared *sh) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ FlatCta cta;
+  if (threadIdx.x == 0) {
+    cta.poll = cta.done = 0;
+    cta.active = cta.left = (int)(blockDim.x >> 5);
+    cta.slot = 0;
+    cta.sum = cta.idle_ns = cta.warp_ns = 0;
+  }
+  __syncthreads();
+  const int me = threadIdx.x >> 5;
+  unsigned char *base = smem + (size_t)me * cfg.warp_bytes;
+  FlatSmem &W = *reinterpret_cast<FlatSmem *>(base);
+  Flat<LAB> f(G, cfg, ctl, tab, sh, (int)blockIdx.x * (int)(blockDim.x >> 5) + me, W, cta, base + sizeof(FlatSmem));
+  f.run();
+}
+
+__global__ void flat_init_kernel(RunCtl *ctl, FlatShared *sh) {
+  for (int i = threadIdx.x; i < (int)(sizeof(RunCtl) / 4); i += blockDim.x) reinterpret_cast<int32_t *>(ctl)[i] = 0;
+  for (int i = threadIdx.x; i < kIdleWords; i += blockDim.x) sh->idle[i] = 0;
+}
+
+template <bool LAB>
+cudaError_t flat_smem(size_t smem) {
+  static std::mutex mu;
+  static size_t set_to[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lk(mu);
+  if (smem <= set_to[dev]) return cudaSuccess;
+  e = cudaFuncSetAttribute(flat_kernel<LAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) set_to[dev] = smem;
+  return e;
+}
+
+}  // namespace
+
+size_t flat_warp_bytes(int entries) {
+  return (sizeof(FlatSmem) + (size_t)entries * 6 + 15) & ~(size_t)15;
+}
+
+int flat_auto_entries() {
+  constexpr int kPerWarp = (228 * 1024 / 4 - 1024 - 128) / 8 & ~15;  // 4 CTAs of 8 warps on 228 KB, 1 KB per CTA reserved
+  static_assert(kPerWarp > (int)sizeof(FlatSmem) + 5 * 64 * 6, "room for 64 entries of every level");
+  return (kPerWarp - (int)sizeof(FlatSmem)) / 6 & ~31;
+}
+
+int flat_max_entries(int warps) { return (227 * 1024 / warps - 48 - (int)sizeof(FlatSmem)) / 6 & ~31; }
+
+int flat_blocks_per_sm(bool labeled, int warps_per_block, size_t smem) {
+  int n = 0;
+  cudaError_t e = labeled ? flat_smem<true>(smem) : flat_smem<false>(smem);
+  if (e == cudaSuccess)
+    e = labeled
+            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flat_kernel<true>, warps_per_block * 32, smem)
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flat_kernel<false>, warps_per_block * 32, smem);
+  return e == cudaSuccess ? n : -1;
+}
+
+int flat_max_blocks(int warps_per_block) { return kBoxes / warps_per_block; }
+
+void init_flat(RunCtl *ctl, SplitUnit *units, cudaStream_t stream) {
+  flat_init_kernel<<<1, 256, 0, stream>>>(ctl, reinterpret_cast<FlatShared *>(units));
+}
+
+int launch_flat(bool labeled, const DevGraph &g, RunCtl *ctl, SlotTable *tab, SplitUnit *units, const FlatCfg &cfg,
+                int blocks, int warps_per_block, cudaStream_t stream) {
+  FlatShared *sh = reinterpret_cast<FlatShared *>(units);
+  const size_t smem = (size_t)cfg.warp_bytes * warps_per_block;
+  const cudaError_t a = labeled ? flat_smem<true>(smem) : flat_smem<false>(smem);
+  if (a != cudaSuccess) return fail(TDFS_ERR_CUDA, "flat kernel shared memory: %s", cudaGetErrorString(a));
+  (void)cudaGetLastError();  // the check below must see this launch's error only
+  const dim3 grid(blocks), block(warps_per_block * 32);
+  if (labeled) flat_kernel<true><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, sh);
+  else flat_kernel<false><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, sh);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(TDFS_ERR_CUDA, "flat kernel launch: %s", cudaGetErrorString(e));
+  return TDFS_OK;
+}
+
+}  // namespace tdfs

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "csr.h"
+#include "flat.cuh"
 #include "graph.h"
 
 namespace tdfs {
@@ -61,6 +62,26 @@ __global__ void narrow_labels_kernel(const int32_t *__restrict__ in, int32_t n, 
     const int32_t l = in[i];
     if (l < 0 || l > 254) atomicExch(bad, 1);
     out[i] = (uint8_t)(l < 0 || l > 254 ? 255 : l);
+  }
+}
+
+// One thread per edge: the neighbour into its row's membership table
+// (row_table_buckets).  A slot is tried only when the ones before it in the
+// bucket are taken, so entries fill a bucket in order whatever the order of
+// the threads.  Bound by the rate of the atomics in L2: 6M edges take 0.3 ms.
+__global__ void row_table_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
+                                 const int32_t *__restrict__ src, int64_t nedges, int32_t *__restrict__ hash) {
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nedges; j += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t v = src[j], x = colidx[j];
+    const int64_t r = rowptr[v], e = rowptr[v + 1];
+    const uint32_t nb = (uint32_t)(e / 3 - r / 3) + 1;
+    int32_t *t = hash + kBucket * (r / 3 + v);
+    uint32_t b = __umulhi((uint32_t)x * kRowHash, nb);
+    bool placed = false;
+    for (uint32_t tries = 0; tries < nb && !placed; ++tries) {
+      for (int i = 0; i < kBucket && !placed; ++i) placed = atomicCAS(t + kBucket * (int64_t)b + i, -1, x) == -1;
+      b = b + 1 == nb ? 0 : b + 1;
+    }
   }
 }
 
@@ -232,6 +253,18 @@ int cuda_fail(cudaError_t e, const char *what) {
 }
 
 }  // namespace
+
+int build_row_tables(const int64_t *rowptr, const int32_t *colidx, const int32_t *src, int64_t n, int64_t nedges,
+                     int32_t *hash, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(hash, 0xff, 4 * kBucket * (size_t)row_table_buckets(n, nedges), st);
+  if (e == cudaSuccess && nedges > 0) {
+    (void)cudaGetLastError();  // the check below must see this launch's error only
+    const int blocks = (int)std::min<int64_t>((nedges + 255) / 256, 148 * 32);
+    row_table_kernel<<<blocks, 256, 0, st>>>(rowptr, colidx, src, nedges, hash);
+    e = cudaGetLastError();
+  }
+  return e == cudaSuccess ? TDFS_OK : cuda_fail(e, "row membership tables");
+}
 
 // Derived per-graph arrays into caller-provided device memory, no allocation:
 // edge -> source, neighbour-degree maxima and (when labels is not null) 8-bit
@@ -533,6 +566,7 @@ void build_label_arrays(int64_t n, int64_t nedges, const int64_t *rowptr, const 
 // 256-byte boundary:
 //   rowptr int64[n+1] | colidx int32[E + kColPad] | src int32[E] | maxnd int32[n]
 //   | label uint8[n] | lperm int32[E] | colidx_l int32[E + kColPad] | loff int32[n (nlab+1)]
+//   | scratch of the label index sort | row membership tables
 // The parts from `label` on are derived on the host into one pinned staging
 // block laid out the same way and uploaded with one copy.  The CSR copies and
 // the two preprocessing kernels are queued first, so the device works while
@@ -575,9 +609,18 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   const size_t o_hist = o_loff + align256(sizeof(int32_t) * (nloff ? nloff : 1));
   const size_t o_goff = o_hist + align256(sizeof(int32_t) * (size_t)(dev_build && ntiles ? (int64_t)G * ntiles : 1));
   const size_t total = dev_build ? o_goff + align256(sizeof(int64_t) * (size_t)(G + 1)) : o_hist;
+  // the row membership tables, where the flat kernel can use them and the
+  // device has room; without them every plan runs on the DFS kernel
+  const int64_t buckets = row_table_buckets(n, nedges);
+  size_t hash_bytes = buckets <= (int64_t)UINT32_MAX && max_degree <= kFlatMaxDegree ? 4 * kBucket * (size_t)buckets : 0;
   void *arrays = nullptr, *stage = nullptr;
   size_t array_bytes = 0, stage_bytes = 0;
-  e = device_blocks().take(device, total, &arrays, &array_bytes);
+  e = device_blocks().take(device, total + hash_bytes, &arrays, &array_bytes);
+  if (e == cudaErrorMemoryAllocation && hash_bytes) {
+    (void)cudaGetLastError();
+    hash_bytes = 0;
+    e = device_blocks().take(device, total, &arrays, &array_bytes);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "graph arrays");
   if (labels) {
     e = pinned_blocks().take(device, dev_build ? (size_t)std::max<int64_t>(n, 1) : total - o_label, &stage,
@@ -608,7 +651,8 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   g->colidx_l = nlab ? reinterpret_cast<int32_t *>(base + o_coll) : nullptr;
   g->loff = nlab ? reinterpret_cast<int32_t *>(base + o_loff) : nullptr;
   g->nlab = nlab;
-  g->bytes = dev_build ? o_hist : total;  // the scratch is not part of the graph
+  g->hash = hash_bytes ? reinterpret_cast<int32_t *>(base + total) : nullptr;
+  g->bytes = (dev_build ? o_hist : total) + hash_bytes;  // the scratch is not part of the graph
   const cudaStream_t st = cudaStreamPerThread;
   e = cudaMemcpyAsync(g->rowptr, rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && nedges)
@@ -623,6 +667,9 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     max_nbr_deg_kernel<<<blocks, threads, 0, st>>>(g->rowptr, g->colidx, (int32_t)n, g->maxnd);
     e = cudaGetLastError();
   }
+  if (e == cudaSuccess && g->hash &&
+      build_row_tables(g->rowptr, g->colidx, g->src, n, nedges, g->hash, st) != TDFS_OK)
+    e = cudaErrorUnknown;
   std::unique_ptr<LabelIndex> lindex;
   if (e == cudaSuccess && labels) {
     char *h = static_cast<char *>(stage);
@@ -738,6 +785,7 @@ DevGraph graph_view(const tdfs_graph *g) {
   v.lperm = g->lperm;
   v.colidx_l = g->colidx_l;
   v.loff = g->loff;
+  v.hash = g->hash;
   v.nlab = g->nlab;
   v.nedges = g->nedges;
   v.n = (int32_t)g->n;

@@ -72,6 +72,7 @@ struct SlotInfo {
   int32_t chunk;     // directed edges per ticket (1, 2, 4, ..., 32)
   int32_t perm;      // 1: level-0 positions index DevGraph::lperm (labeled plans)
   int64_t budget;    // work units this query may spend (0 = unlimited)
+  int64_t ticket0;   // flat kernel: the launch's tickets before this slot's
 };
 
 struct alignas(128) SlotCtl {
@@ -81,16 +82,23 @@ struct alignas(128) SlotCtl {
   char pad1_[120];
   int32_t shutdown;              // host: 1 = no further admissions this launch
   int32_t idle_exit_ms;          // serving: retire after this long with no work
-  char pad2_[120];
+  int32_t slots;                 // host, flat kernel: slots of the launch
+  char pad2_[116];
   unsigned long long first_open; // device hint: slots below this have no tickets left
   char pad3_[120];
+  // flat kernel: tickets run over all slots in order (SlotInfo::ticket0)
+  unsigned long long ticket;     // the next one; the host deals the first ones, one per warp
+  long long tickets;             // host: tickets of all slots
+  char pad4_[112];
+  int32_t pending;               // CTAs with busy warps + units in the ring; 0 = the launch is complete
+  char pad5_[124];
 };
 
 struct SlotTable {
   SlotCtl ctl;
   SlotHot hot[kMaxSlots];
   SlotInfo info[kMaxSlots];
-  DevPlan plan[kMaxSlots];
+  DevPlan plan[kMaxSlots];  // or the FlatPlan of launches of the flat kernel
 };
 
 }  // namespace tdfs
@@ -158,6 +166,7 @@ struct tdfs_graph {
   int32_t *colidx_l;      // label-partitioned rows (labeled graphs with <= kSegLabels labels)
   int32_t *loff;          //   and their segment starts per vertex and label
   int32_t nlab;
+  int32_t *hash;          // row membership tables, or nullptr when they did not fit in device memory
   tdfs::LabelIndex *lindex;  // its host copy and group offsets
   size_t array_bytes;     // size of the `arrays` block (cached for reuse when the graph is freed)
   void *staging;          // pinned host block: the derived arrays as uploaded (labeled graphs)
@@ -183,6 +192,10 @@ void graph_release(tdfs_graph *g);
 int acquire_workspace(tdfs_graph *g);
 void release_graphs(tdfs_graph *g);  // capi.cpp: destroys cached launch graphs
 DevGraph graph_view(const tdfs_graph *g);
+// Row membership tables (common.h, row_table_buckets) of a graph whose `src`
+// array is built, into `hash`; stream-ordered.
+int build_row_tables(const int64_t *rowptr, const int32_t *colidx, const int32_t *src, int64_t n, int64_t nedges,
+                     int32_t *hash, cudaStream_t st);
 int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, const int32_t *labels,
                          int32_t *src, int32_t *maxnd, uint8_t *label8, int32_t *bad, cudaStream_t st);
 inline QueueHdr *queue_hdr(tdfs_graph *g) { return reinterpret_cast<QueueHdr *>(g->queue + kQueueCap); }

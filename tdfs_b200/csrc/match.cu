@@ -1853,6 +1853,7 @@ __global__ void init_kernel(RunCtl *ctl, QueueHdr *qh) {
     ctl->idle_ns = 0;
     ctl->warp_ns = 0;
     ctl->error = 0;
+    ctl->finished = 0;
     qh->head = 0;
     qh->tail = 0;
   }

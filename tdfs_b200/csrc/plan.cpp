@@ -295,7 +295,26 @@ std::string HostPlan::dump_json() const {
   o << ", \"conditions\": [";
   for (size_t c = 0; c < conditions.size(); ++c)
     o << (c ? ", [" : "[") << conditions[c].first << ", " << conditions[c].second << "]";
-  o << "]}";
+  o << "]";
+  FlatPlan f;
+  if (flat_plan(to_device(), &f)) {
+    // the flat kernel's form: sets as [bn, label, larger, less, neq, dep, bnsh]
+    auto set = [](const FlatStep &st) {
+      std::string s = "[[";
+      for (int t = 0; t < st.nbn; ++t) s += (t ? ", " : "") + std::to_string(st.bn[t]);
+      s += "]";
+      for (int v : {st.label, st.larger, st.less, st.neq, st.dep}) s += ", " + std::to_string(v);
+      s += ", [";
+      for (int t = 0; t < st.nsh; ++t) s += (t ? ", " : "") + std::to_string(st.bnsh[t]);
+      return s + "]]";
+    };
+    o << ", \"flat\": {\"s\": " << (int)f.s << ", \"t\": " << (int)f.t << ", \"form\": " << (int)f.form;
+    list("term_of", [&](int i) { return (int)f.term_of[i]; }, 8);
+    list("steps", [&](int i) { return set(f.step[i]); }, f.s - 1);
+    list("terms", [&](int i) { return set(f.term[i]); }, f.nterm);
+    o << "}";
+  }
+  o << "}";
   return o.str();
 }
 

@@ -5,6 +5,7 @@
 #include <cstdint>
 
 #include "common.h"
+#include "flat.cuh"
 #include "graph.h"
 #include "match.cuh"
 
@@ -22,8 +23,24 @@ int launch_shape(const tdfs_graph *g, int kmax, bool labeled, const tdfs_options
 // label index for labeled plans when use_index is set (capi.cpp).
 void level0_range(const tdfs_graph *g, const DevPlan &p, int64_t eb, int64_t ee, bool use_index, SlotInfo *in);
 
-// The device plan table of a compiled pattern (capi.cpp).
+// The device plan table of a compiled pattern, and its form for the flat
+// kernel (nullptr when it has none) (capi.cpp).
 const DevPlan &plan_device_table(const tdfs_plan *p);
+const FlatPlan *plan_flat_table(const tdfs_plan *p);
+
+// Launch shape of the flat kernel for plans enumerated down to level smax
+// (FlatPlan::s), from the options launch_shape has accepted (capi.cpp).
+struct FlatShape {
+  int warps_per_block;
+  int blocks;
+  FlatCfg cfg;
+};
+int flat_shape(int device, int smax, bool labeled, const tdfs_options &o, FlatShape *out);
+
+// Do these options leave the choice of the kernel to the library?  A work
+// budget, stealing switched off, or a value for one of the DFS kernel's own
+// knobs asks for the DFS kernel.
+bool flat_options(const tdfs_options &o);
 
 struct Server;
 size_t query_bytes(int k, int cap, int warps_per_block);

@@ -1,0 +1,100 @@
+"""The flat kernel at the sizes where it can go wrong: buffers that refill after
+every step, single-warp CTAs, one ticket per edge, work given away at once,
+hub rows whose membership tables overflow buckets, rows of 0, 1, 7, 8 and 9
+entries (the bucket size), self-loops, one-directional rows, label segments
+and whole rows with labels, more labels than segments.  Counts are exact and
+equal the oracle's."""
+import random
+
+import numpy as np
+import pytest
+
+from tests.golden.make_golden import random_pattern
+from tests.patterns import CYCLE4, HOUSE, TRIANGLE, clique
+
+pytestmark = pytest.mark.gpu
+
+DIAMOND = "v 0 1\nv 1 1\nv 2 1\nv 3 1\ne 0 1 1\ne 0 2 1\ne 0 3 1\ne 1 2 1\ne 1 3 1\n"
+
+
+def csr(edges, n):
+    rows = [[] for _ in range(n)]
+    for a, b in sorted(edges):
+        rows[a].append(b)
+    return (np.array([0] + list(np.cumsum([len(r) for r in rows])), np.int64),
+            np.array([x for r in rows for x in r], np.int32))
+
+
+def edge_graph():
+    """Rows of 0..9 entries, two hubs adjacent to most vertices, self-loops and
+    some one-directional edges."""
+    n, rng, e = 900, random.Random(5), set()
+    for v in range(2, n):
+        for w in rng.sample(range(2, n), v % 10):
+            e.add((v, w))
+            if v % 3:
+                e.add((w, v))
+    for v in range(2, n - 20):
+        e |= {(0, v), (v, 0)}
+        if v % 2:
+            e |= {(1, v), (v, 1)}
+    e |= {(0, 1), (1, 0)} | {(v, v) for v in range(0, n, 7)}
+    e = {(a, b) for a, b in e if a < n - 3}  # three empty rows
+    return csr(e, n)
+
+
+OPTIONS = [{}, {"chunk_cap": 64, "split_after_us": -1}, {"warps_per_block": 1, "blocks_per_sm": 1},
+           {"edge_chunk": 1, "split_after_us": 1}, {"edge_chunk": 32, "warps_per_block": 3}, {"label_rows": -1},
+           {"label_index": -1, "chunk_cap": 96}, {"graph_capture": 1}]
+
+
+@pytest.fixture(scope="module")
+def cases(T, po):
+    rowptr, colidx = edge_graph()
+    rng = random.Random(8)
+    out = []
+    for nlabels in (3, 20):  # label segments; more labels than segments
+        labels = np.array([rng.randrange(nlabels) % 5 if nlabels > 16 else rng.randrange(nlabels)
+                           for _ in range(len(rowptr) - 1)], np.int32)
+        labels[0] = nlabels - 1
+        out.append((T.GraphPreprocessor(rowptr=rowptr, colidx=colidx, labels=labels, labeled=True),
+                    po.Graph(rowptr.copy(), colidx.copy(), labels.copy()), nlabels))
+    return out
+
+
+@pytest.mark.parametrize("opt", OPTIONS)
+def test_edges_of_the_flat_kernel(T, po, cases, opt):
+    rng = random.Random(4)
+    texts = [(t, False) for t in (TRIANGLE, CYCLE4, DIAMOND, clique(4), clique(5))]
+    texts += [(random_pattern(3 + i % 4, 0.3 + 0.1 * (i % 3), 3, rng), True) for i in range(12)]
+    for dev, ora, nlabels in cases:
+        for text, labeled in texts:
+            if nlabels > 16 and not labeled:
+                continue
+            P = T.PatternPreprocessor(text=text, labeled=labeled)
+            got = T.count(dev, P, T.default_options(**opt)).count
+            assert got == po.count(ora, po.Plan(text, labeled)), (nlabels, text, labeled, opt)
+
+
+@pytest.mark.parametrize("n", [1, 33, 200])
+def test_many_plans_in_one_launch(T, cases, n):
+    """Tickets run over all slots of a launch (a warp finds a ticket's slot 32 at
+    a time); slots without tickets lie between the others."""
+    dev, _, _ = cases[0]
+    rng = random.Random(n)
+    plans = [T.PatternPreprocessor(text=random_pattern(3 + i % 3, 0.5, 4, rng), labeled=True) for i in range(n)]
+    assert T.count_batch(dev, plans)[0] == [T.count(dev, p).count for p in plans]
+
+
+def test_flat_and_dfs_kernels_agree_on_a_power_law_graph(T):
+    g = T.gen_chung_lu(30000, 90000, 2.1, 2500, 3).set_labels(3, 1)
+    dev = T.GraphPreprocessor(csr=g, labeled=True)
+    rng = random.Random(2)
+    texts = [(t, False) for t in (TRIANGLE, CYCLE4, DIAMOND, clique(4), clique(5))]
+    texts += [(random_pattern(4 + i % 2, 0.6, 3, rng), True) for i in range(4)]
+    for text, labeled in texts:
+        P = T.PatternPreprocessor(text=text, labeled=labeled)
+        want = T.count(dev, P, T.default_options(tail_count=1)).count  # a DFS kernel knob: that kernel
+        assert T.count(dev, P).count == want
+        shards = [T.count(dev, P, T.shard_options(r, 3)).count for r in range(3)]
+        assert sum(shards) == want
