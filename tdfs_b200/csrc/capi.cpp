@@ -251,38 +251,45 @@ std::vector<GraphEntry> &graph_cache(tdfs_graph *g) {
   return *static_cast<std::vector<GraphEntry> *>(g->graphs);
 }
 
-void reset_launch(tdfs_graph *g, const Launch &L, cudaStream_t st) {
-  if (L.flat) init_flat(g->ctl, g->queue, st);
-  else init_launch(g->ctl, queue_hdr(g), st);
+// The workspace as a launch of the flat kernel uses it: its records where the
+// slot table is, the mailboxes in the split ring's memory.
+static_assert(kFlatBoxBytes <= sizeof(SplitUnit) * kQueueCap, "the mailboxes fit the split ring");
+FlatTable flat_table(const tdfs_graph *g, int n) {
+  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue));
 }
 
-int enqueue_kernel(tdfs_graph *g, const Launch &L, bool labeled, cudaStream_t st) {
-  if (L.flat)
-    return launch_flat(labeled, graph_view(g), g->ctl, g->tab, g->queue, L.fl.cfg, L.fl.blocks,
-                       L.fl.warps_per_block, st);
-  return launch_match(labeled, graph_view(g), g->ctl, g->tab, g->queue, queue_hdr(g), L.dfs.cfg, L.dfs.blocks,
-                      L.dfs.warps_per_block, st);
-}
-
+// Upload, kernel (between the events k0 and k1, when given) and read-back.
+// Captured launches record the events as external ones, so that they time the
+// kernel when the graph replays (a plain record is only a join point).
 int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStream_t st, cudaEvent_t k0,
-                   cudaEvent_t k1) {
+                   cudaEvent_t k1, unsigned flags) {
   SlotTable *h = g->htab, *d = g->tab;
-  cudaError_t e = cudaMemcpyAsync(&d->ctl, &h->ctl, sizeof h->ctl, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->hot, h->hot, sizeof(SlotHot) * n, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->info, h->info, sizeof(SlotInfo) * n, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->plan, h->plan, sizeof(DevPlan) * n, cudaMemcpyHostToDevice, st);
+  cudaError_t e;
+  if (L.flat) {
+    e = cudaMemcpyAsync(d, h, FlatTable::bytes(n), cudaMemcpyHostToDevice, st);
+  } else {
+    e = cudaMemcpyAsync(&d->ctl, &h->ctl, sizeof h->ctl, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d->hot, h->hot, sizeof(SlotHot) * n, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d->info, h->info, sizeof(SlotInfo) * n, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d->plan, h->plan, sizeof(DevPlan) * n, cudaMemcpyHostToDevice, st);
+  }
   if (e != cudaSuccess) return cuda_err(e, "slot table upload");
-  reset_launch(g, L, st);
-  // external records: captured as event-record nodes, so they time the
-  // kernel when the graph replays (a plain record is only a join point)
-  e = cudaEventRecordWithFlags(k0, st, cudaEventRecordExternal);
+  if (!L.flat) init_launch(g->ctl, queue_hdr(g), st);
+  if (k0) e = cudaEventRecordWithFlags(k0, st, flags);
   if (e != cudaSuccess) return cuda_err(e, "kernel start event");
-  int rc = enqueue_kernel(g, L, labeled, st);
+  const int rc =
+      L.flat ? launch_flat(labeled, graph_view(g), flat_table(g, n), L.fl.cfg, L.fl.blocks, L.fl.warps_per_block, st)
+             : launch_match(labeled, graph_view(g), g->ctl, g->tab, g->queue, queue_hdr(g), L.dfs.cfg, L.dfs.blocks,
+                            L.dfs.warps_per_block, st);
   if (rc) return rc;
-  e = cudaEventRecordWithFlags(k1, st, cudaEventRecordExternal);
+  if (k1) e = cudaEventRecordWithFlags(k1, st, flags);
   if (e != cudaSuccess) return cuda_err(e, "kernel end event");
-  e = cudaMemcpyAsync(h->hot, d->hot, sizeof(SlotHot) * n, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(g->hctl, g->ctl, sizeof(RunCtl), cudaMemcpyDeviceToHost, st);
+  if (L.flat) {
+    e = cudaMemcpyAsync(h, d, FlatTable::readback(n), cudaMemcpyDeviceToHost, st);
+  } else {
+    e = cudaMemcpyAsync(h->hot, d->hot, sizeof(SlotHot) * n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(g->hctl, g->ctl, sizeof(RunCtl), cudaMemcpyDeviceToHost, st);
+  }
   if (e != cudaSuccess) return cuda_err(e, "read-back");
   return TDFS_OK;
 }
@@ -290,13 +297,23 @@ int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStre
 // Counts of a finished launch from the read-back slot lines.  A slot that ran
 // out of its work budget gets status TDFS_ERR_TIMEOUT and count 0; without a
 // status array that fails the call.
-int collect(const RunCtl &hc, const SlotHot *hot, int n, bool flat, unsigned long long *raw, int *status) {
+int collect(tdfs_graph *g, int n, bool flat, unsigned long long *raw, int *status) {
+  if (flat) {
+    const FlatTable t = FlatTable::of(g->htab, n, nullptr);
+    *g->hctl = *t.run;
+    for (int i = 0; i < n; ++i) {
+      raw[i] = t.count[i];
+      if (status) status[i] = TDFS_OK;
+    }
+  }
+  const RunCtl &hc = *g->hctl;
   if (hc.error == TDFS_ERR_TIMEOUT) return fail(TDFS_ERR_TIMEOUT, "a bounded device wait ran out");
   if (hc.error) return fail(hc.error, "device error %d", hc.error);
-  if (flat && !hc.finished) return fail(TDFS_ERR_TIMEOUT, "the launch did not complete");
+  if (flat) return hc.finished ? TDFS_OK : fail(TDFS_ERR_TIMEOUT, "the launch did not complete");
+  const SlotHot *hot = g->htab->hot;
   int first_abort = -1;
   for (int i = 0; i < n; ++i) {
-    if (!flat && hot[i].state != kSlotDone) return fail(TDFS_ERR_TIMEOUT, "slot %d did not complete", i);
+    if (hot[i].state != kSlotDone) return fail(TDFS_ERR_TIMEOUT, "slot %d did not complete", i);
     const bool ab = hot[i].aborted != 0;
     raw[i] = ab ? 0 : hot[i].count;
     if (status) status[i] = ab ? TDFS_ERR_TIMEOUT : TDFS_OK;
@@ -330,7 +347,7 @@ int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms,
     cudaGraph_t graph;
     e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_err(e, "cudaStreamBeginCapture");
-    int rc = enqueue_launch(g, L, labeled, n, st, ent.k0, ent.k1);
+    int rc = enqueue_launch(g, L, labeled, n, st, ent.k0, ent.k1, cudaEventRecordExternal);
     e = cudaStreamEndCapture(st, &graph);
     if (!rc && e == cudaSuccess) {
       e = cudaGraphInstantiate(&ent.exec, graph, 0);
@@ -349,7 +366,57 @@ int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms,
   // the match kernel's own time, from the event nodes around it in the graph
   if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, hit->k0, hit->k1);
   if (e != cudaSuccess) return cuda_err(e, "graph launch");
-  return collect(*g->hctl, g->htab->hot, n, L.flat, raw, status);
+  return collect(g, n, L.flat, raw, status);
+}
+
+// The host image of the slot table for the DFS kernel.
+void fill_slots(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_options &o, int64_t eb, int64_t ee,
+                int stride, int warps) {
+  SlotTable *h = g->htab;
+  std::memset(&h->ctl, 0, sizeof h->ctl);
+  h->ctl.admitted = (unsigned long long)n;
+  h->ctl.shutdown = 1;
+  for (int i = 0; i < n; ++i) {
+    SlotInfo &in = h->info[i];
+    level0_range(g, plans[i]->dev, eb, ee, o.label_index >= 0, &in);
+    in.stride = stride;
+    in.phase = o.edge_phase;
+    in.chunk = auto_chunk(in.e_end - in.e_begin, stride, warps, o.edge_chunk);
+    in.ntickets = ticket_count(in.e_begin, in.e_end, stride, o.edge_phase, in.chunk);
+    in.budget = o.work_budget;
+    std::memset(&h->hot[i], 0, sizeof h->hot[i]);
+    h->hot[i].state = in.ntickets > 0 ? kSlotActive : kSlotDone;  // an empty range is done at once
+    if (in.ntickets == 0) ++h->ctl.completed;
+    h->plan[i] = plans[i]->dev;
+  }
+}
+
+// The host image of the flat kernel's records.
+void fill_flat(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_options &o, int64_t eb, int64_t ee,
+               int stride, const Launch &L) {
+  const FlatTable t = FlatTable::of(g->htab, n, nullptr);
+  std::memset(static_cast<void *>(g->htab), 0, FlatTable::bytes(n) - (size_t)n * sizeof(FlatPlan));
+  t.ctl->ticket = (unsigned long long)L.warps();  // the first ones are dealt one per warp
+  t.ctl->pending = L.fl.blocks;
+  t.ctl->slots = n;
+  int64_t edges = 0;
+  for (int i = 0; i < n; ++i) {
+    SlotInfo in;
+    level0_range(g, plans[i]->dev, eb, ee, o.label_index >= 0, &in);
+    t.info[i].e_begin = in.e_begin;
+    t.info[i].e_end = in.e_end;
+    t.info[i].perm = in.perm;
+    edges += in.e_end - in.e_begin;
+  }
+  for (int i = 0; i < n; ++i) {
+    FlatInfo &in = t.info[i];
+    in.stride = stride;
+    in.phase = o.edge_phase;
+    in.chunk = flat_chunk(edges, plans[i]->flat.s, stride, L.warps(), o.edge_chunk);
+    in.ticket0 = t.ctl->tickets;
+    t.ctl->tickets += ticket_count(in.e_begin, in.e_end, stride, o.edge_phase, in.chunk);
+    t.plan[i] = plans[i]->flat;
+  }
 }
 
 // One launch over n plans of the same mode: slot i counts plans[i] on the
@@ -385,68 +452,26 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
   const int64_t ee = (o.edge_end < 0 || o.edge_end > g->nedges) ? g->nedges : o.edge_end;
   const int stride = o.edge_stride > 0 ? o.edge_stride : 1;
   if (o.edge_phase < 0 || o.edge_phase >= stride) return fail(TDFS_ERR_ARG, "edge_phase must lie in [0, edge_stride)");
-  SlotTable *h = g->htab;
-  std::memset(&h->ctl, 0, sizeof h->ctl);
-  h->ctl.admitted = (unsigned long long)n;
-  h->ctl.shutdown = 1;
   const int warps = L.warps();
-  for (int i = 0; i < n; ++i) {
-    SlotInfo &in = h->info[i];
-    level0_range(g, plans[i]->dev, eb, ee, o.label_index >= 0, &in);
-    in.stride = stride;
-    in.phase = o.edge_phase;
-    in.chunk = auto_chunk(in.e_end - in.e_begin, stride, warps, o.edge_chunk);
-    in.ntickets = ticket_count(in.e_begin, in.e_end, stride, o.edge_phase, in.chunk);
-    in.budget = o.work_budget;
-    std::memset(&h->hot[i], 0, sizeof h->hot[i]);
-    h->hot[i].state = in.ntickets > 0 ? kSlotActive : kSlotDone;  // an empty range is done at once
-    if (in.ntickets == 0) ++h->ctl.completed;
-    if (flat) std::memcpy(&h->plan[i], &plans[i]->flat, sizeof plans[i]->flat);
-    else h->plan[i] = plans[i]->dev;
-  }
-  if (flat) {
-    // tickets run over all slots in order; the first ones are dealt one per
-    // warp, so the warps do not queue for them on one counter
-    for (int i = 0; i < n; ++i) {
-      h->info[i].ticket0 = h->ctl.tickets;
-      h->ctl.tickets += h->info[i].ntickets;
-    }
-    h->ctl.slots = n;
-    h->ctl.ticket = (unsigned long long)warps;
-    h->ctl.pending = L.fl.blocks;
-  }
   g->last_warps = warps;
+  if (flat) fill_flat(g, plans, n, o, eb, ee, stride, L);
+  else fill_slots(g, plans, n, o, eb, ee, stride, warps);
   if (o.graph_capture) return run_captured(g, L, labeled, n, ms, raw, status);
   cudaStream_t st = static_cast<cudaStream_t>(o.stream);
-  SlotTable *d = g->tab;
-  e = cudaMemcpyAsync(&d->ctl, &h->ctl, sizeof h->ctl, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->hot, h->hot, sizeof(SlotHot) * n, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->info, h->info, sizeof(SlotInfo) * n, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->plan, h->plan, sizeof(DevPlan) * n, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return cuda_err(e, "slot table upload");
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  if (ms) {
-    cudaEventCreate(&ev0);
-    cudaEventCreate(&ev1);
-  }
-  reset_launch(g, L, st);
-  if (ms) cudaEventRecord(ev0, st);
-  rc = enqueue_kernel(g, L, labeled, st);
-  if (ms) cudaEventRecord(ev1, st);
-  if (!rc) {
-    e = cudaMemcpyAsync(h->hot, d->hot, sizeof(SlotHot) * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(g->hctl, g->ctl, sizeof(RunCtl), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) rc = cuda_err(e, "match kernel");
-  }
-  if (!rc && ms) {
-    e = cudaEventElapsedTime(ms, ev0, ev1);
-    if (e != cudaSuccess) rc = cuda_err(e, "cudaEventElapsedTime");
-  }
-  if (ev0) cudaEventDestroy(ev0);
-  if (ev1) cudaEventDestroy(ev1);
-  if (rc) return rc;
-  return collect(*g->hctl, h->hot, n, flat, raw, status);
+  if (ms)
+    for (void *&ev : g->ws->ev)
+      if (!ev) {
+        cudaEvent_t x;
+        if ((e = cudaEventCreate(&x)) != cudaSuccess) return cuda_err(e, "cudaEventCreate");
+        ev = x;
+      }
+  const cudaEvent_t k0 = ms ? static_cast<cudaEvent_t>(g->ws->ev[0]) : nullptr;
+  const cudaEvent_t k1 = ms ? static_cast<cudaEvent_t>(g->ws->ev[1]) : nullptr;
+  if ((rc = enqueue_launch(g, L, labeled, n, st, k0, k1, cudaEventRecordDefault))) return rc;
+  e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, k0, k1);
+  if (e != cudaSuccess) return cuda_err(e, "match kernel");
+  return collect(g, n, flat, raw, status);
 }
 
 }  // namespace

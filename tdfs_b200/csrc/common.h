@@ -68,7 +68,6 @@ struct FlatPlan {
   FlatStep step[4];
   FlatStep term[7];
 };
-static_assert(sizeof(FlatPlan) <= sizeof(DevPlan), "a slot's plan record holds either plan");
 
 // The flat form of a plan; false when it has none (flat_plan.cpp).
 bool flat_plan(const DevPlan &d, FlatPlan *out);

@@ -17,9 +17,6 @@ constexpr int kTupleMax = kMaxK - 1;   // phi(0..5): the deepest enumerated leve
 constexpr int kProbeMax = kMaxK - 2;   // lists tested per candidate besides its source
 constexpr int kScanSteps = 64;         // 64-position steps of a leaf scan between two looks at the idle count
 constexpr int kCheckCycles = 16384;    // clocks between those looks
-constexpr int kUnitInts = 156;         // vertices one mailbox carries
-constexpr int kBoxes = 8192;           // mailboxes, one per warp of the grid
-constexpr int kIdleWords = kBoxes / 32;
 
 // Work given away goes straight to an idle warp: each warp has a mailbox and
 // a bit in a grid-wide mask of idle warps.  A busy warp reads 32 words of the
@@ -28,17 +25,6 @@ constexpr int kIdleWords = kBoxes / 32;
 // as they would on a shared ring (which passed 1.2 units per microsecond
 // whatever the demand and left 60-90% of the warps of a power-law launch
 // idle), and an idle warp reads its own line only.
-// A mailbox holds up to 32 partial embeddings (tuples of level + 1 vertices).
-struct FlatBox {
-  int32_t full;  // 0 empty, 1 filled by the warp that cleared the idle bit
-  int32_t level, n, slot;
-  int32_t v[kUnitInts];
-};
-struct FlatShared {
-  FlatBox box[kBoxes];
-  unsigned idle[kIdleWords];
-};
-static_assert(sizeof(FlatShared) <= sizeof(SplitUnit) * kQueueCap, "the mailboxes use the split ring's memory");
 
 struct FlatLevel {
   int32_t next;      // first entry of the block being extended (blocks of 32 entries)
@@ -94,10 +80,7 @@ template <bool LAB>
 struct Flat {
   const DevGraph &G;
   const FlatCfg &cfg;
-  RunCtl *ctl;
-  SlotTable *tab;
-  FlatShared *sh;
-  FlatBox &box;  // this warp's
+  const FlatTable &T;
   const int gid;
   FlatSmem &W;
   FlatCta &C;
@@ -106,9 +89,9 @@ struct Flat {
   unsigned long long count = 0;  // per lane; summed at release
   int lane;
 
-  __device__ Flat(const DevGraph &g, const FlatCfg &c, RunCtl *ct, SlotTable *tb, FlatShared *s, int warp,
-                  FlatSmem &w, FlatCta &cta, unsigned char *bufs)
-      : G(g), cfg(c), ctl(ct), tab(tb), sh(s), box(s->box[warp]), gid(warp), W(w), C(cta), X(reinterpret_cast<int32_t *>(bufs)),
+  __device__ Flat(const DevGraph &g, const FlatCfg &c, const FlatTable &t, int warp, FlatSmem &w, FlatCta &cta,
+                  unsigned char *bufs)
+      : G(g), cfg(c), T(t), gid(warp), W(w), C(cta), X(reinterpret_cast<int32_t *>(bufs)),
         P(reinterpret_cast<uint16_t *>(bufs + (size_t)c.entries * 4)), lane(lane_id()) {}
 
   __device__ __forceinline__ int32_t *xs(int l) const { return X + (l - 2) * W.cap; }
@@ -517,7 +500,7 @@ struct Flat {
   __device__ void load_plan(int s) {
     if (W.slot == s) return;
     flush();
-    const int32_t *srcw = reinterpret_cast<const int32_t *>(&tab->plan[s]);
+    const int32_t *srcw = reinterpret_cast<const int32_t *>(&T.plan[s]);
     int32_t *dstw = reinterpret_cast<int32_t *>(&W.plan);
     for (int t = lane; t < (int)(sizeof(FlatPlan) / 4); t += 32) dstw[t] = __ldcg(srcw + t);
     __syncwarp();
@@ -539,7 +522,7 @@ struct Flat {
     for (int d = 16; d >= 1; d >>= 1) c += __shfl_xor_sync(kFull, c, d);
     if (lane == 0 && c) {
       if (W.slot == C.slot) atomicAdd(&C.sum, c);
-      else atomicAdd(&tab->hot[W.slot].count, c);
+      else atomicAdd(&T.count[W.slot], c);
     }
     __syncwarp();
   }
@@ -547,7 +530,7 @@ struct Flat {
   // Ticket t of slot s: its edges that pass get_job's filter
   // (src/gpu_match.cu:531-556) become level-1 entries.
   __device__ bool fetch_chunk(int s, long long t) {
-    const SlotInfo &in = tab->info[s];
+    const FlatInfo &in = T.info[s];
     const FlatPlan &F = W.plan;
     const int chunk = __ldcg(&in.chunk);
     const int64_t e = __ldcg(&in.e_begin) + (t * __ldcg(&in.stride) + __ldcg(&in.phase)) * (int64_t)chunk + lane;
@@ -593,11 +576,11 @@ struct Flat {
   // Take over ticket t of the launch: find its slot and fetch its edges.
   // Tickets ascend, so the search starts at the slot of the last one.
   __device__ bool start_ticket(long long t, int &hint) {
-    const int n = tab->ctl.slots;
+    const int n = T.ctl->slots;
     int s = hint;
     for (;; s += 31) {
       // the last slot that starts at or before t; slots in [s, s + 32) at a time
-      const bool le = s + lane < n && __ldcg(&tab->info[s + lane].ticket0) <= t;
+      const bool le = s + lane < n && __ldg(&T.info[s + lane].ticket0) <= t;
       const int c = __popc(__ballot_sync(kFull, le));
       if (c < 32) {
         s += c - 1;
@@ -606,16 +589,16 @@ struct Flat {
     }
     hint = s;
     load_plan(s);
-    return fetch_chunk(s, t - __ldcg(&tab->info[s].ticket0));
+    return fetch_chunk(s, t - __ldg(&T.info[s].ticket0));
   }
 
   // The next ticket that yields edges; false when none is left.
   __device__ bool next_ticket(int &hint) {
     for (;;) {
       long long t = 0;
-      if (lane == 0) t = (long long)atomicAdd(&tab->ctl.ticket, 1ull);
+      if (lane == 0) t = (long long)atomicAdd(&T.ctl->ticket, 1ull);
       t = __shfl_sync(kFull, t, 0);
-      if (t >= tab->ctl.tickets) return false;
+      if (t >= T.ctl->tickets) return false;
       if (start_ticket(t, hint)) return true;
     }
   }
@@ -637,7 +620,7 @@ struct Flat {
     if (l > level) return;
     // 32 words of the idle mask, another part of it each time
     const int w = (int)(((unsigned)(clock64() >> 6) + (unsigned)(gid * 7 + lane)) % (unsigned)words);
-    const unsigned idle = *(volatile unsigned *)&sh->idle[w];
+    const unsigned idle = *(volatile unsigned *)&T.idle[w];
     unsigned have = __ballot_sync(kFull, idle != 0 && lane < words);
     if (!have) return;
     bool mine = idle != 0 && lane < words && __popc(have & lanemask_lt()) < take;
@@ -646,23 +629,23 @@ struct Flat {
       const int r = (gid + lane) & 31;  // start at another bit than other warps
       const unsigned rot = __funnelshift_r(idle, idle, r);
       const unsigned bit = 1u << ((__ffs(rot) - 1 + r) & 31);
-      mine = (atomicAnd(&sh->idle[w], ~bit) & bit) != 0;
+      mine = (atomicAnd(&T.idle[w], ~bit) & bit) != 0;
       target = w * 32 + __ffs(bit) - 1;
     }
     have = __ballot_sync(kFull, mine);
     const int boxes = __popc(have);
     if (!boxes) return;
     // entries [from, end) of level l, `per` to a box
-    const int per = min(min(32, kUnitInts / (l + 1)), (take + boxes - 1) / boxes);
+    const int per = min(min(32, kBoxInts / (l + 1)), (take + boxes - 1) / boxes);
     take = min(take, per * boxes);
     const int used = (take + per - 1) / per;
     const int rank = __popc(have & lanemask_lt());
     if (mine) W.cnt[0][rank] = (uint32_t)target;
-    if (lane == 0) atomicAdd(&tab->ctl.pending, used);
+    if (lane == 0) atomicAdd(&T.ctl->pending, used);
     __syncwarp();
     const int from = W.lev[l].end - take;
     for (int t = lane; t < take; t += 32) {
-      int32_t *v = sh->box[W.cnt[0][t / per]].v + (t % per) * (l + 1);
+      int32_t *v = T.box[W.cnt[0][t / per]].v + (t % per) * (l + 1);
       int q = from + t;
       for (int j = l; j >= 2; --j) {
         v[j] = xs(j)[q];
@@ -673,18 +656,18 @@ struct Flat {
     }
     const bool fill = mine && rank < used;
     if (fill) {
-      FlatBox &b = sh->box[target];
+      FlatBox &b = T.box[target];
       b.level = l;
       b.n = min(per, take - rank * per);
       b.slot = W.slot;
     }
     __threadfence();
     __syncwarp();
-    if (fill) *(volatile int32_t *)&sh->box[target].full = 1;
-    else if (mine) atomicOr(&sh->idle[target >> 5], 1u << (target & 31));  // claimed but not needed
+    if (fill) *(volatile int32_t *)&T.box[target].full = 1;
+    else if (mine) atomicOr(&T.idle[target >> 5], 1u << (target & 31));  // claimed but not needed
     if (lane == 0) {
       W.lev[l].end = from;
-      atomicAdd(&ctl->splits, (unsigned long long)used);
+      atomicAdd(&T.run->splits, (unsigned long long)used);
     }
     __syncwarp();
   }
@@ -692,6 +675,7 @@ struct Flat {
   // Take over the entries in this warp's mailbox; returns their level.
   __device__ int open_box() {
     __threadfence();
+    const FlatBox &box = T.box[gid];
     const int l = __ldcg(&box.level), n = __ldcg(&box.n);
     load_plan(__ldcg(&box.slot));
     if (lane < n) {
@@ -716,11 +700,11 @@ struct Flat {
     const unsigned long long t0 = now_ns();
     flush();
     if (lane == 0) {
-      *(volatile int32_t *)&box.full = 0;
+      *(volatile int32_t *)&T.box[gid].full = 0;
       __threadfence();
-      atomicOr(&sh->idle[gid >> 5], 1u << (gid & 31));
-      if (atomicSub(&C.active, 1) == 1 && atomicSub(&tab->ctl.pending, 1) == 1) {
-        ctl->finished = 1;
+      atomicOr(&T.idle[gid >> 5], 1u << (gid & 31));
+      if (atomicSub(&C.active, 1) == 1 && atomicSub(&T.ctl->pending, 1) == 1) {
+        T.run->finished = 1;
         *(volatile int32_t *)&C.done = 1;
       }
     }
@@ -728,16 +712,16 @@ struct Flat {
     unsigned nap = 200;
     for (;;) {
       if (lane == 0) {
-        if (*(volatile int32_t *)&box.full) st = 1;
+        if (*(volatile int32_t *)&T.box[gid].full) st = 1;
         else if (*(volatile int32_t *)&C.done) st = 2;
         else if (poller || (poller = atomicCAS(&C.poll, 0, 1) == 0)) {
-          if (*(volatile int32_t *)&tab->ctl.pending <= 0) {
+          if (*(volatile int32_t *)&T.ctl->pending <= 0) {
             *(volatile int32_t *)&C.done = 1;
             st = 2;
           }
         }
         if (!st && now_ns() - t0 > (unsigned long long)cfg.idle_ms * 1000000ull) {
-          atomicCAS(&ctl->error, 0, TDFS_ERR_TIMEOUT);
+          atomicCAS(&T.run->error, 0, TDFS_ERR_TIMEOUT);
           st = 2;
         }
       }
@@ -749,7 +733,7 @@ struct Flat {
     if (lane == 0) {
       if (poller) atomicExch(&C.poll, 0);
       // the mailbox's place in `pending` becomes the CTA's when it had no busy warp
-      if (st == 1 && atomicAdd(&C.active, 1) > 0) atomicSub(&tab->ctl.pending, 1);
+      if (st == 1 && atomicAdd(&C.active, 1) > 0) atomicSub(&T.ctl->pending, 1);
       W.idle_total += now_ns() - t0;
     }
     __syncwarp();
@@ -767,10 +751,11 @@ struct Flat {
     }
     __syncwarp();
     int level = 0, base = 1, hint = 0;
-    bool dry = false, more = false;
+    bool more = false;
+    bool dry = T.ctl->tickets <= (int)gridDim.x * (int)(blockDim.x >> 5);  // none besides the dealt ones
     long long checked = clock64();
     // the host dealt the first tickets, one per warp
-    if (gid < tab->ctl.tickets && start_ticket(gid, hint)) level = 1;
+    if (gid < T.ctl->tickets && start_ticket(gid, hint)) level = 1;
     for (;;) {
       if (level < base) {
         level = 0;
@@ -810,9 +795,9 @@ struct Flat {
       __threadfence_block();
       if (atomicSub(&C.left, 1) == 1) {
         __threadfence_block();
-        if (C.sum) atomicAdd(&tab->hot[C.slot].count, C.sum);
-        atomicAdd(&ctl->idle_ns, C.idle_ns);
-        atomicAdd(&ctl->warp_ns, C.warp_ns);
+        if (C.sum) atomicAdd(&T.count[C.slot], C.sum);
+        atomicAdd(&T.run->idle_ns, C.idle_ns);
+        atomicAdd(&T.run->warp_ns, C.warp_ns);
       }
     }
   }
@@ -820,8 +805,8 @@ struct Flat {
 
 template <bool LAB>
 __global__ void __launch_bounds__(256, 4) flat_kernel(const __grid_constant__ DevGraph G,
-                                                      const __grid_constant__ FlatCfg cfg, RunCtl *ctl,
-                                                      SlotTable *tab, FlatShared *sh) {
+                                                      const __grid_constant__ FlatCfg cfg,
+                                                      const __grid_constant__ FlatTable T) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ FlatCta cta;
   if (threadIdx.x == 0) {
@@ -834,13 +819,8 @@ __global__ void __launch_bounds__(256, 4) flat_kernel(const __grid_constant__ De
   const int me = threadIdx.x >> 5;
   unsigned char *base = smem + (size_t)me * cfg.warp_bytes;
   FlatSmem &W = *reinterpret_cast<FlatSmem *>(base);
-  Flat<LAB> f(G, cfg, ctl, tab, sh, (int)blockIdx.x * (int)(blockDim.x >> 5) + me, W, cta, base + sizeof(FlatSmem));
+  Flat<LAB> f(G, cfg, T, (int)blockIdx.x * (int)(blockDim.x >> 5) + me, W, cta, base + sizeof(FlatSmem));
   f.run();
-}
-
-__global__ void flat_init_kernel(RunCtl *ctl, FlatShared *sh) {
-  for (int i = threadIdx.x; i < (int)(sizeof(RunCtl) / 4); i += blockDim.x) reinterpret_cast<int32_t *>(ctl)[i] = 0;
-  for (int i = threadIdx.x; i < kIdleWords; i += blockDim.x) sh->idle[i] = 0;
 }
 
 template <bool LAB>
@@ -881,22 +861,29 @@ int flat_blocks_per_sm(bool labeled, int warps_per_block, size_t smem) {
   return e == cudaSuccess ? n : -1;
 }
 
-int flat_max_blocks(int warps_per_block) { return kBoxes / warps_per_block; }
-
-void init_flat(RunCtl *ctl, SplitUnit *units, cudaStream_t stream) {
-  flat_init_kernel<<<1, 256, 0, stream>>>(ctl, reinterpret_cast<FlatShared *>(units));
+int flat_chunk(int64_t edges, int s, int stride, int warps, int edge_chunk) {
+  if (edge_chunk > 0) return edge_chunk;
+  if (stride > 1) return 32;  // the documented round-robin deal
+  // Full lanes at the first levels against even shares: a plan counted at its
+  // edges has little work per edge and wants all 32 lanes (triangles of the
+  // n=4096 ER graph: 87 us with 1 edge per ticket, 39 with 4, 25 with 32);
+  // each level more multiplies an edge's work, and the wider the spread.
+  int c = s <= 1 ? 32 : s == 2 ? 8 : 2;
+  // at least two tickets per warp; a quarter of the warps suffices for the
+  // light edges of s = 1
+  while (c > 1 && edges / c < (s <= 1 ? warps / 4 : 2ll * warps)) c >>= 1;
+  return c;
 }
 
-int launch_flat(bool labeled, const DevGraph &g, RunCtl *ctl, SlotTable *tab, SplitUnit *units, const FlatCfg &cfg,
-                int blocks, int warps_per_block, cudaStream_t stream) {
-  FlatShared *sh = reinterpret_cast<FlatShared *>(units);
+int launch_flat(bool labeled, const DevGraph &g, const FlatTable &t, const FlatCfg &cfg, int blocks,
+                int warps_per_block, cudaStream_t stream) {
   const size_t smem = (size_t)cfg.warp_bytes * warps_per_block;
   const cudaError_t a = labeled ? flat_smem<true>(smem) : flat_smem<false>(smem);
   if (a != cudaSuccess) return fail(TDFS_ERR_CUDA, "flat kernel shared memory: %s", cudaGetErrorString(a));
   (void)cudaGetLastError();  // the check below must see this launch's error only
   const dim3 grid(blocks), block(warps_per_block * 32);
-  if (labeled) flat_kernel<true><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, sh);
-  else flat_kernel<false><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, sh);
+  if (labeled) flat_kernel<true><<<grid, block, smem, stream>>>(g, cfg, t);
+  else flat_kernel<false><<<grid, block, smem, stream>>>(g, cfg, t);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(TDFS_ERR_CUDA, "flat kernel launch: %s", cudaGetErrorString(e));
   return TDFS_OK;

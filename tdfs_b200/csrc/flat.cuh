@@ -36,15 +36,80 @@ int flat_max_entries(int warps);
 
 int flat_blocks_per_sm(bool labeled, int warps_per_block, size_t smem);
 
-// The most CTAs of a launch (every warp has a mailbox in the ring's memory).
-int flat_max_blocks(int warps_per_block);
+// ---- launch records -----------------------------------------------------------
+// What a launch over n slots reads and writes besides the graph, in one block
+// that the host fills and uploads with one copy:
+//   RunCtl | count[n] | FlatCtl | mask of idle warps | FlatInfo[n] | FlatPlan[n]
+// The first two come back with one copy.
+constexpr int kFlatBoxes = 8192;  // mailboxes, one per warp of the grid
+constexpr int kIdleWords = kFlatBoxes / 32;
 
-// Reset the control block and the mask of idle warps (stream-ordered).
-void init_flat(RunCtl *ctl, SplitUnit *units, cudaStream_t stream);
+struct alignas(128) FlatCtl {
+  unsigned long long ticket;  // the next ticket; the host deals the first ones, one per warp
+  char pad0_[120];
+  int32_t pending;            // CTAs with busy warps + filled mailboxes; 0 = the launch is complete
+  char pad1_[124];
+  int64_t tickets;            // tickets of all slots
+  int32_t slots;
+  char pad2_[116];
+};
 
-// Launch over the slot table `tab` (filled by the host); `units` is the split
-// ring's memory.
-int launch_flat(bool labeled, const DevGraph &g, RunCtl *ctl, SlotTable *tab, SplitUnit *units, const FlatCfg &cfg,
-                int blocks, int warps_per_block, cudaStream_t stream);
+// A slot: tickets [ticket0, ..) of the launch are its level-0 chunks.
+struct FlatInfo {
+  int64_t ticket0;
+  int64_t e_begin, e_end;  // as in SlotInfo
+  int32_t stride, phase, chunk, perm;
+};
+
+// A mailbox: up to 32 partial embeddings (tuples of level + 1 vertices).
+constexpr int kBoxInts = 156;
+struct FlatBox {
+  int32_t full;  // 0 empty, 1 filled by the warp that cleared the idle bit
+  int32_t level, n, slot;
+  int32_t v[kBoxInts];
+};
+constexpr size_t kFlatBoxBytes = sizeof(FlatBox) * kFlatBoxes;
+
+struct FlatTable {
+  RunCtl *run;
+  unsigned long long *count;  // raw counts (before the |Aut| multiplier)
+  FlatCtl *ctl;
+  unsigned *idle;
+  FlatInfo *info;
+  FlatPlan *plan;
+  FlatBox *box;
+
+  static size_t at_ctl(int n) { return sizeof(RunCtl) + (((size_t)n * 8 + 127) & ~size_t(127)); }
+  static size_t readback(int n) { return sizeof(RunCtl) + (size_t)n * 8; }
+  static size_t bytes(int n) {
+    return at_ctl(n) + sizeof(FlatCtl) + 4 * kIdleWords + (size_t)n * (sizeof(FlatInfo) + sizeof(FlatPlan));
+  }
+  // The views of the block at `base` (device, or its host image).
+  static FlatTable of(void *base, int n, FlatBox *box) {
+    char *b = static_cast<char *>(base);
+    FlatTable t;
+    t.run = reinterpret_cast<RunCtl *>(b);
+    t.count = reinterpret_cast<unsigned long long *>(b + sizeof(RunCtl));
+    b += at_ctl(n);
+    t.ctl = reinterpret_cast<FlatCtl *>(b);
+    t.idle = reinterpret_cast<unsigned *>(b + sizeof(FlatCtl));
+    t.info = reinterpret_cast<FlatInfo *>(t.idle + kIdleWords);
+    t.plan = reinterpret_cast<FlatPlan *>(t.info + n);
+    t.box = box;
+    return t;
+  }
+};
+
+// The most CTAs of a launch (every warp has a mailbox).
+inline int flat_max_blocks(int warps_per_block) { return kFlatBoxes / warps_per_block; }
+
+// Level-0 edges per ticket of a slot whose plan is enumerated down to level s,
+// in a launch of `edges` level-0 edges over all slots; `edge_chunk` and
+// `stride` as in tdfs_options.
+int flat_chunk(int64_t edges, int s, int stride, int warps, int edge_chunk);
+
+// Launch over the slots of `t` (on the device).
+int launch_flat(bool labeled, const DevGraph &g, const FlatTable &t, const FlatCfg &cfg, int blocks,
+                int warps_per_block, cudaStream_t stream);
 
 }  // namespace tdfs

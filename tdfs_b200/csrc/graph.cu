@@ -295,6 +295,8 @@ void free_workspace(Workspace *w) {
   cudaFree(w->ctl);
   cudaFreeHost(w->htab);
   if (w->gstream) cudaStreamDestroy(static_cast<cudaStream_t>(w->gstream));
+  for (void *e : w->ev)
+    if (e) cudaEventDestroy(static_cast<cudaEvent_t>(e));
   delete w;
 }
 

@@ -72,7 +72,6 @@ struct SlotInfo {
   int32_t chunk;     // directed edges per ticket (1, 2, 4, ..., 32)
   int32_t perm;      // 1: level-0 positions index DevGraph::lperm (labeled plans)
   int64_t budget;    // work units this query may spend (0 = unlimited)
-  int64_t ticket0;   // flat kernel: the launch's tickets before this slot's
 };
 
 struct alignas(128) SlotCtl {
@@ -82,23 +81,16 @@ struct alignas(128) SlotCtl {
   char pad1_[120];
   int32_t shutdown;              // host: 1 = no further admissions this launch
   int32_t idle_exit_ms;          // serving: retire after this long with no work
-  int32_t slots;                 // host, flat kernel: slots of the launch
-  char pad2_[116];
+  char pad2_[120];
   unsigned long long first_open; // device hint: slots below this have no tickets left
   char pad3_[120];
-  // flat kernel: tickets run over all slots in order (SlotInfo::ticket0)
-  unsigned long long ticket;     // the next one; the host deals the first ones, one per warp
-  long long tickets;             // host: tickets of all slots
-  char pad4_[112];
-  int32_t pending;               // CTAs with busy warps + units in the ring; 0 = the launch is complete
-  char pad5_[124];
 };
 
 struct SlotTable {
   SlotCtl ctl;
   SlotHot hot[kMaxSlots];
   SlotInfo info[kMaxSlots];
-  DevPlan plan[kMaxSlots];  // or the FlatPlan of launches of the flat kernel
+  DevPlan plan[kMaxSlots];
 };
 
 }  // namespace tdfs
@@ -119,6 +111,7 @@ struct Workspace {
   SlotTable *htab;     // pinned
   RunCtl *hctl;        // pinned
   void *gstream;       // cudaStream_t for captured launches (created on first use)
+  void *ev[2];         // cudaEvent_t around the kernel of plain launches (created on first use)
 };
 
 }  // namespace tdfs
