@@ -148,7 +148,7 @@ bool flat_options(const tdfs_options &o) {
          o.leaf_steal_min == 0 && o.level_hoist == 0 && o.tail_count == 0 && o.dead_prune == 0;
 }
 
-int flat_shape(int device, int smax, bool labeled, const tdfs_options &o, FlatShape *out) {
+int flat_shape(int device, int smax, int tmax, bool labeled, const tdfs_options &o, FlatShape *out) {
   static int sms[64] = {};
   static std::map<std::tuple<int, bool, int, size_t>, int> occ;  // CTAs per SM, as launch_shape caches them
   static std::mutex mu;
@@ -157,8 +157,11 @@ int flat_shape(int device, int smax, bool labeled, const tdfs_options &o, FlatSh
   s.warps_per_block = o.warps_per_block > 0 ? o.warps_per_block : 8;
   // entries per warp: as many as let 4 CTAs share an SM; chunk_cap asks for
   // that many (at least 64) per level
-  const int levels = std::max(1, smax - 1);
-  s.cfg.entries = o.chunk_cap > 0 ? std::max(64, (o.chunk_cap + 31) & ~31) * levels : smax > 1 ? flat_auto_entries() : 0;
+  const int least = flat_min_entries(smax, tmax);
+  s.cfg.entries = o.chunk_cap > 0 ? std::max(least, ((o.chunk_cap + 31) & ~31) * std::max(1, smax - 1))
+                  : smax > 1      ? flat_auto_entries()
+                                  : least;
+  s.cfg.entries = (s.cfg.entries + 31) & ~31;
   // (launch_shape accepts depths whose buffers fit the DFS kernel's layout)
   s.cfg.entries = std::min(s.cfg.entries, flat_max_entries(s.warps_per_block));
   s.cfg.warp_bytes = (int)flat_warp_bytes(s.cfg.entries);
@@ -427,11 +430,11 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
   if (n <= 0) return TDFS_OK;
   if (n > kMaxSlots) return fail(TDFS_ERR_CAPACITY, "at most %d plans per launch", kMaxSlots);
   const bool labeled = plans[0]->dev.labeled != 0;
-  int kmax = 3, smax = 1;
+  int kmax = 3, smax = 1, tmax = 1;
   for (int i = 0; i < n; ++i) {
     if ((plans[i]->dev.labeled != 0) != labeled) return fail(TDFS_ERR_ARG, "a launch mixes labeled and unlabeled plans");
     kmax = std::max(kmax, (int)plans[i]->dev.k);
-    if (flat) smax = std::max(smax, (int)plans[i]->flat.s);
+    if (flat) smax = std::max(smax, (int)plans[i]->flat.s), tmax = std::max(tmax, (int)plans[i]->flat.t);
   }
   if (labeled && !g->labeled) return fail(TDFS_ERR_ARG, "labeled pattern on a graph opened without labels");
   cudaError_t e = cudaSetDevice(g->device);
@@ -443,7 +446,7 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
   int rc = launch_shape(g, kmax, labeled, o, &shape);  // checks the options for either kernel
   if (rc) return rc;
   if (flat) {
-    if ((rc = flat_shape(g->device, smax, labeled, o, &L.fl))) return rc;
+    if ((rc = flat_shape(g->device, smax, tmax, labeled, o, &L.fl))) return rc;
   } else {
     L.dfs = shape;
   }

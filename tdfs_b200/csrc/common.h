@@ -83,6 +83,7 @@ struct DevGraph {
   const int32_t *colidx_l; // labeled graphs with few labels: every row re-sorted by (label, id), or nullptr
   const int32_t *loff;     // its segment starts: loff[v * (nlab + 1) + l], relative to rowptr[v]
   const int32_t *hash;     // row membership tables (see row_table_buckets), or nullptr
+  const int32_t *loops;    // with hash: not 0 when some row holds its own vertex
   int32_t nlab;            // labels 0..nlab-1 have segments
   int64_t nedges;
   int32_t n;

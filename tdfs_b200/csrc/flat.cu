@@ -15,8 +15,10 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kTupleMax = kMaxK - 1;   // phi(0..5): the deepest enumerated level is 5
 constexpr int kProbeMax = kMaxK - 2;   // lists tested per candidate besides its source
-constexpr int kScanSteps = 64;         // 64-position steps of a leaf scan between two looks at the idle count
-constexpr int kCheckCycles = 16384;    // clocks between those looks
+constexpr int kLookSteps = 32;         // 64-position steps of a scan between two looks at the idle mask
+constexpr int kCheckCycles = 16384;    // clocks between offers of work
+
+constexpr int kCntBytes = 7 * 32 * 4;
 
 // Work given away goes straight to an idle warp: each warp has a mailbox and
 // a bit in a grid-wide mask of idle warps.  A busy warp reads 32 words of the
@@ -50,16 +52,16 @@ struct FlatCta {
 struct alignas(16) FlatSmem {
   FlatPlan plan;
   int32_t slot;                     // slot of `plan`, -1 none
-  int32_t cap;                      // entries per level
+  int32_t cap, levels;              // entries per level, levels that store entries
   FlatLevel lev[kMaxK];             // levels 1..s
-  int64_t base[32];                 // per lane: source list start minus its first position
+  int4 src[32];                     // per list (lanes with one, in order): address minus its first position (in bytes; x, y)
+                                    // and the first row table to test (z first bucket, w bucket count;
+                                    // 0 = no test)
   int32_t phi[kTupleMax][32];       // per lane: the partial embedding being extended
-  uint32_t hb[kProbeMax][32];       // per lane: row tables to test (first bucket, bucket count; 0 = no test)
-  uint32_t nb[kProbeMax][32];
-  uint32_t cnt[7][32];              // per lane: sizes of the tail's sets
+  uint2 more[kProbeMax - 1][32];    // per lane: the other row tables to test
   int32_t er[32], ec[32];           // level-1 entries: edges (phi(0), phi(1))
   uint8_t map[32];                  // rank among the lanes with a list -> lane
-  uint8_t kind[32];                 // per lane: 1 = the source is a range of sibling entries
+  int32_t root;                     // level of the entries this warp was given
   unsigned long long t_work;        // globaltimer when the current base work was taken
   unsigned long long idle_total, t_start;  // diagnostics
 };
@@ -76,6 +78,13 @@ __device__ __forceinline__ unsigned long long now_ns() {
   return t;
 }
 
+// 1 << d, 0 for d > 31.
+__device__ __forceinline__ unsigned bit_at(uint32_t d) {
+  unsigned r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(d));  // PTX clamps the shift
+  return r;
+}
+
 template <bool LAB>
 struct Flat {
   const DevGraph &G;
@@ -84,18 +93,24 @@ struct Flat {
   const int gid;
   FlatSmem &W;
   FlatCta &C;
-  int32_t *X;   // entries: the vertex of the level ...
-  uint16_t *P;  // ... and the parent's entry one level up
+  int32_t *X;  // entries: the vertices of every level, then the parents' entries one level up
   unsigned long long count = 0;  // per lane; summed at release
   int lane;
 
   __device__ Flat(const DevGraph &g, const FlatCfg &c, const FlatTable &t, int warp, FlatSmem &w, FlatCta &cta,
                   unsigned char *bufs)
       : G(g), cfg(c), T(t), gid(warp), W(w), C(cta), X(reinterpret_cast<int32_t *>(bufs)),
-        P(reinterpret_cast<uint16_t *>(bufs + (size_t)c.entries * 4)), lane(lane_id()) {}
+        lane(lane_id()) {}
 
+  // Per lane: sizes of the tail's sets (plans with t >= 2 give up the end of
+  // their entries for them).
+  __device__ __forceinline__ uint32_t *cnt(int u) const {
+    return reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(X) + cfg.entries * 6 - kCntBytes) + 32 * u;
+  }
   __device__ __forceinline__ int32_t *xs(int l) const { return X + (l - 2) * W.cap; }
-  __device__ __forceinline__ uint16_t *ps(int l) const { return P + (l - 2) * W.cap; }
+  __device__ __forceinline__ uint16_t *ps(int l) const {
+    return reinterpret_cast<uint16_t *>(X + W.cap * W.levels) + (l - 2) * W.cap;
+  }
   __device__ __forceinline__ bool segmented() const { return LAB && cfg.segments && G.colidx_l != nullptr; }
   __device__ __forceinline__ const int32_t *lists() const { return segmented() ? G.colidx_l : G.colidx; }
 
@@ -125,23 +140,32 @@ struct Flat {
     nb = (uint32_t)(e / 3 - r / 3) + 1;
     return e > r;
   }
-  // First half of bucket i (the second half shares its sector).
-  __device__ __forceinline__ int4 bucket(uint32_t i) const {
-    return __ldg(reinterpret_cast<const int4 *>(G.hash) + 2 * (size_t)i);
+  struct Bucket {
+    int32_t e[kBucket];
+  };
+  __device__ __forceinline__ Bucket bucket(uint32_t i) const {
+    Bucket q;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(q.e[0]), "=r"(q.e[1]), "=r"(q.e[2]), "=r"(q.e[3]), "=r"(q.e[4]), "=r"(q.e[5]), "=r"(q.e[6]),
+          "=r"(q.e[7])
+        : "l"(G.hash + (size_t)i * kBucket));
+    return q;
   }
-  // Is x in the table, given the first half q of its bucket (offset b)?
-  __device__ __forceinline__ bool found(int4 q, uint32_t hb, uint32_t nb, uint32_t b, int32_t x) const {
-    if (q.x == x || q.y == x || q.z == x || q.w == x) return true;
-    if (q.w < 0) return false;  // entries fill a bucket in order
-    const int4 *h = reinterpret_cast<const int4 *>(G.hash);
-    uint32_t half = 2 * b + 1;  // 16-byte halves, cyclically within the row
-    for (uint32_t t = 1; t < 2 * nb; ++t) {
-      q = __ldg(h + 2 * (size_t)hb + half);
-      if (q.x == x || q.y == x || q.z == x || q.w == x) return true;
-      if (q.w < 0) return false;
-      half = half + 1 == 2 * nb ? 0 : half + 1;
+  __device__ __forceinline__ static bool holds(const Bucket &q, int32_t x) {
+    bool h = false;
+#pragma unroll
+    for (int i = 0; i < kBucket; ++i) h |= q.e[i] == x;
+    return h;
+  }
+  // Is x in the table, given its bucket q (offset b)?
+  __device__ __forceinline__ bool found(Bucket q, uint32_t hb, uint32_t nb, uint32_t b, int32_t x) const {
+    bool h = holds(q, x);
+    for (uint32_t t = 1; t < nb && !h && q.e[kBucket - 1] >= 0; ++t) {  // full: it may have overflowed
+      b = b + 1 == nb ? 0 : b + 1;
+      q = bucket(hb + b);
+      h = holds(q, x);
     }
-    return false;
+    return h;
   }
   __device__ __forceinline__ bool member(int32_t v, int32_t x) const {
     uint32_t hb, nb;
@@ -197,9 +221,9 @@ struct Flat {
   }
 
   // Set up this lane's candidate scan for st (its embedding: entry p of level
-  // L).  Writes the source start (W.base, W.kind) and the row tables to test
-  // (W.hb, W.nb); returns the number of source positions.
-  __device__ int setup_lane(const FlatStep &st, int L, int p) {
+  // L): the source's address, the first row table to test, and the others
+  // (W.more).  Returns the number of source positions.
+  __device__ int setup_lane(const FlatStep &st, int L, int p, int64_t &base, uint2 &first) {
     const int e = load_tuple(L, p, st.dep);
     // the shortest list is scanned, the others are tested
     uint32_t best = UINT_MAX;
@@ -254,57 +278,84 @@ struct Flat {
       else trim(lists(), gb, len, lo, hi);
     }
     if (len <= 0) return 0;
-    const int M = st.nbn - 1;
     int u = 0;
     const int nt = sib ? st.nsh : st.nbn;
+    uint32_t hb0 = 0, nb0 = 0;
     for (int t = 0; t < nt; ++t) {
       if (!sib && t == tb) continue;
       uint32_t hb, nb;
       if (!table(W.phi[sib ? st.bnsh[t] : st.bn[t]][lane], hb, nb)) return 0;
-      W.hb[u][lane] = hb;
-      W.nb[u][lane] = nb;
+      if (u == 0) {
+        hb0 = hb;
+        nb0 = nb;
+      } else {
+        W.more[u - 1][lane] = make_uint2(hb, nb);
+      }
       ++u;
     }
-    for (; u < M; ++u) W.nb[u][lane] = 0;
-    W.base[lane] = sib ? (int64_t)sb : gb;
-    W.kind[lane] = sib;
+    for (u = max(u, 1); u < st.nbn - 1; ++u) W.more[u - 1][lane] = make_uint2(0u, 0u);
+    base = reinterpret_cast<int64_t>(sib ? xs(dep) + sb : lists() + gb);
+    first = make_uint2(hb0, nb0);
     return len;
+  }
+
+  // Entries of level l that no scan has touched.
+  __device__ __forceinline__ int untouched(int l) const {
+    const FlatLevel &H = W.lev[l];
+    return H.end - (H.pos ? H.started : H.next);
+  }
+  // 32 words of the idle mask, another part of it each time; lanes beyond the
+  // grid's words get 0.
+  __device__ __forceinline__ unsigned idle_word(int &w) const {
+    const unsigned words = (gridDim.x * (blockDim.x >> 5) + 31) >> 5;
+    w = (int)(((unsigned)(clock64() >> 6) + (unsigned)(gid * 7 + lane)) % words);
+    return lane < words ? *(volatile unsigned *)&T.idle[w] : 0u;
+  }
+  // May this warp give work away yet (its base work is old enough)?
+  __device__ __forceinline__ bool may_give() const {
+    return now_ns() - W.t_work >= (unsigned long long)cfg.split_ns;
+  }
+  __device__ __forceinline__ bool someone_idle() const {
+    int w;
+    return __any_sync(kFull, idle_word(w) != 0 && may_give());
   }
 
   // The candidates of st for the block of up to 32 entries at W.lev[L].next.
   // mode 0: stored as entries of level L + 1 (until that buffer is full);
-  // mode 1: counted into `count`; mode 2: counted per entry into cnt[].
+  // mode 1: counted into `count`; mode 2: counted per entry into sizes[].
   // Modes 0 and 1 resume at, and leave, the block's position in W.lev[L]; they
-  // return false when they stopped after kScanSteps steps, so that the caller
-  // can look for idle warps.
+  // return false when they stopped early because a warp is idle and there are
+  // entries to give it.
   template <int mode>
-  __device__ __forceinline__ bool scan(const FlatStep &st, int L, uint32_t *cnt) {
+  __device__ __forceinline__ bool scan(const FlatStep &st, int L, uint32_t *sizes) {
     FlatLevel &H = W.lev[L];
     const int first = H.next;
     int len = 0;
-    if (first + lane < H.end) len = setup_lane(st, L, first + lane);
+    int64_t base = 0;
+    uint2 table0 = make_uint2(0u, 0u);
+    if (first + lane < H.end) len = setup_lane(st, L, first + lane, base, table0);
     uint32_t incl = (uint32_t)len;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
       const uint32_t t = __shfl_up_sync(kFull, incl, s);
       if (lane >= s) incl += t;
     }
-    const uint32_t off = incl - (uint32_t)len;
+    const uint32_t off = len > 0 ? incl - (uint32_t)len : ~0u;  // lanes without a list start nowhere
     const uint32_t total = __shfl_sync(kFull, incl, 31);
     const unsigned act = __ballot_sync(kFull, len > 0);
     if (len > 0) {
-      W.map[__popc(act & lanemask_lt())] = (uint8_t)lane;
-      W.base[lane] -= (int64_t)off;
+      const int rank = __popc(act & lanemask_lt());
+      base -= 4 * (int64_t)off;
+      W.map[rank] = (uint8_t)lane;
+      W.src[rank] = make_int4((int)base, (int)(base >> 32), (int)table0.x, (int)table0.y);
     }
     __syncwarp();
     uint32_t pos = mode < 2 ? H.pos : 0u;
-    int cur = __popc(__ballot_sync(kFull, len > 0 && off < pos));  // lists that start before pos
+    int cur = __popc(__ballot_sync(kFull, off < pos));  // lists that start before pos
     const unsigned le = lanemask_lt() | (1u << lane);
     const int M = st.nbn - 1;
     const unsigned neq = st.neq;
     const bool lab = LAB && !segmented();
-    const int32_t *L0 = lists();
-    const int32_t *Ls = st.dep ? xs(st.dep) : nullptr;
     int32_t *ox = nullptr;
     uint16_t *op = nullptr;
     int n = 0;
@@ -314,27 +365,39 @@ struct Flat {
       n = W.lev[L + 1].n;
     }
     const int room = W.cap - 64;
-    int step = 0;
-    for (; pos < total; ++step, pos += 64) {
-      if (mode < 2 && step >= kScanSteps) break;
+    bool early = false;
+    for (int step = 0; pos < total; ++step, pos += 64) {
       if (mode == 0 && n > room) break;
+      if (mode < 2 && (step & (kLookSteps - 1)) == kLookSteps - 1 && someone_idle()) {
+        bool give = H.end > first + 32 || __any_sync(kFull, len > 0 && off >= pos);
+        for (int l = W.root; l < L; ++l) give |= untouched(l) > 0;
+        if (give) {
+          early = true;
+          break;
+        }
+      }
       int o[2];
       int32_t x[2];
+      uint2 t0[2] = {make_uint2(0u, 0u), make_uint2(0u, 0u)};
       bool ok[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const uint32_t b = pos + 32 * u;
         // the lists that start inside these 32 positions, as a bit mask: a
         // lane's owner is the last one that starts at or before it
-        const unsigned m = __reduce_or_sync(kFull, len > 0 && off - b < 32u ? 1u << (off - b) : 0u);
+        const unsigned m = __reduce_or_sync(kFull, bit_at(off - b));
         const int r = cur + __popc(m & le) - 1;
         cur += __popc(m);
         ok[u] = b + (uint32_t)lane < total;
-        o[u] = ok[u] ? W.map[r] : 0;
+        o[u] = 0;
         x[u] = 0;
         if (ok[u]) {
-          const int64_t i = W.base[o[u]] + (int64_t)(b + (uint32_t)lane);
-          x[u] = W.kind[o[u]] ? Ls[i] : L0[i];
+          const int4 src = W.src[r];
+          o[u] = W.map[r];
+          // (a generic load: sources lie in global or in shared memory)
+          const int64_t at = ((int64_t)src.y << 32 | (uint32_t)src.x) + 4 * (int64_t)(b + (uint32_t)lane);
+          x[u] = *reinterpret_cast<const int32_t *>(at);
+          t0[u] = make_uint2((unsigned)src.z, (unsigned)src.w);
         }
       }
 #pragma unroll
@@ -342,19 +405,15 @@ struct Flat {
         if (lab && ok[u]) ok[u] = G.label[x[u]] == st.label;
         for (unsigned m = neq; m; m &= m - 1) ok[u] &= W.phi[__ffs(m) - 1][o[u]] != x[u];
       }
-      for (int m = 0; m < M; ++m) {
-        uint32_t nb[2], hb[2], b[2];
-        int4 q[2];
+      for (int m = 0; m < M && __any_sync(kFull, ok[0] || ok[1]); ++m) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          nb[u] = ok[u] ? W.nb[m][o[u]] : 0u;
-          hb[u] = W.hb[m][o[u]];
-          b[u] = __umulhi((uint32_t)x[u] * kRowHash, nb[u]);
-          if (nb[u]) q[u] = bucket(hb[u] + b[u]);
+          if (m > 0) t0[u] = W.more[m - 1][o[u]];
+          if (ok[u] && t0[u].y) {
+            const uint32_t at = __umulhi((uint32_t)x[u] * kRowHash, t0[u].y);
+            ok[u] = found(bucket(t0[u].x + at), t0[u].x, t0[u].y, at, x[u]);
+          }
         }
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-          if (nb[u]) ok[u] = found(q[u], hb[u], nb[u], b[u], x[u]);
       }
       if (mode == 0) {
 #pragma unroll
@@ -372,14 +431,14 @@ struct Flat {
       } else {
 #pragma unroll
         for (int u = 0; u < 2; ++u)
-          if (ok[u]) atomicAdd(&cnt[o[u]], 1u);
+          if (ok[u]) atomicAdd(&sizes[o[u]], 1u);
       }
     }
     __syncwarp();
     if (mode == 2) return true;
     const bool done = pos >= total;
-    const unsigned in = __ballot_sync(kFull, len > 0 && off < pos && off + (uint32_t)len > pos);
-    const unsigned before = __ballot_sync(kFull, len > 0 && off < pos);
+    const unsigned in = __ballot_sync(kFull, off < pos && off + (uint32_t)len > pos);
+    const unsigned before = __ballot_sync(kFull, off < pos);
     if (lane == 0) {
       if (mode == 0) W.lev[L + 1].n = n;
       if (done) {
@@ -394,11 +453,11 @@ struct Flat {
       }
     }
     __syncwarp();
-    return done || step < kScanSteps;
+    return !early;
   }
 
   // Fill level L + 1 from the entries of level L; `more`: go on filling.
-  // Returns true when it stopped early (kScanSteps).
+  // Returns true when it stopped early.
   __device__ bool expand(int L, bool more) {
     FlatLevel &H = W.lev[L], &D = W.lev[L + 1];
     if (lane == 0 && !more) {
@@ -454,7 +513,11 @@ struct Flat {
     }
     const int p = H.next + lane;
     const bool mine = p < H.end;
-    for (int u = 0; u < F.nterm; ++u) {
+    if (F.t == 1 && mine) {
+      load_tuple(L, p, 0);
+      count += closed_count(F.term[0]);
+    }
+    for (int u = 0; F.t > 1 && u < F.nterm; ++u) {
       const FlatStep &st = F.term[u];
       uint32_t c = 0;
       if (st.nbn == 1 && single) {
@@ -462,23 +525,21 @@ struct Flat {
           load_tuple(L, p, 0);
           c = closed_count(st);
         }
-        W.cnt[u][lane] = c;
+        cnt(u)[lane] = c;
       } else {
-        W.cnt[u][lane] = 0;
+        cnt(u)[lane] = 0;
         __syncwarp();
-        scan<2>(st, L, W.cnt[u]);
+        scan<2>(st, L, cnt(u));
       }
       __syncwarp();
     }
-    if (mine) {
+    if (F.t > 1 && mine) {
       auto at = [&](int m) -> unsigned long long {
         const int u = F.term_of[m];
-        return u == kNoTerm ? 0ull : (unsigned long long)W.cnt[u][lane];
+        return u == kNoTerm ? 0ull : (unsigned long long)cnt(u)[lane];
       };
       const unsigned long long a = at(1);
-      if (F.t == 1) {
-        count += a;
-      } else if (F.form == 1) {
+      if (F.form == 1) {
         count += F.t == 2 ? a * (a - 1) / 2 : a * (a - 1) / 2 * (a - 2) / 3;
       } else if (F.t == 2) {
         count += a * at(2) - at(3);
@@ -504,10 +565,15 @@ struct Flat {
     int32_t *dstw = reinterpret_cast<int32_t *>(&W.plan);
     for (int t = lane; t < (int)(sizeof(FlatPlan) / 4); t += 32) dstw[t] = __ldcg(srcw + t);
     __syncwarp();
+    if (lane < 11 && !*G.loops) {
+      // no self-loops: a neighbour of phi(j) differs from phi(j)
+      FlatStep &st = lane < 4 ? W.plan.step[lane] : W.plan.term[lane - 4];
+      for (int t = 0; t < st.nbn; ++t) st.neq &= (uint8_t)~(1u << st.bn[t]);
+    }
     if (lane == 0) {
       W.slot = s;
-      const int levels = max(1, (int)W.plan.s - 1);  // levels 2..s
-      W.cap = (cfg.entries / levels) & ~31;
+      W.levels = max(1, (int)W.plan.s - 1);  // levels 2..s
+      W.cap = ((cfg.entries - (W.plan.t > 1 ? kCntBytes / 6 + 1 : 0)) / W.levels) & ~31;
     }
     __syncwarp();
   }
@@ -568,6 +634,7 @@ struct Flat {
         H.groups = 0;
       }
       W.lev[l].end = W.lev[l].n = n;
+      W.root = l;
       W.t_work = now_ns();
     }
     __syncwarp();
@@ -608,22 +675,19 @@ struct Flat {
   // Give up to half of the untouched entries of the shallowest level that has
   // some to idle warps, if there are any.
   __device__ void donate(int base, int level) {
-    const int words = ((int)gridDim.x * (int)(blockDim.x >> 5) + 31) >> 5;
     int l = base, take = 0;
     for (; l <= level; ++l) {
-      const FlatLevel &H = W.lev[l];
-      const int avail = H.end - (H.pos ? H.started : H.next);
-      const bool other = l < level || H.pos;  // work stays here besides these entries
+      const int avail = untouched(l);
+      const bool other = l < level || W.lev[l].pos;  // work stays here besides these entries
       take = other ? (avail + 1) >> 1 : avail >> 1;
       if (take > 0) break;
     }
     if (l > level) return;
-    // 32 words of the idle mask, another part of it each time
-    const int w = (int)(((unsigned)(clock64() >> 6) + (unsigned)(gid * 7 + lane)) % (unsigned)words);
-    const unsigned idle = *(volatile unsigned *)&T.idle[w];
-    unsigned have = __ballot_sync(kFull, idle != 0 && lane < words);
+    int w;
+    const unsigned idle = idle_word(w);
+    unsigned have = __ballot_sync(kFull, idle != 0);
     if (!have) return;
-    bool mine = idle != 0 && lane < words && __popc(have & lanemask_lt()) < take;
+    bool mine = idle != 0 && __popc(have & lanemask_lt()) < take;
     int target = 0;
     if (mine) {
       const int r = (gid + lane) & 31;  // start at another bit than other warps
@@ -640,12 +704,12 @@ struct Flat {
     take = min(take, per * boxes);
     const int used = (take + per - 1) / per;
     const int rank = __popc(have & lanemask_lt());
-    if (mine) W.cnt[0][rank] = (uint32_t)target;
+    if (mine) W.src[rank].x = target;
     if (lane == 0) atomicAdd(&T.ctl->pending, used);
     __syncwarp();
     const int from = W.lev[l].end - take;
     for (int t = lane; t < take; t += 32) {
-      int32_t *v = T.box[W.cnt[0][t / per]].v + (t % per) * (l + 1);
+      int32_t *v = T.box[W.src[t / per].x].v + (t % per) * (l + 1);
       int q = from + t;
       for (int j = l; j >= 2; --j) {
         v[j] = xs(j)[q];
@@ -784,7 +848,7 @@ struct Flat {
       int due = 0;
       if (c - checked > kCheckCycles) {
         checked = c;
-        due = now_ns() - W.t_work >= (unsigned long long)cfg.split_ns;
+        due = may_give();
       }
       if (__shfl_sync(kFull, due, 0)) donate(base, level);
     }
@@ -838,6 +902,8 @@ cudaError_t flat_smem(size_t smem) {
 }
 
 }  // namespace
+
+int flat_min_entries(int smax, int tmax) { return 64 * (smax > 1 ? smax - 1 : 0) + (tmax > 1 ? kCntBytes / 6 + 33 : 0); }
 
 size_t flat_warp_bytes(int entries) {
   return (sizeof(FlatSmem) + (size_t)entries * 6 + 15) & ~(size_t)15;

@@ -27,10 +27,12 @@ struct FlatCfg {
 // Vertices up to this degree: 32 lists laid end to end stay within 32 bits.
 constexpr int64_t kFlatMaxDegree = int64_t(1) << 26;
 
-// Shared memory per warp with `entries` buffered partial embeddings, the
+// Shared memory per warp with `entries` buffered partial embeddings, the least
+// that a launch's plans can work with, the
 // entries that let 4 CTAs of 8 warps share an SM, and the most that one CTA of
 // `warps` warps can have.
 size_t flat_warp_bytes(int entries);
+int flat_min_entries(int smax, int tmax);  // plans enumerated down to smax, with tails of up to tmax vertices
 int flat_auto_entries();
 int flat_max_entries(int warps);
 

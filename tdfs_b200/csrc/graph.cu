@@ -70,9 +70,11 @@ __global__ void narrow_labels_kernel(const int32_t *__restrict__ in, int32_t n, 
 // bucket are taken, so entries fill a bucket in order whatever the order of
 // the threads.  Bound by the rate of the atomics in L2: 6M edges take 0.3 ms.
 __global__ void row_table_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                 const int32_t *__restrict__ src, int64_t nedges, int32_t *__restrict__ hash) {
+                                 const int32_t *__restrict__ src, int64_t nedges, int32_t *__restrict__ hash,
+                                 int32_t *__restrict__ loops) {
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nedges; j += (int64_t)gridDim.x * blockDim.x) {
     const int32_t v = src[j], x = colidx[j];
+    if (v == x) *loops = 1;
     const int64_t r = rowptr[v], e = rowptr[v + 1];
     const uint32_t nb = (uint32_t)(e / 3 - r / 3) + 1;
     int32_t *t = hash + kBucket * (r / 3 + v);
@@ -255,12 +257,13 @@ int cuda_fail(cudaError_t e, const char *what) {
 }  // namespace
 
 int build_row_tables(const int64_t *rowptr, const int32_t *colidx, const int32_t *src, int64_t n, int64_t nedges,
-                     int32_t *hash, cudaStream_t st) {
+                     int32_t *hash, int32_t *loops, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(hash, 0xff, 4 * kBucket * (size_t)row_table_buckets(n, nedges), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(loops, 0, sizeof(int32_t), st);
   if (e == cudaSuccess && nedges > 0) {
     (void)cudaGetLastError();  // the check below must see this launch's error only
     const int blocks = (int)std::min<int64_t>((nedges + 255) / 256, 148 * 32);
-    row_table_kernel<<<blocks, 256, 0, st>>>(rowptr, colidx, src, nedges, hash);
+    row_table_kernel<<<blocks, 256, 0, st>>>(rowptr, colidx, src, nedges, hash, loops);
     e = cudaGetLastError();
   }
   return e == cudaSuccess ? TDFS_OK : cuda_fail(e, "row membership tables");
@@ -617,7 +620,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   size_t hash_bytes = buckets <= (int64_t)UINT32_MAX && max_degree <= kFlatMaxDegree ? 4 * kBucket * (size_t)buckets : 0;
   void *arrays = nullptr, *stage = nullptr;
   size_t array_bytes = 0, stage_bytes = 0;
-  e = device_blocks().take(device, total + hash_bytes, &arrays, &array_bytes);
+  e = device_blocks().take(device, total + hash_bytes + 256, &arrays, &array_bytes);
   if (e == cudaErrorMemoryAllocation && hash_bytes) {
     (void)cudaGetLastError();
     hash_bytes = 0;
@@ -654,6 +657,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   g->loff = nlab ? reinterpret_cast<int32_t *>(base + o_loff) : nullptr;
   g->nlab = nlab;
   g->hash = hash_bytes ? reinterpret_cast<int32_t *>(base + total) : nullptr;
+  g->loops = hash_bytes ? reinterpret_cast<int32_t *>(base + total + hash_bytes) : nullptr;
   g->bytes = (dev_build ? o_hist : total) + hash_bytes;  // the scratch is not part of the graph
   const cudaStream_t st = cudaStreamPerThread;
   e = cudaMemcpyAsync(g->rowptr, rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
@@ -670,7 +674,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && g->hash &&
-      build_row_tables(g->rowptr, g->colidx, g->src, n, nedges, g->hash, st) != TDFS_OK)
+      build_row_tables(g->rowptr, g->colidx, g->src, n, nedges, g->hash, g->loops, st) != TDFS_OK)
     e = cudaErrorUnknown;
   std::unique_ptr<LabelIndex> lindex;
   if (e == cudaSuccess && labels) {
@@ -788,6 +792,7 @@ DevGraph graph_view(const tdfs_graph *g) {
   v.colidx_l = g->colidx_l;
   v.loff = g->loff;
   v.hash = g->hash;
+  v.loops = g->loops;
   v.nlab = g->nlab;
   v.nedges = g->nedges;
   v.n = (int32_t)g->n;

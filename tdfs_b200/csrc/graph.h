@@ -160,6 +160,7 @@ struct tdfs_graph {
   int32_t *loff;          //   and their segment starts per vertex and label
   int32_t nlab;
   int32_t *hash;          // row membership tables, or nullptr when they did not fit in device memory
+  int32_t *loops;         // with them: a flag, some row holds its own vertex
   tdfs::LabelIndex *lindex;  // its host copy and group offsets
   size_t array_bytes;     // size of the `arrays` block (cached for reuse when the graph is freed)
   void *staging;          // pinned host block: the derived arrays as uploaded (labeled graphs)
@@ -186,9 +187,9 @@ int acquire_workspace(tdfs_graph *g);
 void release_graphs(tdfs_graph *g);  // capi.cpp: destroys cached launch graphs
 DevGraph graph_view(const tdfs_graph *g);
 // Row membership tables (common.h, row_table_buckets) of a graph whose `src`
-// array is built, into `hash`; stream-ordered.
+// array is built, into `hash`, and the self-loop flag; stream-ordered.
 int build_row_tables(const int64_t *rowptr, const int32_t *colidx, const int32_t *src, int64_t n, int64_t nedges,
-                     int32_t *hash, cudaStream_t st);
+                     int32_t *hash, int32_t *loops, cudaStream_t st);
 int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, const int32_t *labels,
                          int32_t *src, int32_t *maxnd, uint8_t *label8, int32_t *bad, cudaStream_t st);
 inline QueueHdr *queue_hdr(tdfs_graph *g) { return reinterpret_cast<QueueHdr *>(g->queue + kQueueCap); }

@@ -159,6 +159,7 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   g.colidx_l = nullptr;  // nor label-partitioned rows: labeled plans test labels per candidate
   g.loff = nullptr;
   g.hash = nullptr;
+  g.loops = nullptr;
   g.nlab = 0;
   g.nedges = nedges;
   g.n = (int32_t)n;
