@@ -148,18 +148,20 @@ bool flat_options(const tdfs_options &o) {
          o.leaf_steal_min == 0 && o.level_hoist == 0 && o.tail_count == 0 && o.dead_prune == 0;
 }
 
-int flat_shape(int device, int smax, int tmax, bool labeled, const tdfs_options &o, FlatShape *out) {
+int flat_shape(int device, int levels, int tmax, bool skewed, bool big, bool labeled, const tdfs_options &o,
+               FlatShape *out) {
   static int sms[64] = {};
-  static std::map<std::tuple<int, bool, int, size_t>, int> occ;  // CTAs per SM, as launch_shape caches them
+  static std::map<std::tuple<int, bool, bool, bool, int, size_t>, int> occ;  // CTAs per SM, as launch_shape caches them
   static std::mutex mu;
   FlatShape s;
   std::memset(&s, 0, sizeof s);
   s.warps_per_block = o.warps_per_block > 0 ? o.warps_per_block : 8;
+  s.cfg.wide = skewed ? 1 : 0;
   // entries per warp: as many as let 4 CTAs share an SM; chunk_cap asks for
   // that many (at least 64) per level
-  const int least = flat_min_entries(smax, tmax);
-  s.cfg.entries = o.chunk_cap > 0 ? std::max(least, ((o.chunk_cap + 31) & ~31) * std::max(1, smax - 1))
-                  : smax > 1      ? flat_auto_entries()
+  const int least = flat_min_entries(levels, tmax);
+  s.cfg.entries = o.chunk_cap > 0 ? std::max(least, ((o.chunk_cap + 31) & ~31) * std::max(1, levels))
+                  : levels > 0    ? flat_auto_entries()
                                   : least;
   s.cfg.entries = (s.cfg.entries + 31) & ~31;
   // (launch_shape accepts depths whose buffers fit the DFS kernel's layout)
@@ -174,10 +176,10 @@ int flat_shape(int device, int smax, int tmax, bool labeled, const tdfs_options 
     const cudaError_t e = cudaDeviceGetAttribute(&sms[device], cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return cuda_err(e, "cudaDeviceGetAttribute");
   }
-  const auto key = std::make_tuple(device, labeled, s.warps_per_block, smem);
+  const auto key = std::make_tuple(device, labeled, skewed, big, s.warps_per_block, smem);
   auto it = occ.find(key);
   if (it == occ.end()) {
-    const int fit = flat_blocks_per_sm(labeled, s.warps_per_block, smem);
+    const int fit = flat_blocks_per_sm(labeled, skewed, big, s.warps_per_block, smem);
     if (fit < 0) return fail(TDFS_ERR_CUDA, "occupancy query failed: %s", cudaGetErrorString(cudaGetLastError()));
     it = occ.emplace(key, fit).first;
   }
@@ -216,6 +218,7 @@ int64_t ticket_count(int64_t b, int64_t e, int stride, int phase, int chunk) {
 // One launch of either kernel.
 struct Launch {
   bool flat;
+  bool big;         // flat: level 2 of some plan is held in global memory
   LaunchShape dfs;  // !flat
   FlatShape fl;     // flat
   int warps() const { return flat ? fl.blocks * fl.warps_per_block : dfs.blocks * dfs.warps_per_block; }
@@ -257,8 +260,9 @@ std::vector<GraphEntry> &graph_cache(tdfs_graph *g) {
 // The workspace as a launch of the flat kernel uses it: its records where the
 // slot table is, the mailboxes in the split ring's memory.
 static_assert(kFlatBoxBytes <= sizeof(SplitUnit) * kQueueCap, "the mailboxes fit the split ring");
-FlatTable flat_table(const tdfs_graph *g, int n) {
-  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue));
+FlatTable flat_table(const tdfs_graph *g, int n, bool big) {
+  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue),
+                       big ? static_cast<int32_t *>(g->ws->big) : nullptr);
 }
 
 // Upload, kernel (between the events k0 and k1, when given) and read-back.
@@ -281,7 +285,7 @@ int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStre
   if (k0) e = cudaEventRecordWithFlags(k0, st, flags);
   if (e != cudaSuccess) return cuda_err(e, "kernel start event");
   const int rc =
-      L.flat ? launch_flat(labeled, graph_view(g), flat_table(g, n), L.fl.cfg, L.fl.blocks, L.fl.warps_per_block, st)
+      L.flat ? launch_flat(labeled, graph_view(g), flat_table(g, n, L.big), L.fl.cfg, L.fl.blocks, L.fl.warps_per_block, st)
              : launch_match(labeled, graph_view(g), g->ctl, g->tab, g->queue, queue_hdr(g), L.dfs.cfg, L.dfs.blocks,
                             L.dfs.warps_per_block, st);
   if (rc) return rc;
@@ -302,7 +306,7 @@ int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStre
 // status array that fails the call.
 int collect(tdfs_graph *g, int n, bool flat, unsigned long long *raw, int *status) {
   if (flat) {
-    const FlatTable t = FlatTable::of(g->htab, n, nullptr);
+    const FlatTable t = FlatTable::of(g->htab, n, nullptr, nullptr);
     *g->hctl = *t.run;
     for (int i = 0; i < n; ++i) {
       raw[i] = t.count[i];
@@ -397,7 +401,7 @@ void fill_slots(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_
 // The host image of the flat kernel's records.
 void fill_flat(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_options &o, int64_t eb, int64_t ee,
                int stride, const Launch &L) {
-  const FlatTable t = FlatTable::of(g->htab, n, nullptr);
+  const FlatTable t = FlatTable::of(g->htab, n, nullptr, nullptr);
   std::memset(static_cast<void *>(g->htab), 0, FlatTable::bytes(n) - (size_t)n * sizeof(FlatPlan));
   t.ctl->ticket = (unsigned long long)L.warps();  // the first ones are dealt one per warp
   t.ctl->pending = L.fl.blocks;
@@ -430,11 +434,10 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
   if (n <= 0) return TDFS_OK;
   if (n > kMaxSlots) return fail(TDFS_ERR_CAPACITY, "at most %d plans per launch", kMaxSlots);
   const bool labeled = plans[0]->dev.labeled != 0;
-  int kmax = 3, smax = 1, tmax = 1;
+  int kmax = 3;
   for (int i = 0; i < n; ++i) {
     if ((plans[i]->dev.labeled != 0) != labeled) return fail(TDFS_ERR_ARG, "a launch mixes labeled and unlabeled plans");
     kmax = std::max(kmax, (int)plans[i]->dev.k);
-    if (flat) smax = std::max(smax, (int)plans[i]->flat.s), tmax = std::max(tmax, (int)plans[i]->flat.t);
   }
   if (labeled && !g->labeled) return fail(TDFS_ERR_ARG, "labeled pattern on a graph opened without labels");
   cudaError_t e = cudaSetDevice(g->device);
@@ -445,12 +448,29 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
   LaunchShape shape;
   int rc = launch_shape(g, kmax, labeled, o, &shape);  // checks the options for either kernel
   if (rc) return rc;
+  if ((rc = acquire_workspace(g))) return rc;
   if (flat) {
-    if ((rc = flat_shape(g->device, smax, tmax, labeled, o, &L.fl))) return rc;
+    // with hubs of more than kSkewDegree neighbours, candidate sets outgrow
+    // shared memory and long scans dominate
+    constexpr int32_t kSkewDegree = 4096;
+    const bool skewed = g->max_degree > kSkewDegree;
+    L.big = false;
+    for (int i = 0; i < n; ++i) L.big |= skewed && plans[i]->flat.reuse2;
+    if (L.big && !g->ws->big && cudaMalloc(&g->ws->big, kBigBytes * kFlatBoxes) != cudaSuccess) {
+      (void)cudaGetLastError();  // no room: level 2 stays in shared memory
+      g->ws->big = nullptr;
+      L.big = false;
+    }
+    int levels = 0, tmax = 1;
+    for (int i = 0; i < n; ++i) {
+      const FlatPlan &f = plans[i]->flat;
+      levels = std::max(levels, f.s - 1 - (L.big && f.reuse2 ? 1 : 0));
+      tmax = std::max(tmax, (int)f.t);
+    }
+    if ((rc = flat_shape(g->device, levels, tmax, skewed, L.big, labeled, o, &L.fl))) return rc;
   } else {
     L.dfs = shape;
   }
-  if ((rc = acquire_workspace(g))) return rc;
   const int64_t eb = std::max<int64_t>(0, o.edge_begin);
   const int64_t ee = (o.edge_end < 0 || o.edge_end > g->nedges) ? g->nedges : o.edge_end;
   const int stride = o.edge_stride > 0 ? o.edge_stride : 1;

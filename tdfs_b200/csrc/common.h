@@ -64,6 +64,8 @@ struct FlatPlan {
   int32_t deg[3];
   int32_t label[2];     // of pattern vertices 0 and 1
   uint8_t s, t, form, nterm;
+  uint8_t reuse2;       // 1: some set is taken from the candidate sets of vertex 2
+  uint8_t pad_[3];
   uint8_t term_of[8];
   FlatStep step[4];
   FlatStep term[7];

@@ -19,6 +19,7 @@ constexpr int kLookSteps = 32;         // 64-position steps of a scan between tw
 constexpr int kCheckCycles = 16384;    // clocks between offers of work
 
 constexpr int kCntBytes = 7 * 32 * 4;
+constexpr int kRangeMin = 4;           // children of one parent given away as a range
 
 // Work given away goes straight to an idle warp: each warp has a mailbox and
 // a bit in a grid-wide mask of idle warps.  A busy warp reads 32 words of the
@@ -52,7 +53,9 @@ struct FlatCta {
 struct alignas(16) FlatSmem {
   FlatPlan plan;
   int32_t slot;                     // slot of `plan`, -1 none
-  int32_t cap, levels;              // entries per level, levels that store entries
+  int32_t cap, levels;              // entries per level and levels held in shared memory
+  int32_t low;                      // the first of them: 2, or 3 when level 2 is in global memory
+  int32_t rlevel, rlo, rhi;         // entries of level rlevel are extended only in [rlo, rhi]; rlevel 0: no range
   FlatLevel lev[kMaxK];             // levels 1..s
   int4 src[32];                     // per list (lanes with one, in order): address minus its first position (in bytes; x, y)
                                     // and the first row table to test (z first bucket, w bucket count;
@@ -85,7 +88,7 @@ __device__ __forceinline__ unsigned bit_at(uint32_t d) {
   return r;
 }
 
-template <bool LAB>
+template <bool LAB, bool BIG>
 struct Flat {
   const DevGraph &G;
   const FlatCfg &cfg;
@@ -107,10 +110,14 @@ struct Flat {
   __device__ __forceinline__ uint32_t *cnt(int u) const {
     return reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(X) + cfg.entries * 6 - kCntBytes) + 32 * u;
   }
-  __device__ __forceinline__ int32_t *xs(int l) const { return X + (l - 2) * W.cap; }
+  __device__ __forceinline__ int32_t *big() const { return T.big + (size_t)gid * (kBigBytes / 4); }
+  __device__ __forceinline__ int low() const { return BIG ? W.low : 2; }
+  __device__ __forceinline__ int32_t *xs(int l) const { return BIG && l < W.low ? big() : X + (l - low()) * W.cap; }
   __device__ __forceinline__ uint16_t *ps(int l) const {
-    return reinterpret_cast<uint16_t *>(X + W.cap * W.levels) + (l - 2) * W.cap;
+    return BIG && l < W.low ? reinterpret_cast<uint16_t *>(big() + kBigEntries)
+                            : reinterpret_cast<uint16_t *>(X + W.cap * W.levels) + (l - low()) * W.cap;
   }
+  __device__ __forceinline__ int room(int l) const { return (BIG && l < W.low ? kBigEntries : W.cap) - 64; }
   __device__ __forceinline__ bool segmented() const { return LAB && cfg.segments && G.colidx_l != nullptr; }
   __device__ __forceinline__ const int32_t *lists() const { return segmented() ? G.colidx_l : G.colidx; }
 
@@ -364,10 +371,10 @@ struct Flat {
       op = ps(L + 1);
       n = W.lev[L + 1].n;
     }
-    const int room = W.cap - 64;
+    const int most = mode == 0 ? room(L + 1) : 0;
     bool early = false;
     for (int step = 0; pos < total; ++step, pos += 64) {
-      if (mode == 0 && n > room) break;
+      if (mode == 0 && n > most) break;
       if (mode < 2 && (step & (kLookSteps - 1)) == kLookSteps - 1 && someone_idle()) {
         bool give = H.end > first + 32 || __any_sync(kFull, len > 0 && off >= pos);
         for (int l = W.root; l < L; ++l) give |= untouched(l) > 0;
@@ -469,14 +476,34 @@ struct Flat {
       D.groups = 1;
     }
     __syncwarp();
-    while (H.next < H.end && D.n <= W.cap - 64)
+    while (H.next < H.end && D.n <= room(L + 1))
       if (!scan<0>(W.plan.step[L - 1], L, nullptr)) return true;
     if (lane == 0) {
       D.end = D.n;
       D.tcut = H.pos ? H.cutp : -1;
+      if (BIG && W.rlevel == L + 1) {
+        // given a range of one entry's children: the others serve as siblings only
+        const int32_t *x = xs(L + 1);
+        D.next = below(x, D.n, W.rlo);
+        D.end = below(x, D.n, W.rhi + 1);
+        if (D.end < D.n) {  // nothing in range beyond this fill
+          H.next = H.end;
+          H.pos = 0;
+        }
+      }
     }
     __syncwarp();
     return false;
+  }
+
+  // Entries of the ascending x[0, n) below v.
+  __device__ __forceinline__ static int below(const int32_t *x, int n, int32_t v) {
+    int a = 0, z = n;
+    while (a < z) {
+      const int m = (a + z) >> 1;
+      if (x[m] < v) a = m + 1; else z = m;
+    }
+    return a;
   }
 
   // Size of the set st of this lane's embedding (in W.phi), st having a single
@@ -572,7 +599,8 @@ struct Flat {
     }
     if (lane == 0) {
       W.slot = s;
-      W.levels = max(1, (int)W.plan.s - 1);  // levels 2..s
+      W.low = BIG && W.plan.reuse2 ? 3 : 2;
+      W.levels = max(1, (int)W.plan.s - W.low + 1);  // levels low..s
       W.cap = ((cfg.entries - (W.plan.t > 1 ? kCntBytes / 6 + 1 : 0)) / W.levels) & ~31;
     }
     __syncwarp();
@@ -635,6 +663,7 @@ struct Flat {
       }
       W.lev[l].end = W.lev[l].n = n;
       W.root = l;
+      W.rlevel = 0;
       W.t_work = now_ns();
     }
     __syncwarp();
@@ -673,12 +702,30 @@ struct Flat {
   // ---- giving work away -------------------------------------------------------
 
   // Give up to half of the untouched entries of the shallowest level that has
-  // some to idle warps, if there are any.
+  // some to idle warps, if there are any.  Entries whose extension reads their
+  // siblings (reuse) go as a range of one parent's children: the receiver
+  // makes the parent's children again, so that it has the siblings too.
   __device__ void donate(int base, int level) {
-    int l = base, take = 0;
+    int l = base, take = 0, parent = -1;
     for (; l <= level; ++l) {
-      const int avail = untouched(l);
-      const bool other = l < level || W.lev[l].pos;  // work stays here besides these entries
+      const FlatLevel &H = W.lev[l];
+      int avail = untouched(l);
+      bool other = l < level || H.pos;  // work stays here besides these entries
+      if (BIG && avail >= 2 * kRangeMin && l >= 2 && H.groups &&
+          (l < W.plan.s ? W.plan.step[l - 1] : W.plan.term[0]).dep == l) {
+        const uint16_t *pp = ps(l);
+        const int me = pp[H.end - 1];
+        int a = H.end - avail, z = H.end - 1;  // the first untouched child of me
+        while (a < z) {
+          const int m = (a + z) >> 1;
+          if (pp[m] < me) a = m + 1; else z = m;
+        }
+        if (H.end - a >= 2 * kRangeMin) {
+          parent = me;
+          other |= a > H.end - avail;
+          avail = H.end - a;
+        }
+      }
       take = other ? (avail + 1) >> 1 : avail >> 1;
       if (take > 0) break;
     }
@@ -700,7 +747,8 @@ struct Flat {
     const int boxes = __popc(have);
     if (!boxes) return;
     // entries [from, end) of level l, `per` to a box
-    const int per = min(min(32, kBoxInts / (l + 1)), (take + boxes - 1) / boxes);
+    const int per = parent >= 0 ? max(kRangeMin, (take + boxes - 1) / boxes)
+                                : min(min(32, kBoxInts / (l + 1)), (take + boxes - 1) / boxes);
     take = min(take, per * boxes);
     const int used = (take + per - 1) / per;
     const int rank = __popc(have & lanemask_lt());
@@ -708,7 +756,7 @@ struct Flat {
     if (lane == 0) atomicAdd(&T.ctl->pending, used);
     __syncwarp();
     const int from = W.lev[l].end - take;
-    for (int t = lane; t < take; t += 32) {
+    for (int t = lane; t < take && parent < 0; t += 32) {
       int32_t *v = T.box[W.src[t / per].x].v + (t % per) * (l + 1);
       int q = from + t;
       for (int j = l; j >= 2; --j) {
@@ -721,9 +769,22 @@ struct Flat {
     const bool fill = mine && rank < used;
     if (fill) {
       FlatBox &b = T.box[target];
-      b.level = l;
-      b.n = min(per, take - rank * per);
       b.slot = W.slot;
+      const int mine_n = min(per, take - rank * per);
+      if (BIG && parent >= 0) {
+        int q = parent;
+        for (int j = l - 1; j >= 2; --j) {
+          b.v[j] = xs(j)[q];
+          q = ps(j)[q];
+        }
+        b.v[0] = W.er[q];
+        b.v[1] = W.ec[q];
+        b.lo = xs(l)[from + rank * per];
+        b.hi = xs(l)[from + rank * per + mine_n - 1];
+      }
+      b.level = parent >= 0 ? l - 1 : l;
+      b.n = parent >= 0 ? 1 : mine_n;
+      b.range = parent >= 0;
     }
     __threadfence();
     __syncwarp();
@@ -752,6 +813,12 @@ struct Flat {
       }
     }
     install(l, n);
+    if (BIG && lane == 0 && __ldcg(&box.range)) {
+      W.rlevel = l + 1;
+      W.rlo = __ldcg(&box.lo);
+      W.rhi = __ldcg(&box.hi);
+    }
+    __syncwarp();
     return l;
   }
 
@@ -867,8 +934,13 @@ struct Flat {
   }
 };
 
-template <bool LAB>
-__global__ void __launch_bounds__(256, 4) flat_kernel(const __grid_constant__ DevGraph G,
+// Two register budgets of one kernel: 64 for 4 CTAs of 256 threads per SM, and
+// 80 for 3, whose scan step has more loads in flight: on skewed graphs, where
+// long scans dominate, it is the faster one (R-MAT 4-clique share 17.0 against
+// 19.0 ms, house slice 38.5 against 40.4), on small uniform graphs the warps
+// count (64-query burst 0.243 against 0.219 ms).
+template <bool LAB, int MINB, bool BIG>
+__global__ void __launch_bounds__(256, MINB) flat_kernel(const __grid_constant__ DevGraph G,
                                                       const __grid_constant__ FlatCfg cfg,
                                                       const __grid_constant__ FlatTable T) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -883,11 +955,11 @@ __global__ void __launch_bounds__(256, 4) flat_kernel(const __grid_constant__ De
   const int me = threadIdx.x >> 5;
   unsigned char *base = smem + (size_t)me * cfg.warp_bytes;
   FlatSmem &W = *reinterpret_cast<FlatSmem *>(base);
-  Flat<LAB> f(G, cfg, T, (int)blockIdx.x * (int)(blockDim.x >> 5) + me, W, cta, base + sizeof(FlatSmem));
+  Flat<LAB, BIG> f(G, cfg, T, (int)blockIdx.x * (int)(blockDim.x >> 5) + me, W, cta, base + sizeof(FlatSmem));
   f.run();
 }
 
-template <bool LAB>
+template <bool LAB, int MINB, bool BIG>
 cudaError_t flat_smem(size_t smem) {
   static std::mutex mu;
   static size_t set_to[64] = {};
@@ -896,14 +968,14 @@ cudaError_t flat_smem(size_t smem) {
   if (e != cudaSuccess || dev < 0 || dev >= 64) return e != cudaSuccess ? e : cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lk(mu);
   if (smem <= set_to[dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(flat_kernel<LAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = cudaFuncSetAttribute(flat_kernel<LAB, MINB, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) set_to[dev] = smem;
   return e;
 }
 
 }  // namespace
 
-int flat_min_entries(int smax, int tmax) { return 64 * (smax > 1 ? smax - 1 : 0) + (tmax > 1 ? kCntBytes / 6 + 33 : 0); }
+int flat_min_entries(int levels, int tmax) { return 64 * levels + (tmax > 1 ? kCntBytes / 6 + 33 : 0); }
 
 size_t flat_warp_bytes(int entries) {
   return (sizeof(FlatSmem) + (size_t)entries * 6 + 15) & ~(size_t)15;
@@ -917,14 +989,33 @@ int flat_auto_entries() {
 
 int flat_max_entries(int warps) { return (227 * 1024 / warps - 48 - (int)sizeof(FlatSmem)) / 6 & ~31; }
 
-int flat_blocks_per_sm(bool labeled, int warps_per_block, size_t smem) {
+namespace {
+
+template <bool LAB, int MINB, bool BIG>
+int flat_fit(int threads, size_t smem) {
   int n = 0;
-  cudaError_t e = labeled ? flat_smem<true>(smem) : flat_smem<false>(smem);
-  if (e == cudaSuccess)
-    e = labeled
-            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flat_kernel<true>, warps_per_block * 32, smem)
-            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flat_kernel<false>, warps_per_block * 32, smem);
+  cudaError_t e = flat_smem<LAB, MINB, BIG>(smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flat_kernel<LAB, MINB, BIG>, threads, smem);
   return e == cudaSuccess ? n : -1;
+}
+
+template <bool LAB, int MINB, bool BIG>
+cudaError_t flat_go(const DevGraph &g, const FlatTable &t, const FlatCfg &cfg, int blocks, int threads, size_t smem,
+                    cudaStream_t stream) {
+  const cudaError_t e = flat_smem<LAB, MINB, BIG>(smem);
+  if (e != cudaSuccess) return e;
+  (void)cudaGetLastError();  // the check below must see this launch's error only
+  flat_kernel<LAB, MINB, BIG><<<blocks, threads, smem, stream>>>(g, cfg, t);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+int flat_blocks_per_sm(bool labeled, bool wide, bool big, int warps_per_block, size_t smem) {
+  const int threads = warps_per_block * 32;
+  if (big) return labeled ? flat_fit<true, 3, true>(threads, smem) : flat_fit<false, 3, true>(threads, smem);
+  if (wide) return labeled ? flat_fit<true, 3, false>(threads, smem) : flat_fit<false, 3, false>(threads, smem);
+  return labeled ? flat_fit<true, 4, false>(threads, smem) : flat_fit<false, 4, false>(threads, smem);
 }
 
 int flat_chunk(int64_t edges, int s, int stride, int warps, int edge_chunk) {
@@ -944,13 +1035,12 @@ int flat_chunk(int64_t edges, int s, int stride, int warps, int edge_chunk) {
 int launch_flat(bool labeled, const DevGraph &g, const FlatTable &t, const FlatCfg &cfg, int blocks,
                 int warps_per_block, cudaStream_t stream) {
   const size_t smem = (size_t)cfg.warp_bytes * warps_per_block;
-  const cudaError_t a = labeled ? flat_smem<true>(smem) : flat_smem<false>(smem);
-  if (a != cudaSuccess) return fail(TDFS_ERR_CUDA, "flat kernel shared memory: %s", cudaGetErrorString(a));
-  (void)cudaGetLastError();  // the check below must see this launch's error only
-  const dim3 grid(blocks), block(warps_per_block * 32);
-  if (labeled) flat_kernel<true><<<grid, block, smem, stream>>>(g, cfg, t);
-  else flat_kernel<false><<<grid, block, smem, stream>>>(g, cfg, t);
-  const cudaError_t e = cudaGetLastError();
+  const int threads = warps_per_block * 32;
+  auto go = [&](auto f) { return f(g, t, cfg, blocks, threads, smem, stream); };
+  const cudaError_t e = t.big      ? labeled ? go(flat_go<true, 3, true>) : go(flat_go<false, 3, true>)
+                        : cfg.wide ? labeled ? go(flat_go<true, 3, false>) : go(flat_go<false, 3, false>)
+                        : labeled  ? go(flat_go<true, 4, false>)
+                                   : go(flat_go<false, 4, false>);
   if (e != cudaSuccess) return fail(TDFS_ERR_CUDA, "flat kernel launch: %s", cudaGetErrorString(e));
   return TDFS_OK;
 }

@@ -22,6 +22,7 @@ struct FlatCfg {
   int32_t idle_ms;     // bounded idle wait before a warp reports a timeout
   int32_t split_ns;    // work may be given away after this long on one base subtree
   int32_t segments;    // 1: labeled plans read the label segments of rows (DevGraph::colidx_l)
+  int32_t wide;        // 1: the 80-register build (3 CTAs of 256 threads per SM)
 };
 
 // Vertices up to this degree: 32 lists laid end to end stay within 32 bits.
@@ -32,11 +33,11 @@ constexpr int64_t kFlatMaxDegree = int64_t(1) << 26;
 // entries that let 4 CTAs of 8 warps share an SM, and the most that one CTA of
 // `warps` warps can have.
 size_t flat_warp_bytes(int entries);
-int flat_min_entries(int smax, int tmax);  // plans enumerated down to smax, with tails of up to tmax vertices
+int flat_min_entries(int levels, int tmax);  // `levels` levels in shared memory, tails of up to tmax vertices
 int flat_auto_entries();
 int flat_max_entries(int warps);
 
-int flat_blocks_per_sm(bool labeled, int warps_per_block, size_t smem);
+int flat_blocks_per_sm(bool labeled, bool wide, bool big, int warps_per_block, size_t smem);
 
 // ---- launch records -----------------------------------------------------------
 // What a launch over n slots reads and writes besides the graph, in one block
@@ -64,13 +65,25 @@ struct FlatInfo {
 };
 
 // A mailbox: up to 32 partial embeddings (tuples of level + 1 vertices).
-constexpr int kBoxInts = 156;
+// With `range`, one embedding, of whose children only those in [lo, hi] are
+// to be extended.
+constexpr int kBoxInts = 153;
 struct FlatBox {
   int32_t full;  // 0 empty, 1 filled by the warp that cleared the idle bit
   int32_t level, n, slot;
+  int32_t range, lo, hi;
   int32_t v[kBoxInts];
 };
 constexpr size_t kFlatBoxBytes = sizeof(FlatBox) * kFlatBoxes;
+
+// Level 2 of plans that reuse its candidate sets (FlatPlan::reuse2), on graphs
+// whose sets may not fit shared memory: a buffer per warp in global memory.
+// An entry whose siblings are all there is extended from them with one test
+// per candidate; one whose siblings were cut off, from its shortest list with
+// a test per other list (90% of a 5-clique's candidates on the power-law graph
+// with 320 entries in shared memory).
+constexpr int kBigEntries = 2048;
+constexpr size_t kBigBytes = (size_t)kBigEntries * 6;
 
 struct FlatTable {
   RunCtl *run;
@@ -80,6 +93,7 @@ struct FlatTable {
   FlatInfo *info;
   FlatPlan *plan;
   FlatBox *box;
+  int32_t *big;  // kBigBytes per warp, or nullptr
 
   static size_t at_ctl(int n) { return sizeof(RunCtl) + (((size_t)n * 8 + 127) & ~size_t(127)); }
   static size_t readback(int n) { return sizeof(RunCtl) + (size_t)n * 8; }
@@ -87,7 +101,7 @@ struct FlatTable {
     return at_ctl(n) + sizeof(FlatCtl) + 4 * kIdleWords + (size_t)n * (sizeof(FlatInfo) + sizeof(FlatPlan));
   }
   // The views of the block at `base` (device, or its host image).
-  static FlatTable of(void *base, int n, FlatBox *box) {
+  static FlatTable of(void *base, int n, FlatBox *box, int32_t *big) {
     char *b = static_cast<char *>(base);
     FlatTable t;
     t.run = reinterpret_cast<RunCtl *>(b);
@@ -98,6 +112,7 @@ struct FlatTable {
     t.info = reinterpret_cast<FlatInfo *>(t.idle + kIdleWords);
     t.plan = reinterpret_cast<FlatPlan *>(t.info + n);
     t.box = box;
+    t.big = big;
     return t;
   }
 };

@@ -146,6 +146,8 @@ bool flat_plan(const DevPlan &d, FlatPlan *out) {
       if (meet) f.term_of[m] = add(st);
     }
   }
+  for (int i = 0; i < s - 1; ++i) f.reuse2 |= f.step[i].dep == 2;
+  for (int u = 0; u < f.nterm; ++u) f.reuse2 |= f.term[u].dep == 2;
   *out = f;
   return true;
 }

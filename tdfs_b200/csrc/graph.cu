@@ -297,6 +297,7 @@ constexpr int kIdlePerDevice = 4;       // idle workspaces kept per device; more
 void free_workspace(Workspace *w) {
   cudaFree(w->ctl);
   cudaFreeHost(w->htab);
+  cudaFree(w->big);
   if (w->gstream) cudaStreamDestroy(static_cast<cudaStream_t>(w->gstream));
   for (void *e : w->ev)
     if (e) cudaEventDestroy(static_cast<cudaEvent_t>(e));

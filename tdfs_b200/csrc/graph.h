@@ -111,6 +111,7 @@ struct Workspace {
   SlotTable *htab;     // pinned
   RunCtl *hctl;        // pinned
   void *gstream;       // cudaStream_t for captured launches (created on first use)
+  void *big;           // the flat kernel's level-2 buffers (allocated on first use)
   void *ev[2];         // cudaEvent_t around the kernel of plain launches (created on first use)
 };
 

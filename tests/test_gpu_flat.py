@@ -98,3 +98,29 @@ def test_flat_and_dfs_kernels_agree_on_a_power_law_graph(T):
         assert T.count(dev, P).count == want
         shards = [T.count(dev, P, T.shard_options(r, 3)).count for r in range(3)]
         assert sum(shards) == want
+
+
+def test_level_two_in_global_memory(T):
+    """On graphs with hubs of more than 4096 neighbours, plans that extend a
+    vertex from its siblings keep level 2 in global memory, refilled when a
+    candidate set outgrows it, and give children away as ranges."""
+    n, hubs = 7000, 24
+    rng = np.random.default_rng(6)
+    e = set()
+    for h in range(hubs):  # hubs adjacent to each other and to most vertices: sets beyond 2048 entries
+        e |= {(h, int(v)) for v in rng.choice(n, 5200, replace=False) if v > h}
+    e |= {(int(a), int(b)) for a, b in rng.integers(hubs, n, (9000, 2)) if a < b}
+    e |= {(b, a) for a, b in e}
+    rowptr, colidx = csr(e, n)
+    labels = (np.arange(n) % 2).astype(np.int32)
+    dev = T.GraphPreprocessor(rowptr=rowptr, colidx=colidx, labels=labels, labeled=True)
+    assert dev.max_degree > 4096
+    # labeled: the same set reused by two later vertices
+    fan = "".join(f"v {i} {int(i > 1)}\n" for i in range(5)) + "".join(
+        f"e {a} {b} 1\n" for a, b in ((0, 1), (0, 2), (1, 2), (0, 3), (1, 3), (2, 3), (3, 4)))
+    for text, labeled in ((clique(4), False), (clique(5), False), (DIAMOND, False), (fan, True)):
+        P = T.PatternPreprocessor(text=text, labeled=labeled)
+        want = T.count(dev, P, T.default_options(tail_count=1)).count  # the DFS kernel
+        assert want > 0
+        for opt in ({}, {"split_after_us": -1, "edge_chunk": 1}, {"warps_per_block": 2, "chunk_cap": 64}):
+            assert T.count(dev, P, T.default_options(**opt)).count == want, (text, opt)
