@@ -525,7 +525,7 @@ int tdfs_graph_open(const char *prefix, int labeled, int device, tdfs_graph **ou
   int rc = tdfs_csr_read(prefix, labeled, &c);
   if (rc) return rc;
   rc = graph_upload(c->n, c->nedges, c->rowptr.data(), c->colidx.data(), labeled ? c->labels.data() : nullptr,
-                    device, c->max_degree, out);
+                    device, c->max_degree, false, out);
   delete c;
   return rc;
 }
@@ -533,10 +533,8 @@ int tdfs_graph_open(const char *prefix, int labeled, int device, tdfs_graph **ou
 int tdfs_graph_from_csr(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx,
                         const int32_t *labels, int device, tdfs_graph **out) {
   if (!rowptr || (!colidx && nedges) || !out) return fail(TDFS_ERR_ARG, "null argument");
-  int32_t md = 0;
-  int rc = validate_csr(n, nedges, rowptr, colidx, &md);
-  if (rc) return rc;
-  return graph_upload(n, nedges, rowptr, colidx, labels, device, md, out);
+  if (const int rc = check_csr_frame(n, nedges, rowptr)) return rc;
+  return graph_upload(n, nedges, rowptr, colidx, labels, device, 0, true, out);
 }
 
 int tdfs_graph_info(const tdfs_graph *g, int64_t *n, int64_t *nedges, int32_t *max_degree, int *labeled,

@@ -96,12 +96,13 @@ struct DevGraph {
 // Every adjacency row again as a hash table of 8-entry buckets (32 bytes: one
 // load, one sector): "is y in row v?" costs one load, whatever the row's
 // length, where a binary search costs log2(degree) dependent ones.  Row v owns
-// the buckets [first, first + count) with first = rowptr[v] / 3 + v, so no
-// offset array is needed and a bucket holds 3 entries on average.  Entries
-// fill a bucket in order, -1 is empty; a full bucket (about one in a hundred)
+// the buckets [first, first + count) with first = row_table_at(rowptr[v]) + v, so
+// no offset array is needed and a bucket holds 3.2 entries on average.  Entries
+// fill a bucket in order, -1 is empty; a full bucket (about two in a hundred)
 // overflows into the next one, cyclically within the row.
 constexpr int kBucket = 8;
-inline int64_t row_table_buckets(int64_t n, int64_t nedges) { return nedges / 3 + n + 1; }
+constexpr int64_t row_table_at(int64_t r) { return (r >> 2) + (r >> 4); }
+inline int64_t row_table_buckets(int64_t n, int64_t nedges) { return row_table_at(nedges) + n + 1; }
 constexpr uint32_t kRowHash = 0x9E3779B1u;  // 2^32 / golden ratio: neighbouring ids spread over the buckets
 
 // Per-launch control block in device memory.  Counters that many warps touch

@@ -65,10 +65,21 @@ int write_array(const std::string &path, const T *src, size_t count) {
 
 }  // namespace
 
-int validate_csr(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx,
-                 int32_t *max_degree) {
+int check_csr_frame(int64_t n, int64_t nedges, const int64_t *rowptr) {
   if (n < 0 || n > INT32_MAX - 1 || nedges < 0) return fail(TDFS_ERR_FORMAT, "bad graph size");
   if (rowptr[0] != 0 || rowptr[n] != nedges) return fail(TDFS_ERR_FORMAT, "rowptr must span [0, E]");
+  return TDFS_OK;
+}
+
+int csr_fault(int kind, int64_t row) {
+  if (kind == 1) return fail(TDFS_ERR_FORMAT, "rowptr decreases at vertex %lld", (long long)row);
+  if (kind == 2) return fail(TDFS_ERR_FORMAT, "neighbour id out of range in row %lld", (long long)row);
+  return fail(TDFS_ERR_FORMAT, "row %lld not strictly increasing (unsorted or duplicate edge)", (long long)row);
+}
+
+int validate_csr(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx,
+                 int32_t *max_degree) {
+  if (const int rc = check_csr_frame(n, nedges, rowptr)) return rc;
   std::atomic<int> bad{0};
   std::atomic<int64_t> where{-1};
   std::vector<int32_t> part_max(hw_threads() + 1, 0);
@@ -88,11 +99,7 @@ int validate_csr(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     }
     part_max[slot++] = md;
   }, n + nedges);
-  if (bad == 1) return fail(TDFS_ERR_FORMAT, "rowptr decreases at vertex %lld", (long long)where.load());
-  if (bad == 2) return fail(TDFS_ERR_FORMAT, "neighbour id out of range in row %lld", (long long)where.load());
-  if (bad == 3)
-    return fail(TDFS_ERR_FORMAT, "row %lld not strictly increasing (unsorted or duplicate edge)",
-                (long long)where.load());
+  if (bad) return csr_fault(bad, where.load());
   if (max_degree) *max_degree = *std::max_element(part_max.begin(), part_max.end());
   return TDFS_OK;
 }

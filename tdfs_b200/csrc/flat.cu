@@ -143,8 +143,8 @@ struct Flat {
   // Row v's membership table: false when the row is empty.
   __device__ __forceinline__ bool table(int32_t v, uint32_t &hb, uint32_t &nb) const {
     const int64_t r = G.rowptr[v], e = G.rowptr[v + 1];
-    hb = (uint32_t)(r / 3 + v);
-    nb = (uint32_t)(e / 3 - r / 3) + 1;
+    hb = (uint32_t)(row_table_at(r) + v);
+    nb = (uint32_t)(row_table_at(e) - row_table_at(r)) + 1;
     return e > r;
   }
   struct Bucket {

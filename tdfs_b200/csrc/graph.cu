@@ -18,6 +18,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <string>
 #include <thread>
 #include <vector>
 
@@ -29,61 +30,12 @@ namespace tdfs {
 
 namespace {
 
-// One warp per vertex: writes the vertex id over its edge range.
-__global__ void build_src_kernel(const int64_t *__restrict__ rowptr, int32_t n, int32_t *__restrict__ src) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * blockDim.x / 32;
-  for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; v < n; v += warps) {
-    const int64_t b = rowptr[v], e = rowptr[v + 1];
-    for (int64_t j = b + lane; j < e; j += 32) src[j] = (int32_t)v;
-  }
-}
-
-// One warp per vertex: max over neighbours w of deg(w).
-__global__ void max_nbr_deg_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                   int32_t n, int32_t *__restrict__ maxnd) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * blockDim.x / 32;
-  for (int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; v < n; v += warps) {
-    const int64_t b = rowptr[v], e = rowptr[v + 1];
-    int32_t m = -1;
-    for (int64_t j = b + lane; j < e; j += 32) {
-      const int32_t w = colidx[j];
-      m = max(m, (int32_t)(rowptr[w + 1] - rowptr[w]));
-    }
-    m = __reduce_max_sync(0xffffffffu, (unsigned)(m + 1)) - 1;
-    if (lane == 0) maxnd[v] = m;
-  }
-}
-
 __global__ void narrow_labels_kernel(const int32_t *__restrict__ in, int32_t n, uint8_t *__restrict__ out,
                                      int32_t *__restrict__ bad) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int32_t l = in[i];
     if (l < 0 || l > 254) atomicExch(bad, 1);
     out[i] = (uint8_t)(l < 0 || l > 254 ? 255 : l);
-  }
-}
-
-// One thread per edge: the neighbour into its row's membership table
-// (row_table_buckets).  A slot is tried only when the ones before it in the
-// bucket are taken, so entries fill a bucket in order whatever the order of
-// the threads.  Bound by the rate of the atomics in L2: 6M edges take 0.3 ms.
-__global__ void row_table_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                 const int32_t *__restrict__ src, int64_t nedges, int32_t *__restrict__ hash,
-                                 int32_t *__restrict__ loops) {
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nedges; j += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v = src[j], x = colidx[j];
-    if (v == x) *loops = 1;
-    const int64_t r = rowptr[v], e = rowptr[v + 1];
-    const uint32_t nb = (uint32_t)(e / 3 - r / 3) + 1;
-    int32_t *t = hash + kBucket * (r / 3 + v);
-    uint32_t b = __umulhi((uint32_t)x * kRowHash, nb);
-    bool placed = false;
-    for (uint32_t tries = 0; tries < nb && !placed; ++tries) {
-      for (int i = 0; i < kBucket && !placed; ++i) placed = atomicCAS(t + kBucket * (int64_t)b + i, -1, x) == -1;
-      b = b + 1 == nb ? 0 : b + 1;
-    }
   }
 }
 
@@ -110,51 +62,220 @@ inline int64_t tile_edges(int64_t nedges) {
 }
 constexpr int kBuildWarps = 8;    // warps per CTA of the build kernels
 
-// One warp per vertex: its row again, stably partitioned by neighbour label
-// (col_l), and each label's segment start relative to the row start (loff,
-// nl + 1 per vertex, the last one the row length).  Two passes over the row:
-// the label counts, then the scatter.
-__global__ void label_rows_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                  const uint8_t *__restrict__ lab, int32_t n, int nl, int32_t *__restrict__ col_l,
-                                  int32_t *__restrict__ loff) {
-  __shared__ int32_t cnt_s[kBuildWarps][kSegLabels];
+// ---- the CSR's rules ------------------------------------------------------------
+struct CsrCheck {
+  int32_t kind;  // 0, or what is wrong: 1 rowptr, 2 a neighbour id, 3 a row's order (as validate_csr, csr.cpp)
+  int32_t max_degree;
+  int64_t row;
+};
+
+// The rules of validate_csr on the device copy.  Reads inside the arrays
+// whatever they hold: a row's range is only compared, and a descending pair of
+// neighbours is looked up among the row starts.  6M edges take 0.10 ms; the
+// host's pass took 2.8 ms with 16 threads (the first of them had the hubs).
+__global__ void check_csr_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, int64_t n,
+                                 int64_t nedges, CsrCheck *out) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto bad = [&](int kind, int64_t row) {
+    if (atomicCAS(&out->kind, 0, kind) == 0) out->row = row;
+  };
+  int32_t md = 0;
+  for (int64_t v = first; v < n; v += step) {
+    const int64_t lo = rowptr[v], hi = rowptr[v + 1];
+    if (lo < 0 || hi > nedges || hi < lo || hi - lo > INT32_MAX) bad(1, v);
+    else md = max(md, (int32_t)(hi - lo));
+  }
+  md = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)md);
+  if ((threadIdx.x & 31) == 0 && md > 0) atomicMax(&out->max_degree, md);
+  for (int64_t j = first; j < nedges; j += step) {
+    const int32_t c = colidx[j];
+    const bool range = c < 0 || c >= n, falls = j + 1 < nedges && c >= colidx[j + 1];
+    if (!range && !falls) continue;
+    int64_t a = 0, z = n;  // the first row that starts after j
+    while (a < z) {
+      const int64_t m = (a + z) >> 1;
+      if (rowptr[m] <= j) a = m + 1; else z = m;
+    }
+    if (range) bad(2, a - 1);
+    else if (rowptr[a] != j + 1) bad(3, a - 1);
+  }
+}
+
+// ---- what every row gives -------------------------------------------------------
+// One pass over the rows writes all that is derived from them: the source of
+// every edge, the largest degree among a vertex's neighbours, the row's
+// membership table (row_table_buckets, cleared before), and on labeled graphs
+// with segments the row again, stably partitioned by neighbour label (col_l),
+// with each label's segment start relative to the row start (loff, nl + 1 per
+// vertex, the last one the row length).
+//
+// A warp takes a row; rows of more than kLongRow edges are left to the whole
+// CTA, each warp a contiguous part.  Neighbouring vertices go to different
+// CTAs: with ids in degree order the hubs come first and would otherwise meet
+// in one.  Bound by the chain of dependent loads per row (row, neighbours,
+// their degrees and labels): 6M edges over 1.1M vertices take 0.48 ms, where the
+// four kernels it replaces took 1.17 ms, 0.76 of them with one warp on a
+// 21 000-edge row.
+constexpr int kRowWarps = 16;
+constexpr int64_t kLongRow = 512;
+
+struct Rows {
+  const int64_t *rowptr;
+  const int32_t *colidx;
+  int32_t n;
+  int32_t *src, *maxnd;
+  int32_t *hash, *loops;   // nullptr: no tables
+  const uint8_t *lab;      // nullptr: no segments
+  int32_t nl;
+  int32_t *col_l, *loff;
+};
+
+// Into row [r, e)'s table: a slot is tried only when the ones before it in its
+// bucket are taken, so entries fill a bucket in order whatever the order of
+// the threads.
+__device__ __forceinline__ void table_insert(int32_t *hash, int32_t v, int64_t r, int64_t e, int32_t x) {
+  const uint32_t nb = (uint32_t)(row_table_at(e) - row_table_at(r)) + 1;
+  int32_t *t = hash + kBucket * (row_table_at(r) + v);
+  uint32_t b = __umulhi((uint32_t)x * kRowHash, nb);
+  for (uint32_t tries = 0; tries < nb; ++tries) {
+    for (int i = 0; i < kBucket; ++i)
+      if (atomicCAS(t + kBucket * (int64_t)b + i, -1, x) == -1) return;
+    b = b + 1 == nb ? 0 : b + 1;
+  }
+}
+
+// First pass over edges [j0, j1) of row v = [b, e), a warp: sources, table, the
+// largest neighbour degree + 1 (0 for none), and the label counts into cnt.
+template <bool LAB>
+__device__ __forceinline__ unsigned row_first(const Rows &R, int32_t v, int64_t b, int64_t e, int64_t j0, int64_t j1,
+                                              int32_t *cnt) {
+  const int lane = threadIdx.x & 31;
+  unsigned m = 0;
+  const bool whole = e - b <= 32;  // this warp has the row at once: its table needs no atomics
+  for (int64_t c0 = j0; c0 < j1; c0 += 32) {
+    const int64_t j = c0 + lane;
+    const bool valid = j < j1;
+    int key = -1;
+    int32_t w = 0;
+    if (valid) {
+      w = R.colidx[j];
+      R.src[j] = v;
+      m = max(m, (unsigned)(R.rowptr[w + 1] - R.rowptr[w]) + 1u);
+      if (LAB) key = (int)R.lab[w];
+    }
+    if (R.hash) {
+      if (valid && w == v) *R.loops = 1;
+      bool left = valid;
+      if (whole) {
+        const uint32_t nb = (uint32_t)(row_table_at(e) - row_table_at(b)) + 1;
+        const int bk = valid ? (int)__umulhi((uint32_t)w * kRowHash, nb) : -1;
+        const int rank = __popc(__match_any_sync(0xffffffffu, bk) & lanes_below());
+        left = valid && rank >= kBucket;
+        if (valid && !left) R.hash[kBucket * (row_table_at(b) + v + bk) + rank] = w;
+        if (__any_sync(0xffffffffu, left)) {  // a bucket overflows: its other entries are in place first
+          __threadfence();
+          __syncwarp();
+        }
+      }
+      if (left) table_insert(R.hash, v, b, e, w);
+    }
+    if (LAB) {
+      const unsigned same = __match_any_sync(0xffffffffu, key);
+      if (valid && lane == __ffs(same) - 1) cnt[key] += __popc(same);
+      __syncwarp();
+    }
+  }
+  return m;
+}
+
+// Second pass: every neighbour to its label's next place (cursors in cnt).
+__device__ __forceinline__ void row_scatter(const Rows &R, int64_t b, int64_t j0, int64_t j1, int32_t *cnt) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t c0 = j0; c0 < j1; c0 += 32) {
+    const int64_t j = c0 + lane;
+    const bool valid = j < j1;
+    const int32_t w = valid ? R.colidx[j] : 0;
+    const int key = valid ? (int)R.lab[w] : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, key);
+    if (valid) R.col_l[b + cnt[key] + __popc(same & lanes_below())] = w;
+    __syncwarp();
+    if (valid && lane == __ffs(same) - 1) cnt[key] += __popc(same);
+    __syncwarp();
+  }
+}
+
+template <bool LAB>
+__global__ void __launch_bounds__(32 * kRowWarps) rows_kernel(const Rows R) {
+  __shared__ int32_t cnt_s[kRowWarps][kSegLabels];
+  __shared__ unsigned max_s[kRowWarps];
+  __shared__ int32_t long_s[32 * kRowWarps];
+  __shared__ int nlong;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   int32_t *cnt = cnt_s[wib];
-  const int64_t warps = (int64_t)gridDim.x * kBuildWarps;
-  for (int64_t v = (int64_t)blockIdx.x * kBuildWarps + wib; v < n; v += warps) {
-    const int64_t b = rowptr[v], e = rowptr[v + 1];
-    if (lane < kSegLabels) cnt[lane] = 0;
+  // this CTA's rows: blockIdx.x + k * gridDim.x
+  for (int64_t v = blockIdx.x + (int64_t)wib * gridDim.x; v < R.n; v += (int64_t)kRowWarps * gridDim.x) {
+    const int64_t b = R.rowptr[v], e = R.rowptr[v + 1];
+    if (e - b > kLongRow) continue;
+    if (LAB && lane < kSegLabels) cnt[lane] = 0;
     __syncwarp();
-    for (int64_t c0 = b; c0 < e; c0 += 32) {
-      const int64_t j = c0 + lane;
-      const bool valid = j < e;
-      const int key = valid ? (int)lab[colidx[j]] : -1;
-      const unsigned m = __match_any_sync(0xffffffffu, key);
-      if (valid && lane == __ffs(m) - 1) cnt[key] += __popc(m);
-      __syncwarp();
-    }
-    const int32_t c = lane < nl ? cnt[lane] : 0;
-    int32_t incl = c;
+    const unsigned m = __reduce_max_sync(0xffffffffu, row_first<LAB>(R, (int32_t)v, b, e, b, e, cnt));
+    if (lane == 0) R.maxnd[v] = (int32_t)m - 1;
+    if (LAB) {
+      const int32_t c = lane < R.nl ? cnt[lane] : 0;
+      int32_t incl = c;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int32_t t = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += t;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
+      }
+      if (lane <= R.nl) R.loff[v * (R.nl + 1) + lane] = incl - c;  // lane nl: the row length
+      __syncwarp();
+      if (lane < R.nl) cnt[lane] = incl - c;  // scatter cursors
+      __syncwarp();
+      row_scatter(R, b, b, e, cnt);
+      __syncwarp();
     }
-    const int32_t excl = incl - c;  // lane nl: the row length
-    if (lane <= nl) loff[v * (nl + 1) + lane] = excl;
-    __syncwarp();
-    if (lane < nl) cnt[lane] = excl;  // scatter cursors
-    __syncwarp();
-    for (int64_t c0 = b; c0 < e; c0 += 32) {
-      const int64_t j = c0 + lane;
-      const bool valid = j < e;
-      const int32_t w = valid ? colidx[j] : 0;
-      const int key = valid ? (int)lab[w] : -1;
-      const unsigned m = __match_any_sync(0xffffffffu, key);
-      if (valid) col_l[b + cnt[key] + __popc(m & lanes_below())] = w;
+  }
+  for (int64_t k0 = 0; blockIdx.x + k0 * gridDim.x < R.n; k0 += 32 * kRowWarps) {
+    __syncthreads();
+    if (threadIdx.x == 0) nlong = 0;
+    __syncthreads();
+    const int64_t v = blockIdx.x + (k0 + threadIdx.x) * gridDim.x;
+    if (v < R.n && R.rowptr[v + 1] - R.rowptr[v] > kLongRow) long_s[atomicAdd(&nlong, 1)] = (int32_t)v;
+    __syncthreads();
+    for (int k = 0; k < nlong; ++k) {
+      const int64_t u = long_s[k];
+      const int64_t b = R.rowptr[u], e = R.rowptr[u + 1];
+      const int64_t part = ((e - b + kRowWarps - 1) / kRowWarps + 31) & ~(int64_t)31;
+      const int64_t j0 = min(e, b + wib * part), j1 = min(e, j0 + part);
+      if (LAB && lane < kSegLabels) cnt[lane] = 0;
       __syncwarp();
-      if (valid && lane == __ffs(m) - 1) cnt[key] += __popc(m);
-      __syncwarp();
+      const unsigned m = __reduce_max_sync(0xffffffffu, row_first<LAB>(R, (int32_t)u, b, e, j0, j1, cnt));
+      if (lane == 0) max_s[wib] = m;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        unsigned all = 0;
+        for (int w = 0; w < kRowWarps; ++w) all = max(all, max_s[w]);
+        R.maxnd[u] = (int32_t)all - 1;
+      }
+      if (LAB) {
+        if (threadIdx.x == 0) {  // every warp's first place per label, label by label
+          int32_t run = 0;
+          for (int l = 0; l < R.nl; ++l) {
+            R.loff[u * (R.nl + 1) + l] = run;
+            for (int w = 0; w < kRowWarps; ++w) {
+              const int32_t c = cnt_s[w][l];
+              cnt_s[w][l] = run;
+              run += c;
+            }
+          }
+          R.loff[u * (R.nl + 1) + R.nl] = run;
+        }
+        __syncthreads();
+        row_scatter(R, b, j0, j1, cnt);
+      }
+      __syncthreads();
     }
   }
 }
@@ -188,33 +309,46 @@ __global__ void edge_hist_kernel(const int32_t *__restrict__ src, const int32_t 
   }
 }
 
-// One CTA of 1024 threads: exclusive scan of the histogram in place (each
-// thread a contiguous run, then a scan of the run sums in shared memory), and
-// the group offsets goff[key] (goff[G] = the edge count).
+// One CTA of 1024 threads: exclusive scan of the histogram in place, 4096
+// entries at a time (four per thread, coalesced, then a scan of the warps'
+// sums), and the group offsets goff[key] (goff[G] = the edge count).  125 000
+// entries take 0.06 ms; each thread on a run of its own, as before, 0.22 ms.
 __global__ void __launch_bounds__(1024) index_scan_kernel(int32_t *__restrict__ a, int64_t N, int G,
                                                           int32_t ntiles, int64_t nedges,
                                                           int64_t *__restrict__ goff) {
-  __shared__ int64_t part[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (N + 1023) / 1024;
-  const int64_t b = t * per < N ? t * per : N, e = b + per < N ? b + per : N;
-  int64_t s = 0;
-  for (int64_t i = b; i < e; ++i) s += a[i];
-  part[t] = s;
-  __syncthreads();
-  for (int d = 1; d < 1024; d <<= 1) {
-    const int64_t v = t >= d ? part[t - d] : 0;
+  __shared__ int32_t sums[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  int32_t carry = 0;  // edge ids fit 31 bits on labeled graphs
+  for (int64_t i0 = 0; i0 < N; i0 += 4096) {
+    const int64_t i = i0 + 4 * t;
+    int32_t x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = i + k < N ? a[i + k] : 0;
+    const int32_t mine = x[0] + x[1] + x[2] + x[3];
+    int32_t incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    if (lane == 31) sums[w] = incl;
     __syncthreads();
-    part[t] += v;
+    const int32_t s = sums[lane];
+    int32_t all = s;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int32_t u = __shfl_up_sync(0xffffffffu, all, d);
+      if (lane >= d) all += u;
+    }
+    int32_t run = carry + __shfl_sync(0xffffffffu, all - s, w) + incl - mine;
+    carry += __shfl_sync(0xffffffffu, all, 31);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < N) a[i + k] = run;
+      run += x[k];
+    }
     __syncthreads();
   }
-  int64_t run = part[t] - s;
-  for (int64_t i = b; i < e; ++i) {
-    const int32_t x = a[i];
-    a[i] = (int32_t)run;
-    run += x;
-  }
-  __syncthreads();
   for (int k = t; k < G; k += 1024) goff[k] = a[(int64_t)k * ntiles];
   if (t == 0) goff[G] = nedges;
 }
@@ -256,33 +390,36 @@ int cuda_fail(cudaError_t e, const char *what) {
 
 }  // namespace
 
-int build_row_tables(const int64_t *rowptr, const int32_t *colidx, const int32_t *src, int64_t n, int64_t nedges,
-                     int32_t *hash, int32_t *loops, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(hash, 0xff, 4 * kBucket * (size_t)row_table_buckets(n, nedges), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(loops, 0, sizeof(int32_t), st);
-  if (e == cudaSuccess && nedges > 0) {
+namespace {
+
+int run_rows(const Rows &R, int64_t nedges, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  if (R.hash) {
+    e = cudaMemsetAsync(R.hash, 0xff, 4 * kBucket * (size_t)row_table_buckets(R.n, nedges), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(R.loops, 0, sizeof(int32_t), st);
+  }
+  if (e == cudaSuccess && R.n > 0) {
     (void)cudaGetLastError();  // the check below must see this launch's error only
-    const int blocks = (int)std::min<int64_t>((nedges + 255) / 256, 148 * 32);
-    row_table_kernel<<<blocks, 256, 0, st>>>(rowptr, colidx, src, nedges, hash, loops);
+    const int blocks = (int)std::min<int64_t>((R.n + kRowWarps - 1) / kRowWarps, 148 * 4);
+    if (R.lab) rows_kernel<true><<<blocks, 32 * kRowWarps, 0, st>>>(R);
+    else rows_kernel<false><<<blocks, 32 * kRowWarps, 0, st>>>(R);
     e = cudaGetLastError();
   }
-  return e == cudaSuccess ? TDFS_OK : cuda_fail(e, "row membership tables");
+  return e == cudaSuccess ? TDFS_OK : cuda_fail(e, "graph preparation kernels");
 }
+
+}  // namespace
 
 // Derived per-graph arrays into caller-provided device memory, no allocation:
 // edge -> source, neighbour-degree maxima and (when labels is not null) 8-bit
 // labels.  *bad becomes nonzero when a label lies outside [0, 254].
-int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, const int32_t *labels,
-                         int32_t *src, int32_t *maxnd, uint8_t *label8, int32_t *bad, cudaStream_t st) {
-  (void)cudaGetLastError();  // the check below must see these launches' errors only
-  if (n > 0) {
-    const int threads = 256;
-    const int64_t want = ((int64_t)n * 32 + threads - 1) / threads;
-    const int blocks = (int)std::min<int64_t>(want, 148 * 16);
-    build_src_kernel<<<blocks, threads, 0, st>>>(rowptr, n, src);
-    max_nbr_deg_kernel<<<blocks, threads, 0, st>>>(rowptr, colidx, n, maxnd);
-    if (labels) narrow_labels_kernel<<<148 * 4, 256, 0, st>>>(labels, n, label8, bad);
-  }
+int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, int64_t nedges,
+                         const int32_t *labels, int32_t *src, int32_t *maxnd, uint8_t *label8, int32_t *bad,
+                         int32_t *hash, int32_t *loops, cudaStream_t st) {
+  const Rows R{rowptr, colidx, n, src, maxnd, hash, loops, nullptr, 0, nullptr, nullptr};
+  const int rc = run_rows(R, nedges, st);
+  if (rc || !labels || n <= 0) return rc;
+  narrow_labels_kernel<<<148 * 4, 256, 0, st>>>(labels, n, label8, bad);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TDFS_OK : cuda_fail(e, "graph preparation kernels");
 }
@@ -416,20 +553,33 @@ class BlockCache {
     return e;
   }
 
-  // Keep a block for reuse (within the cache's byte cap), else free it.
+  // Keep a block for reuse, in the place of the ones idle the longest where
+  // the cache is full (blocks of sizes no longer asked for would otherwise
+  // make every create and free of a graph go to the driver); a block beyond
+  // the byte cap is freed.
   void give(int device, void *p, size_t bytes) {
     if (!p) return;
-    {
+    std::vector<void *> out;
+    if (bytes > cap_) {
+      out.push_back(p);
+    } else {
       std::lock_guard<std::mutex> lk(mu_);
       int mine = 0;
       for (const Block &b : idle_) mine += b.device == device;
-      if (idle_bytes_ + bytes <= cap_ && mine < kPerDevice) {
-        idle_.push_back(Block{device, bytes, p});
-        idle_bytes_ += bytes;
-        return;
+      for (size_t i = 0; i < idle_.size() && (mine >= kPerDevice || idle_bytes_ + bytes > cap_);) {
+        if (idle_bytes_ + bytes > cap_ || idle_[i].device == device) {
+          mine -= idle_[i].device == device;
+          idle_bytes_ -= idle_[i].bytes;
+          out.push_back(idle_[i].p);
+          idle_.erase(idle_.begin() + (long)i);
+        } else {
+          ++i;
+        }
       }
+      idle_.push_back(Block{device, bytes, p});
+      idle_bytes_ += bytes;
     }
-    release(p);
+    for (void *x : out) release(x);
   }
 
  private:
@@ -572,24 +722,37 @@ void build_label_arrays(int64_t n, int64_t nedges, const int64_t *rowptr, const 
 // 256-byte boundary:
 //   rowptr int64[n+1] | colidx int32[E + kColPad] | src int32[E] | maxnd int32[n]
 //   | label uint8[n] | lperm int32[E] | colidx_l int32[E + kColPad] | loff int32[n (nlab+1)]
-//   | scratch of the label index sort | row membership tables
+//   | scratch of the label index sort | row membership tables | self-loop flag and check result
 // The parts from `label` on are derived on the host into one pinned staging
 // block laid out the same way and uploaded with one copy.  The CSR copies and
 // the two preprocessing kernels are queued first, so the device works while
 // the host sorts; one synchronisation at the end.
 int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx, const int32_t *labels,
-                 int device, int32_t max_degree, tdfs_graph **out) {
+                 int device, int32_t max_degree, bool check, tdfs_graph **out) {
   int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
-    return fail(TDFS_ERR_CUDA, "no CUDA device visible (the tdfs engine has no CPU path)");
-  if (device < 0 || device >= ndev) return fail(TDFS_ERR_ARG, "device %d out of range", device);
+  // where the device cannot check the CSR the host does, so that what is wrong
+  // with it is still what the caller is told
+  auto checked = [&](int rc) {
+    const std::string msg = tdfs_last_error();
+    if (check)
+      if (const int bad = validate_csr(n, nedges, rowptr, colidx, nullptr)) return bad;
+    return fail(rc, "%s", msg.c_str());
+  };
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+    (void)cudaGetLastError();
+    return checked(fail(TDFS_ERR_CUDA, "no CUDA device visible (the tdfs engine has no CPU path)"));
+  }
+  if (device < 0 || device >= ndev) return checked(fail(TDFS_ERR_ARG, "device %d out of range", device));
   int nl = 0;
   if (labels) {
-    for (int64_t i = 0; i < n; ++i) {
-      if (labels[i] < 0 || labels[i] > 254)
-        return fail(TDFS_ERR_FORMAT, "vertex labels must lie in [0, 254] for the device label array");
-      nl = std::max(nl, labels[i] + 1);
+    int32_t least = 0, most = -1;
+    for (int64_t i = 0; i < n; ++i) {  // (no early exit: the loop vectorises)
+      least = std::min(least, labels[i]);
+      most = std::max(most, labels[i]);
     }
+    if (least < 0 || most > 254)
+      return checked(fail(TDFS_ERR_FORMAT, "vertex labels must lie in [0, 254] for the device label array"));
+    nl = most + 1;
     if (nedges > INT32_MAX) return fail(TDFS_ERR_CAPACITY, "labeled graphs hold at most 2^31 - 1 directed edges");
   }
   // label-partitioned rows for graphs with at most kSegLabels labels
@@ -618,16 +781,16 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   // the row membership tables, where the flat kernel can use them and the
   // device has room; without them every plan runs on the DFS kernel
   const int64_t buckets = row_table_buckets(n, nedges);
-  size_t hash_bytes = buckets <= (int64_t)UINT32_MAX && max_degree <= kFlatMaxDegree ? 4 * kBucket * (size_t)buckets : 0;
+  size_t hash_bytes = buckets <= (int64_t)UINT32_MAX ? 4 * kBucket * (size_t)buckets : 0;
   void *arrays = nullptr, *stage = nullptr;
   size_t array_bytes = 0, stage_bytes = 0;
   e = device_blocks().take(device, total + hash_bytes + 256, &arrays, &array_bytes);
   if (e == cudaErrorMemoryAllocation && hash_bytes) {
     (void)cudaGetLastError();
     hash_bytes = 0;
-    e = device_blocks().take(device, total, &arrays, &array_bytes);
+    e = device_blocks().take(device, total + 256, &arrays, &array_bytes);
   }
-  if (e != cudaSuccess) return cuda_fail(e, "graph arrays");
+  if (e != cudaSuccess) return checked(cuda_fail(e, "graph arrays"));
   if (labels) {
     e = pinned_blocks().take(device, dev_build ? (size_t)std::max<int64_t>(n, 1) : total - o_label, &stage,
                              &stage_bytes);
@@ -665,39 +828,54 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   if (e == cudaSuccess && nedges)
     e = cudaMemcpyAsync(g->colidx, colidx, sizeof(int32_t) * nedges, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(g->colidx + nedges, 0x7f, sizeof(int32_t) * kColPad, st);
-  if (e == cudaSuccess && n > 0) {
-    (void)cudaGetLastError();  // the check below must see these launches' errors only
-    const int threads = 256;
-    const int64_t want = ((int64_t)n * 32 + threads - 1) / threads;
-    const int blocks = (int)std::min<int64_t>(want, 148 * 16);
-    build_src_kernel<<<blocks, threads, 0, st>>>(g->rowptr, (int32_t)n, g->src);
-    max_nbr_deg_kernel<<<blocks, threads, 0, st>>>(g->rowptr, g->colidx, (int32_t)n, g->maxnd);
-    e = cudaGetLastError();
+  auto *lab8 = static_cast<uint8_t *>(stage);
+  CsrCheck ck{0, max_degree, 0};
+  if (e == cudaSuccess && check) {
+    // nothing below may read rows that break the rules: wait for the verdict
+    // (and narrow the labels meanwhile)
+    auto *dck = reinterpret_cast<CsrCheck *>(base + total + hash_bytes + 128);
+    e = cudaMemsetAsync(dck, 0, sizeof *dck, st);
+    if (e == cudaSuccess) {
+      (void)cudaGetLastError();  // the check below must see this launch's error only
+      const int blocks = (int)std::min<int64_t>((std::max(n, nedges) + 255) / 256 + 1, 148 * 8);
+      check_csr_kernel<<<blocks, 256, 0, st>>>(g->rowptr, g->colidx, n, nedges, dck);
+      e = cudaGetLastError();
+    }
+    if (labels)
+      for (int64_t i = 0; i < n; ++i) lab8[i] = (uint8_t)labels[i];
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&ck, dck, sizeof ck, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && ck.kind) {
+      pinned_blocks().give(device, stage, stage_bytes);
+      device_blocks().give(device, arrays, array_bytes);
+      delete g;
+      return csr_fault(ck.kind, ck.row);
+    }
+    g->max_degree = ck.max_degree;
+  } else if (labels) {
+    for (int64_t i = 0; i < n; ++i) lab8[i] = (uint8_t)labels[i];
   }
-  if (e == cudaSuccess && g->hash &&
-      build_row_tables(g->rowptr, g->colidx, g->src, n, nedges, g->hash, g->loops, st) != TDFS_OK)
-    e = cudaErrorUnknown;
+  if (g->max_degree > kFlatMaxDegree) g->hash = nullptr;  // the flat kernel's positions would not fit 32 bits
+  Rows R{g->rowptr, g->colidx, (int32_t)n, g->src, g->maxnd, g->hash, g->loops, nullptr, 0, nullptr, nullptr};
+  if (e == cudaSuccess && !nlab && run_rows(R, nedges, st) != TDFS_OK) e = cudaErrorUnknown;
   std::unique_ptr<LabelIndex> lindex;
   if (e == cudaSuccess && labels) {
     char *h = static_cast<char *>(stage);
-    auto *lab8 = reinterpret_cast<uint8_t *>(h);
-    for (int64_t i = 0; i < n; ++i) lab8[i] = (uint8_t)labels[i];
     lindex.reset(new LabelIndex);
     lindex->nl = nl;
     lindex->nedges = nedges;
     if (dev_build) {
-      // label rows and label index by the kernels above, after the CSR's
-      // preprocessing in stream order; the host keeps the group offsets
+      // label rows and label index by the kernels above; the host keeps the
+      // group offsets
       lindex->dev_perm = g->lperm;
       lindex->off.assign((size_t)G + 1, 0);
       e = cudaMemcpyAsync(g->label, lab8, (size_t)n, cudaMemcpyHostToDevice, st);
       if (e == cudaSuccess) e = cudaMemsetAsync(g->colidx_l + nedges, 0x7f, sizeof(int32_t) * kColPad, st);
-      if (e == cudaSuccess && n > 0) {
-        const int blocks = (int)std::min<int64_t>((n + kBuildWarps - 1) / kBuildWarps, 148 * 16);
-        label_rows_kernel<<<blocks, 32 * kBuildWarps, 0, st>>>(g->rowptr, g->colidx, g->label, (int32_t)n, nl,
-                                                              g->colidx_l, g->loff);
-        e = cudaGetLastError();
-      }
+      R.lab = g->label;
+      R.nl = nl;
+      R.col_l = g->colidx_l;
+      R.loff = g->loff;
+      if (e == cudaSuccess && run_rows(R, nedges, st) != TDFS_OK) e = cudaErrorUnknown;
       if (e == cudaSuccess && ntiles > 0) {
         auto *hist = reinterpret_cast<int32_t *>(base + o_hist);
         auto *goff = reinterpret_cast<int64_t *>(base + o_goff);

@@ -179,20 +179,20 @@ struct tdfs_graph {
 
 namespace tdfs {
 
+// check: the rows were not checked yet (validate_csr); max_degree is then taken
+// from the rows.
 int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx, const int32_t *labels,
-                 int device, int32_t max_degree, tdfs_graph **out);
+                 int device, int32_t max_degree, bool check, tdfs_graph **out);
 void graph_release(tdfs_graph *g);
 // Give g a launch workspace from its device's pool (allocating one when none
 // is idle); the device must be current.  Idempotent.
 int acquire_workspace(tdfs_graph *g);
 void release_graphs(tdfs_graph *g);  // capi.cpp: destroys cached launch graphs
 DevGraph graph_view(const tdfs_graph *g);
-// Row membership tables (common.h, row_table_buckets) of a graph whose `src`
-// array is built, into `hash`, and the self-loop flag; stream-ordered.
-int build_row_tables(const int64_t *rowptr, const int32_t *colidx, const int32_t *src, int64_t n, int64_t nedges,
-                     int32_t *hash, int32_t *loops, cudaStream_t st);
-int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, const int32_t *labels,
-                         int32_t *src, int32_t *maxnd, uint8_t *label8, int32_t *bad, cudaStream_t st);
+// hash (with loops) may be nullptr: no row membership tables.
+int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, int64_t nedges,
+                         const int32_t *labels, int32_t *src, int32_t *maxnd, uint8_t *label8, int32_t *bad,
+                         int32_t *hash, int32_t *loops, cudaStream_t st);
 inline QueueHdr *queue_hdr(tdfs_graph *g) { return reinterpret_cast<QueueHdr *>(g->queue + kQueueCap); }
 
 }  // namespace tdfs

@@ -146,8 +146,8 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   int32_t *bad = reinterpret_cast<int32_t *>(base + L.bad);
   e = cudaMemsetAsync(bad, 0, sizeof(int32_t), st);
   if (e != cudaSuccess) return cuda_fail_static("scratch clear: %s", e);
-  int rc = prepare_graph_arrays(d_rowptr, d_colidx, (int32_t)n, plan.labeled ? d_labels : nullptr, src, maxnd,
-                                label8, bad, st);
+  int rc = prepare_graph_arrays(d_rowptr, d_colidx, (int32_t)n, nedges, plan.labeled ? d_labels : nullptr, src,
+                                maxnd, label8, bad, nullptr, nullptr, st);
   if (rc) return rc;
   DevGraph g;
   g.rowptr = d_rowptr;

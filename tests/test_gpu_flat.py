@@ -124,3 +124,54 @@ def test_level_two_in_global_memory(T):
         assert want > 0
         for opt in ({}, {"split_after_us": -1, "edge_chunk": 1}, {"warps_per_block": 2, "chunk_cap": 64}):
             assert T.count(dev, P, T.default_options(**opt)).count == want, (text, opt)
+
+
+def test_rows_that_break_the_rules_are_refused(T):
+    """The CSR's rules, checked on the device: the error and what it says are
+    those of the host's check, at the edges of rows, blocks and the arrays."""
+    rowptr, colidx = edge_graph()
+    n, E = len(rowptr) - 1, len(colidx)
+    good = T.GraphPreprocessor(rowptr=rowptr, colidx=colidx)
+    assert good.max_degree == int(np.diff(rowptr).max())
+    rows = [v for v in range(n) if rowptr[v + 1] - rowptr[v] >= 2]
+    for v in (rows[0], rows[len(rows) // 2], rows[-1]):
+        b, e = int(rowptr[v]), int(rowptr[v + 1])
+        for at, val, what in ((b, -1, "out of range"), (e - 1, n, "out of range"), (b + 1, colidx[b], "strictly increasing")):
+            c = colidx.copy()
+            c[at] = val
+            with pytest.raises(T.TdfsError) as ei:
+                T.GraphPreprocessor(rowptr=rowptr, colidx=c)
+            assert ei.value.code == 2 and what in str(ei.value) and f"row {v}" in str(ei.value)
+        r = rowptr.copy()
+        r[v + 1] = r[v] - 1 if r[v] else E + 5
+        with pytest.raises(T.TdfsError) as ei:
+            T.GraphPreprocessor(rowptr=r, colidx=colidx)
+        assert ei.value.code == 2 and "rowptr decreases" in str(ei.value)
+    for bad in (rowptr[:-1], rowptr + 1):  # the ends do not span the edges
+        with pytest.raises(T.TdfsError) as ei:
+            T.GraphPreprocessor(rowptr=bad, colidx=colidx)
+        assert ei.value.code == 2
+
+
+@pytest.mark.parametrize("nlabels", [1, 4, 16])
+def test_long_rows_are_split_over_a_block(T, po, nlabels):
+    """Rows around the length from which a whole CTA takes them (512) and far
+    beyond: sources, neighbour degrees, tables and label segments, through
+    the counts that use them."""
+    n, rng, e = 3000, np.random.default_rng(nlabels), set()
+    for h, d in enumerate((511, 512, 513, 1024, 2600)):
+        for v in rng.choice(np.arange(10, n), d, replace=False):
+            e |= {(h, int(v)), (int(v), h)}
+    for a, b in rng.integers(5, n, (4000, 2)):
+        if a != b:
+            e |= {(int(a), int(b)), (int(b), int(a))}
+    rowptr, colidx = csr(e, n)
+    labels = rng.integers(0, nlabels, n).astype(np.int32)
+    labels[0] = nlabels - 1
+    dev = T.GraphPreprocessor(rowptr=rowptr, colidx=colidx, labels=labels, labeled=True)
+    ora = po.Graph(rowptr.copy(), colidx.copy(), labels.copy())
+    r = random.Random(nlabels)
+    for text, labeled in [(TRIANGLE, False), (CYCLE4, False)] + [(random_pattern(3 + i % 3, 0.5, nlabels, r), True)
+                                                                for i in range(5)]:
+        P = T.PatternPreprocessor(text=text, labeled=labeled)
+        assert T.count(dev, P).count == po.count(ora, po.Plan(text, labeled)), (text, labeled)
