@@ -95,9 +95,9 @@ struct FlatTable {
   FlatBox *box;
   int32_t *big;  // kBigBytes per warp, or nullptr
 
-  static size_t at_ctl(int n) { return sizeof(RunCtl) + (((size_t)n * 8 + 127) & ~size_t(127)); }
-  static size_t readback(int n) { return sizeof(RunCtl) + (size_t)n * 8; }
-  static size_t bytes(int n) {
+  static constexpr size_t at_ctl(int n) { return sizeof(RunCtl) + (((size_t)n * 8 + 127) & ~size_t(127)); }
+  static constexpr size_t readback(int n) { return sizeof(RunCtl) + (size_t)n * 8; }
+  static constexpr size_t bytes(int n) {
     return at_ctl(n) + sizeof(FlatCtl) + 4 * kIdleWords + (size_t)n * (sizeof(FlatInfo) + sizeof(FlatPlan));
   }
   // The views of the block at `base` (device, or its host image).

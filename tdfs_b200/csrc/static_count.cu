@@ -3,7 +3,7 @@
 // Some callers cannot call cudaMalloc: a host process whose device memory is
 // carved up by another runtime (an inference server's caching allocator, a
 // plugin loaded into an application that owns every byte of the GPU).  For them,
-// tdfs_count_static runs the same match kernel as tdfs_count with all of its
+// tdfs_count_static runs the same kernels as tdfs_count with all of its
 // working memory taken from one fixed array that lives in the library's
 // device image: kScratchBytes per GPU, held from the first use of the library
 // on that GPU until the process exits.
@@ -44,6 +44,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "flat.cuh"
 #include "graph.h"
 #include "match.cuh"
 #include "plan.h"
@@ -72,6 +73,7 @@ int cuda_fail_static(const char *what, cudaError_t e) {
 // Fixed layout of the array (offsets in bytes).
 struct Layout {
   size_t ctl, bad, units, qhdr, tab, src, maxnd, label, end;
+  size_t hash, hash_end;  // the row membership tables, where they fit (the flat kernel's launches)
 };
 
 Layout layout(int64_t n, int64_t nedges) {
@@ -86,6 +88,8 @@ Layout layout(int64_t n, int64_t nedges) {
   L.maxnd = o; o = align_up(o + sizeof(int32_t) * (size_t)(n > 0 ? n : 1));
   L.label = o; o = align_up(o + (size_t)(n > 0 ? n : 1));
   L.end = o;
+  L.hash = o;
+  L.hash_end = o + 4 * kBucket * (size_t)row_table_buckets(n, nedges > 0 ? nedges : 0);
   return L;
 }
 
@@ -132,6 +136,10 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
     if (cs != cudaStreamCaptureStatusNone)
       return fail(TDFS_ERR_ARG, "tdfs_count_static cannot be called on a stream that is being captured");
   }
+  // the flat kernel, where the plan has its form and the row membership tables
+  // fit the array too
+  const FlatPlan *fp = plan_flat_table(p);
+  const bool flat = fp && flat_options(o) && L.hash_end <= kScratchBytes;
   // 16-byte window loads may round the last list's end up to 4 ints: without
   // that slack after colidx[E-1], search the lists directly instead
   if (nedges % 4 != 0) o.merge_window = -1;
@@ -144,10 +152,12 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   uint8_t *label8 = plan.labeled ? reinterpret_cast<uint8_t *>(base + L.label) : nullptr;
   // derived graph arrays, written into the scratch (each call recomputes them)
   int32_t *bad = reinterpret_cast<int32_t *>(base + L.bad);
-  e = cudaMemsetAsync(bad, 0, sizeof(int32_t), st);
+  int32_t *loops = bad + 1;
+  e = cudaMemsetAsync(bad, 0, 2 * sizeof(int32_t), st);
   if (e != cudaSuccess) return cuda_fail_static("scratch clear: %s", e);
   int rc = prepare_graph_arrays(d_rowptr, d_colidx, (int32_t)n, nedges, plan.labeled ? d_labels : nullptr, src,
-                                maxnd, label8, bad, nullptr, nullptr, st);
+                                maxnd, label8, bad, flat ? reinterpret_cast<int32_t *>(base + L.hash) : nullptr,
+                                flat ? loops : nullptr, st);
   if (rc) return rc;
   DevGraph g;
   g.rowptr = d_rowptr;
@@ -158,13 +168,13 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   g.lperm = nullptr;  // no label index here: labeled slots walk the edge ids
   g.colidx_l = nullptr;  // nor label-partitioned rows: labeled plans test labels per candidate
   g.loff = nullptr;
-  g.hash = nullptr;
-  g.loops = nullptr;
+  g.hash = flat ? reinterpret_cast<int32_t *>(base + L.hash) : nullptr;
+  g.loops = flat ? loops : nullptr;
   g.nlab = 0;
   g.nedges = nedges;
   g.n = (int32_t)n;
   g.max_degree = 0;
-  LaunchShape s;
+  LaunchShape s;     // (checks the options for either kernel)
   tdfs_graph probe;  // launch_shape reads only the device index
   std::memset(&probe, 0, sizeof probe);
   probe.device = device;
@@ -176,6 +186,40 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   const int64_t ee = std::max(eb, (o.edge_end < 0 || o.edge_end > nedges) ? nedges : o.edge_end);
   const int stride = o.edge_stride > 0 ? o.edge_stride : 1;
   if (o.edge_phase < 0 || o.edge_phase >= stride) return fail(TDFS_ERR_ARG, "edge_phase must lie in [0, edge_stride)");
+  int32_t h_bad = 0;
+  if (flat) {
+    FlatShape fs;
+    if ((rc = flat_shape(device, fp->s - 1, fp->t, false, false, plan.labeled != 0, o, &fs))) return rc;
+    constexpr size_t kImage = FlatTable::bytes(1);
+    alignas(128) unsigned char image[kImage] = {};
+    const FlatTable h = FlatTable::of(image, 1, nullptr, nullptr);
+    h.ctl->ticket = (unsigned long long)fs.blocks * fs.warps_per_block;
+    h.ctl->pending = fs.blocks;
+    h.ctl->slots = 1;
+    FlatInfo &in = h.info[0];
+    in.e_begin = eb;
+    in.e_end = ee;
+    in.stride = stride;
+    in.phase = o.edge_phase;
+    in.chunk = flat_chunk(ee - eb, fp->s, stride, fs.blocks * fs.warps_per_block, o.edge_chunk);
+    const int64_t chunks = (ee - eb + in.chunk - 1) / in.chunk;
+    h.ctl->tickets = chunks <= o.edge_phase ? 0 : (chunks - o.edge_phase + stride - 1) / stride;
+    h.plan[0] = *fp;
+    const FlatTable d = FlatTable::of(tab, 1, reinterpret_cast<FlatBox *>(units), nullptr);
+    e = cudaMemcpyAsync(tab, image, kImage, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return cuda_fail_static("slot upload: %s", e);
+    if ((rc = launch_flat(plan.labeled != 0, g, d, fs.cfg, fs.blocks, fs.warps_per_block, st))) return rc;
+    e = cudaMemcpyAsync(image, tab, FlatTable::readback(1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && plan.labeled)
+      e = cudaMemcpyAsync(&h_bad, bad, sizeof h_bad, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail_static("flat kernel: %s", e);
+    if (h_bad) return fail(TDFS_ERR_FORMAT, "vertex labels must lie in [0, 254]");
+    if (h.run->error) return fail(h.run->error, "device error %d", h.run->error);
+    if (!h.run->finished) return fail(TDFS_ERR_TIMEOUT, "the query did not complete");
+    *count = (uint64_t)(h.count[0] * (unsigned long long)plan.multiplicity);
+    return TDFS_OK;
+  }
   SlotCtl h_ctl;
   SlotHot h_hot;
   SlotInfo h_info;
@@ -203,7 +247,6 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   init_launch(ctl, qh, st);  // clears the control block and the split ring
   rc = launch_match(plan.labeled != 0, g, ctl, tab, units, qh, s.cfg, s.blocks, s.warps_per_block, st);
   if (rc) return rc;
-  int32_t h_bad = 0;
   e = cudaMemcpyAsync(&h_hot, &tab->hot[0], sizeof h_hot, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h_bad, bad, sizeof h_bad, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&h_run, ctl, sizeof h_run, cudaMemcpyDeviceToHost, st);
