@@ -331,10 +331,17 @@ struct Flat {
   // mode 0: stored as entries of level L + 1 (until that buffer is full);
   // mode 1: counted into `count`; mode 2: counted per entry into sizes[].
   // Modes 0 and 1 resume at, and leave, the block's position in W.lev[L]; they
-  // return false when they stopped early because a warp is idle and there are
-  // entries to give it.
-  template <int mode>
-  __device__ __forceinline__ bool scan(const FlatStep &st, int L, uint32_t *sizes) {
+  // stop early (false) when a warp is idle and there are entries to give it.
+  // FIXED -1: the mode is an argument and one copy of this code serves all
+  // three.  Labeled launches take it: the warps of an SM run many small plans
+  // there, and with a copy per mode the kernel outgrew the instruction cache
+  // (no_instruction 10.6 cycles per issue; power-law labeled batch 3.62 against
+  // 2.92 ms, ER 0.187 against 0.150).  Unlabeled ones run long scans of few
+  // plans and do better without the mode's tests in the step (5-clique share
+  // 21.4 against 25.1 ms).
+  template <int FIXED>
+  __device__ __forceinline__ bool scan(const FlatStep &st, int L, int how, uint32_t *sizes) {
+    const int mode = FIXED >= 0 ? FIXED : how;
     FlatLevel &H = W.lev[L];
     const int first = H.next;
     int len = 0;
@@ -463,11 +470,10 @@ struct Flat {
     return !early;
   }
 
-  // Fill level L + 1 from the entries of level L; `more`: go on filling.
-  // Returns true when it stopped early.
-  __device__ bool expand(int L, bool more) {
+  // Start filling level L + 1 from the entries of level L.
+  __device__ void fill_begin(int L) {
     FlatLevel &H = W.lev[L], &D = W.lev[L + 1];
-    if (lane == 0 && !more) {
+    if (lane == 0) {
       D.next = D.end = D.n = 0;
       D.pos = 0;
       D.started = 0;
@@ -476,8 +482,10 @@ struct Flat {
       D.groups = 1;
     }
     __syncwarp();
-    while (H.next < H.end && D.n <= room(L + 1))
-      if (!scan<0>(W.plan.step[L - 1], L, nullptr)) return true;
+  }
+  // Level L + 1 is full, or level L has no entries left.
+  __device__ void fill_end(int L) {
+    FlatLevel &H = W.lev[L], &D = W.lev[L + 1];
     if (lane == 0) {
       D.end = D.n;
       D.tcut = H.pos ? H.cutp : -1;
@@ -493,7 +501,6 @@ struct Flat {
       }
     }
     __syncwarp();
-    return false;
   }
 
   // Entries of the ascending x[0, n) below v.
@@ -529,58 +536,80 @@ struct Flat {
     return (uint32_t)c;
   }
 
-  // Count below a block of level-s entries.
-  __device__ void leaf(int L) {
+  // Single lists are counted in closed form, except on whole rows with labels.
+  __device__ __forceinline__ bool closed(const FlatStep &st) const { return st.nbn == 1 && (!LAB || segmented()); }
+
+  // The tuples of distinct vertices below this lane's entry, from the sizes of
+  // the tail's sets in cnt().
+  __device__ __forceinline__ unsigned long long tuples() const {
+    const FlatPlan &F = W.plan;
+    auto at = [&](int m) -> unsigned long long {
+      const int u = F.term_of[m];
+      return u == kNoTerm ? 0ull : (unsigned long long)cnt(u)[lane];
+    };
+    const unsigned long long a = at(1);
+    if (F.form == 1) return F.t == 2 ? a * (a - 1) / 2 : a * (a - 1) / 2 * (a - 2) / 3;
+    const unsigned long long b = at(2);
+    if (F.t == 2) return a * b - at(3);
+    const unsigned long long c = at(4);
+    return a * b * c - at(3) * c - at(5) * b - at(6) * a + 2 * at(7);
+  }
+
+  // One block of level L: extended into level L + 1, or, at level s, counted.
+  // `filling`: level L + 1 is being filled.  Returns whether it still is.
+  __device__ bool advance(int L, bool filling) {
     FlatLevel &H = W.lev[L];
     const FlatPlan &F = W.plan;
-    const bool single = !LAB || segmented();  // single lists are counted in closed form
-    if (F.t == 1 && !(F.term[0].nbn == 1 && single)) {
-      scan<1>(F.term[0], L, nullptr);
-      return;
+    const bool leaf = L == F.s, tail = leaf && F.t > 1;
+    if (!leaf && !filling) fill_begin(L);
+    if (!LAB && !leaf) {
+      while (H.next < H.end && W.lev[L + 1].n <= room(L + 1))
+        if (!scan<0>(F.step[L - 1], L, 0, nullptr)) return true;
+      fill_end(L);
+      return false;
+    }
+    if (!LAB && F.t == 1 && !closed(F.term[0])) {
+      scan<1>(F.term[0], L, 1, nullptr);
+      return false;
     }
     const int p = H.next + lane;
     const bool mine = p < H.end;
-    if (F.t == 1 && mine) {
-      load_tuple(L, p, 0);
-      count += closed_count(F.term[0]);
-    }
-    for (int u = 0; F.t > 1 && u < F.nterm; ++u) {
-      const FlatStep &st = F.term[u];
-      uint32_t c = 0;
-      if (st.nbn == 1 && single) {
+    bool scanned = false;
+    const int sets = tail ? F.nterm : 1;
+    for (int u = 0; u < sets; ++u) {
+      const FlatStep &st = leaf ? F.term[u] : F.step[L - 1];
+      if (leaf && closed(st)) {
+        uint32_t c = 0;
         if (mine) {
           load_tuple(L, p, 0);
           c = closed_count(st);
         }
-        cnt(u)[lane] = c;
+        if (tail) cnt(u)[lane] = c;
+        else count += c;
       } else {
-        cnt(u)[lane] = 0;
+        if (tail) cnt(u)[lane] = 0;
         __syncwarp();
-        scan<2>(st, L, cnt(u));
+        if (LAB) scan<-1>(st, L, tail ? 2 : leaf ? 1 : 0, tail ? cnt(u) : nullptr);
+        else scan<2>(st, L, 2, cnt(u));
+        scanned = true;
       }
       __syncwarp();
     }
-    if (F.t > 1 && mine) {
-      auto at = [&](int m) -> unsigned long long {
-        const int u = F.term_of[m];
-        return u == kNoTerm ? 0ull : (unsigned long long)cnt(u)[lane];
-      };
-      const unsigned long long a = at(1);
-      if (F.form == 1) {
-        count += F.t == 2 ? a * (a - 1) / 2 : a * (a - 1) / 2 * (a - 2) / 3;
-      } else if (F.t == 2) {
-        count += a * at(2) - at(3);
-      } else {
-        const unsigned long long b = at(2), c = at(4);
-        count += a * b * c - at(3) * c - at(5) * b - at(6) * a + 2 * at(7);
+    if (LAB && !leaf) {
+      if (H.next < H.end && W.lev[L + 1].n <= room(L + 1)) return true;
+      fill_end(L);
+      return false;
+    }
+    if (tail && mine) count += tuples();
+    __syncwarp();
+    if (tail || !scanned) {  // the whole block is done (a scan of mode 1 keeps its own place)
+      if (lane == 0) {
+        H.next = min(H.next + 32, H.end);
+        H.started = H.next;
       }
+      __syncwarp();
     }
-    __syncwarp();
-    if (lane == 0) {
-      H.next = min(H.next + 32, H.end);
-      H.started = H.next;
-    }
-    __syncwarp();
+    return false;
   }
 
   // ---- query slots -------------------------------------------------------------
@@ -905,12 +934,9 @@ struct Flat {
         --level;
         continue;
       }
-      if (level == W.plan.s) {
-        leaf(level);
-      } else {
-        more = expand(level, more);
-        if (!more && W.lev[level + 1].n > 0) ++level;
-      }
+      const bool inner = level < W.plan.s;
+      more = advance(level, more);
+      if (inner && !more && W.lev[level + 1].n > 0) ++level;
       const long long c = clock64();
       int due = 0;
       if (c - checked > kCheckCycles) {
