@@ -224,7 +224,8 @@ struct Launch {
   int warps() const { return flat ? fl.blocks * fl.warps_per_block : dfs.blocks * dfs.warps_per_block; }
 };
 
-// Captured launches: one CUDA graph per (batch size, mode, launch shape)
+// Captured launches: one CUDA graph per (batch size, mode, launch shape), made
+// at the shape's second launch (exec is null until then),
 // holding the slot-table upload from the pinned staging copy, the control
 // reset, the kernel and the read-back; replays read the staging copy as it is
 // at replay time.
@@ -242,6 +243,7 @@ void release_graphs(tdfs_graph *g) {
   if (!g->graphs) return;
   auto *v = static_cast<std::vector<GraphEntry> *>(g->graphs);
   for (auto &c : *v) {
+    if (!c.exec) continue;
     cudaGraphExecDestroy(c.exec);
     cudaEventDestroy(c.k0);
     cudaEventDestroy(c.k1);
@@ -331,6 +333,25 @@ int collect(tdfs_graph *g, int n, bool flat, unsigned long long *raw, int *statu
   return TDFS_OK;
 }
 
+int run_plain(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStream_t st, float *ms,
+              unsigned long long *raw, int *status) {
+  cudaError_t e;
+  if (ms)
+    for (void *&ev : g->ws->ev)
+      if (!ev) {
+        cudaEvent_t x;
+        if ((e = cudaEventCreate(&x)) != cudaSuccess) return cuda_err(e, "cudaEventCreate");
+        ev = x;
+      }
+  const cudaEvent_t k0 = ms ? static_cast<cudaEvent_t>(g->ws->ev[0]) : nullptr;
+  const cudaEvent_t k1 = ms ? static_cast<cudaEvent_t>(g->ws->ev[1]) : nullptr;
+  if (const int rc = enqueue_launch(g, L, labeled, n, st, k0, k1, cudaEventRecordDefault)) return rc;
+  e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, k0, k1);
+  if (e != cudaSuccess) return cuda_err(e, "match kernel");
+  return collect(g, n, L.flat, raw, status);
+}
+
 int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms, unsigned long long *raw,
                  int *status) {
   cudaError_t e;
@@ -342,12 +363,19 @@ int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms,
   }
   cudaStream_t st = static_cast<cudaStream_t>(g->ws->gstream);
   auto &cache = graph_cache(g);
-  const GraphEntry *hit = nullptr;
+  GraphEntry *hit = nullptr;
   for (auto &c : cache)
     if (c.n == n && c.labeled == labeled && !std::memcmp(&c.launch, &L, sizeof L))
       hit = &c;
   if (!hit) {
-    GraphEntry ent{n, labeled, L, nullptr, nullptr, nullptr};
+    // a shape's first launch on this graph runs without a capture: capturing,
+    // instantiating and destroying a graph costs 280 us, and a request that
+    // opens a graph, counts once and frees it would pay that for nothing
+    cache.push_back(GraphEntry{n, labeled, L, nullptr, nullptr, nullptr});
+    return run_plain(g, L, labeled, n, st, ms, raw, status);
+  }
+  if (!hit->exec) {
+    GraphEntry ent = *hit;
     e = cudaEventCreate(&ent.k0);
     if (e == cudaSuccess) e = cudaEventCreate(&ent.k1);
     if (e != cudaSuccess) return cuda_err(e, "cudaEventCreate");
@@ -365,8 +393,7 @@ int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms,
       cudaEventDestroy(ent.k1);
       return rc ? rc : cuda_err(e, "capturing the launch");
     }
-    cache.push_back(ent);
-    hit = &cache.back();
+    *hit = ent;
   }
   e = cudaGraphLaunch(hit->exec, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -480,21 +507,7 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
   if (flat) fill_flat(g, plans, n, o, eb, ee, stride, L);
   else fill_slots(g, plans, n, o, eb, ee, stride, warps);
   if (o.graph_capture) return run_captured(g, L, labeled, n, ms, raw, status);
-  cudaStream_t st = static_cast<cudaStream_t>(o.stream);
-  if (ms)
-    for (void *&ev : g->ws->ev)
-      if (!ev) {
-        cudaEvent_t x;
-        if ((e = cudaEventCreate(&x)) != cudaSuccess) return cuda_err(e, "cudaEventCreate");
-        ev = x;
-      }
-  const cudaEvent_t k0 = ms ? static_cast<cudaEvent_t>(g->ws->ev[0]) : nullptr;
-  const cudaEvent_t k1 = ms ? static_cast<cudaEvent_t>(g->ws->ev[1]) : nullptr;
-  if ((rc = enqueue_launch(g, L, labeled, n, st, k0, k1, cudaEventRecordDefault))) return rc;
-  e = cudaStreamSynchronize(st);
-  if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, k0, k1);
-  if (e != cudaSuccess) return cuda_err(e, "match kernel");
-  return collect(g, n, flat, raw, status);
+  return run_plain(g, L, labeled, n, static_cast<cudaStream_t>(o.stream), ms, raw, status);
 }
 
 }  // namespace
