@@ -1044,17 +1044,22 @@ int flat_blocks_per_sm(bool labeled, bool wide, bool big, int warps_per_block, s
   return labeled ? flat_fit<true, 4, false>(threads, smem) : flat_fit<false, 4, false>(threads, smem);
 }
 
-int flat_chunk(int64_t edges, int s, int stride, int warps, int edge_chunk) {
+int flat_chunk(int64_t edges, int s, bool skewed, int stride, int warps, int edge_chunk) {
   if (edge_chunk > 0) return edge_chunk;
   if (stride > 1) return 32;  // the documented round-robin deal
-  // Full lanes at the first levels against even shares: a plan counted at its
+  // Full lanes at the first levels against even shares.  A plan counted at its
   // edges has little work per edge and wants all 32 lanes (triangles of the
-  // n=4096 ER graph: 87 us with 1 edge per ticket, 39 with 4, 25 with 32);
-  // each level more multiplies an edge's work, and the wider the spread.
-  int c = s <= 1 ? 32 : s == 2 ? 8 : 2;
-  // at least two tickets per warp; a quarter of the warps suffices for the
-  // light edges of s = 1
-  while (c > 1 && edges / c < (s <= 1 ? warps / 4 : 2ll * warps)) c >>= 1;
+  // n=4096 ER graph: 87 us with 1 edge per ticket, 39 with 4, 25 with 32); each
+  // level more multiplies an edge's work (64-query burst, s up to 4: 0.50 ms
+  // with 1, 0.17 with 4, 0.17 with 8).  Where hubs make some edges thousands of
+  // times heavier than others, consecutive ones (a hub's) go to different
+  // warps: power-law labeled batch 2.6 ms with 1, 3.0 with 4; triangles 0.16
+  // with 4, 0.22 with 32.
+  int c = s <= 1 ? (skewed ? 8 : 32) : s == 2 ? 8 : skewed ? 1 : 4;
+  // enough tickets to even the warps out; a quarter of the warps suffices for
+  // the light edges of s = 1
+  const int64_t least = s <= 1 ? warps / 4 : s == 2 ? 2ll * warps : 3ll * warps;
+  while (c > 1 && edges / c < least) c >>= 1;
   return c;
 }
 

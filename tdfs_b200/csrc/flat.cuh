@@ -121,9 +121,10 @@ struct FlatTable {
 inline int flat_max_blocks(int warps_per_block) { return kFlatBoxes / warps_per_block; }
 
 // Level-0 edges per ticket of a slot whose plan is enumerated down to level s,
-// in a launch of `edges` level-0 edges over all slots; `edge_chunk` and
-// `stride` as in tdfs_options.
-int flat_chunk(int64_t edges, int s, int stride, int warps, int edge_chunk);
+// in a launch of `edges` level-0 edges over all slots; skewed: on a graph with
+// hubs (kHubDegree); `edge_chunk` and `stride` as in tdfs_options.
+constexpr int32_t kHubDegree = 512;
+int flat_chunk(int64_t edges, int s, bool skewed, int stride, int warps, int edge_chunk);
 
 // Launch over the slots of `t` (on the device).
 int launch_flat(bool labeled, const DevGraph &g, const FlatTable &t, const FlatCfg &cfg, int blocks,

@@ -201,7 +201,7 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
     in.e_end = ee;
     in.stride = stride;
     in.phase = o.edge_phase;
-    in.chunk = flat_chunk(ee - eb, fp->s, stride, fs.blocks * fs.warps_per_block, o.edge_chunk);
+    in.chunk = flat_chunk(ee - eb, fp->s, false, stride, fs.blocks * fs.warps_per_block, o.edge_chunk);
     const int64_t chunks = (ee - eb + in.chunk - 1) / in.chunk;
     h.ctl->tickets = chunks <= o.edge_phase ? 0 : (chunks - o.edge_phase + stride - 1) / stride;
     h.plan[0] = *fp;
