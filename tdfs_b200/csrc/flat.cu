@@ -859,6 +859,12 @@ struct Flat {
     int st = 0;  // 1: the mailbox is full, 2: stop
     const unsigned long long t0 = now_ns();
     flush();
+    if (!cfg.share) {
+      // light, even work: nothing to wait for
+      if (lane == 0 && atomicSub(&C.active, 1) == 1 && atomicSub(&T.ctl->pending, 1) == 1) T.run->finished = 1;
+      __syncwarp();
+      return 0;
+    }
     if (lane == 0) {
       *(volatile int32_t *)&T.box[gid].full = 0;
       __threadfence();
@@ -945,7 +951,8 @@ struct Flat {
       }
       if (__shfl_sync(kFull, due, 0)) donate(base, level);
     }
-    // the CTA's sums, by its last warp
+    // the CTA's sums, by its last warp; the results, by the grid's
+    int last = 0;
     if (lane == 0) {
       atomicAdd(&C.idle_ns, W.idle_total);
       atomicAdd(&C.warp_ns, now_ns() - W.t_start);
@@ -955,7 +962,17 @@ struct Flat {
         if (C.sum) atomicAdd(&T.count[C.slot], C.sum);
         atomicAdd(&T.run->idle_ns, C.idle_ns);
         atomicAdd(&T.run->warp_ns, C.warp_ns);
+        if (T.host) {
+          __threadfence();
+          last = atomicAdd(&T.ctl->gone, 1) == (int)gridDim.x - 1;
+        }
       }
+    }
+    if (__shfl_sync(kFull, last, 0)) {
+      __threadfence();
+      const int words = (int)(FlatTable::readback(T.ctl->slots) / 4);
+      for (int i = lane; i < words; i += 32)
+        static_cast<volatile int32_t *>(T.host)[i] = __ldcg(reinterpret_cast<const int32_t *>(T.run) + i);
     }
   }
 };

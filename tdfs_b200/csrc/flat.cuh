@@ -23,6 +23,7 @@ struct FlatCfg {
   int32_t split_ns;    // work may be given away after this long on one base subtree
   int32_t segments;    // 1: labeled plans read the label segments of rows (DevGraph::colidx_l)
   int32_t wide;        // 1: the 80-register build (3 CTAs of 256 threads per SM)
+  int32_t share;       // 1: idle warps wait to be given work; 0: they leave
 };
 
 // Vertices up to this degree: 32 lists laid end to end stay within 32 bits.
@@ -43,7 +44,9 @@ int flat_blocks_per_sm(bool labeled, bool wide, bool big, int warps_per_block, s
 // What a launch over n slots reads and writes besides the graph, in one block
 // that the host fills and uploads with one copy:
 //   RunCtl | count[n] | FlatCtl | mask of idle warps | FlatInfo[n] | FlatPlan[n]
-// The first two come back with one copy.
+// The first two come back with one copy, or, with FlatTable::host set, are
+// written to (pinned) host memory by the last CTA: a copy after the kernel
+// costs a small launch 4 us more.
 constexpr int kFlatBoxes = 8192;  // mailboxes, one per warp of the grid
 constexpr int kIdleWords = kFlatBoxes / 32;
 
@@ -52,6 +55,8 @@ struct alignas(128) FlatCtl {
   char pad0_[120];
   int32_t pending;            // CTAs with busy warps + filled mailboxes; 0 = the launch is complete
   char pad1_[124];
+  int32_t gone;               // CTAs that have left
+  char pad3_[124];
   int64_t tickets;            // tickets of all slots
   int32_t slots;
   char pad2_[116];
@@ -94,6 +99,7 @@ struct FlatTable {
   FlatPlan *plan;
   FlatBox *box;
   int32_t *big;  // kBigBytes per warp, or nullptr
+  void *host;    // where RunCtl and count[] go at the end, or nullptr
 
   static constexpr size_t at_ctl(int n) { return sizeof(RunCtl) + (((size_t)n * 8 + 127) & ~size_t(127)); }
   static constexpr size_t readback(int n) { return sizeof(RunCtl) + (size_t)n * 8; }
@@ -101,7 +107,7 @@ struct FlatTable {
     return at_ctl(n) + sizeof(FlatCtl) + 4 * kIdleWords + (size_t)n * (sizeof(FlatInfo) + sizeof(FlatPlan));
   }
   // The views of the block at `base` (device, or its host image).
-  static FlatTable of(void *base, int n, FlatBox *box, int32_t *big) {
+  static FlatTable of(void *base, int n, FlatBox *box, int32_t *big, void *host) {
     char *b = static_cast<char *>(base);
     FlatTable t;
     t.run = reinterpret_cast<RunCtl *>(b);
@@ -113,6 +119,7 @@ struct FlatTable {
     t.plan = reinterpret_cast<FlatPlan *>(t.info + n);
     t.box = box;
     t.big = big;
+    t.host = host;
     return t;
   }
 };

@@ -31,13 +31,15 @@ const FlatPlan *plan_flat_table(const tdfs_plan *p);
 // Launch shape of the flat kernel for plans enumerated down to level smax
 // (FlatPlan::s) with tails of up to tmax vertices, holding `levels` levels in
 // shared memory (big: and level 2 in global memory), on a skewed graph or not,
-// from the options launch_shape has accepted (capi.cpp).
+// idle warps waiting to be given work (share) or leaving, from the options
+// launch_shape has accepted (capi.cpp).
 struct FlatShape {
   int warps_per_block;
   int blocks;
   FlatCfg cfg;
 };
-int flat_shape(int device, int levels, int tmax, bool skewed, bool big, bool labeled, const tdfs_options &o, FlatShape *out);
+int flat_shape(int device, int levels, int tmax, bool skewed, bool big, bool share, bool labeled, const tdfs_options &o,
+               FlatShape *out);
 
 // Do these options leave the choice of the kernel to the library?  A work
 // budget, stealing switched off, or a value for one of the DFS kernel's own

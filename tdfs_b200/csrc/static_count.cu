@@ -189,10 +189,10 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
   int32_t h_bad = 0;
   if (flat) {
     FlatShape fs;
-    if ((rc = flat_shape(device, fp->s - 1, fp->t, false, false, plan.labeled != 0, o, &fs))) return rc;
+    if ((rc = flat_shape(device, fp->s - 1, fp->t, false, false, true, plan.labeled != 0, o, &fs))) return rc;
     constexpr size_t kImage = FlatTable::bytes(1);
     alignas(128) unsigned char image[kImage] = {};
-    const FlatTable h = FlatTable::of(image, 1, nullptr, nullptr);
+    const FlatTable h = FlatTable::of(image, 1, nullptr, nullptr, nullptr);
     h.ctl->ticket = (unsigned long long)fs.blocks * fs.warps_per_block;
     h.ctl->pending = fs.blocks;
     h.ctl->slots = 1;
@@ -205,7 +205,7 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
     const int64_t chunks = (ee - eb + in.chunk - 1) / in.chunk;
     h.ctl->tickets = chunks <= o.edge_phase ? 0 : (chunks - o.edge_phase + stride - 1) / stride;
     h.plan[0] = *fp;
-    const FlatTable d = FlatTable::of(tab, 1, reinterpret_cast<FlatBox *>(units), nullptr);
+    const FlatTable d = FlatTable::of(tab, 1, reinterpret_cast<FlatBox *>(units), nullptr, nullptr);
     e = cudaMemcpyAsync(tab, image, kImage, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail_static("slot upload: %s", e);
     if ((rc = launch_flat(plan.labeled != 0, g, d, fs.cfg, fs.blocks, fs.warps_per_block, st))) return rc;
