@@ -170,7 +170,8 @@ int flat_shape(int device, int levels, int tmax, bool skewed, bool big, bool sha
   s.cfg.entries = std::min(s.cfg.entries, flat_max_entries(s.warps_per_block));
   s.cfg.warp_bytes = (int)flat_warp_bytes(s.cfg.entries);
   s.cfg.idle_ms = o.wait_limit_ms > 0 ? o.wait_limit_ms : 30000;
-  s.cfg.split_ns = o.split_after_us > 0 ? o.split_after_us * 1000 : (o.split_after_us < 0 ? 0 : 60000);
+  s.cfg.split_ns = o.split_after_us > 0 ? o.split_after_us * 1000 : (o.split_after_us < 0 ? 0 : kSplitNs);
+  s.cfg.check = kCheckCycles;
   s.cfg.segments = o.label_rows < 0 ? 0 : 1;
   const size_t smem = (size_t)s.cfg.warp_bytes * s.warps_per_block;
   std::lock_guard<std::mutex> lk(mu);
@@ -427,7 +428,7 @@ void fill_slots(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_
 
 // The host image of the flat kernel's records.
 void fill_flat(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_options &o, int64_t eb, int64_t ee,
-               int stride, const Launch &L) {
+               int stride, Launch &L) {
   const FlatTable t = FlatTable::of(g->htab, n, nullptr, nullptr, nullptr);
   std::memset(static_cast<void *>(g->htab), 0, FlatTable::bytes(n) - (size_t)n * sizeof(FlatPlan));
   t.ctl->ticket = (unsigned long long)L.warps();  // the first ones are dealt one per warp
@@ -442,11 +443,16 @@ void fill_flat(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_o
     t.info[i].perm = in.perm;
     edges += in.e_end - in.e_begin;
   }
+  const bool hubs = g->max_degree > kHubDegree;
+  if (hubs && edges < (int64_t)kFewEdges * L.warps()) {
+    if (o.split_after_us == 0) L.fl.cfg.split_ns = kFewSplitNs;
+    L.fl.cfg.check = kFewCheckCycles;
+  }
   for (int i = 0; i < n; ++i) {
     FlatInfo &in = t.info[i];
     in.stride = stride;
     in.phase = o.edge_phase;
-    in.chunk = flat_chunk(edges, plans[i]->flat.s, g->max_degree > kHubDegree, stride, L.warps(), o.edge_chunk);
+    in.chunk = flat_chunk(edges, plans[i]->flat.s, hubs, stride, L.warps(), o.edge_chunk);
     in.ticket0 = t.ctl->tickets;
     t.ctl->tickets += ticket_count(in.e_begin, in.e_end, stride, o.edge_phase, in.chunk);
     t.plan[i] = plans[i]->flat;

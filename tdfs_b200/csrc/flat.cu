@@ -15,8 +15,13 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kTupleMax = kMaxK - 1;   // phi(0..5): the deepest enumerated level is 5
 constexpr int kProbeMax = kMaxK - 2;   // lists tested per candidate besides its source
+// A tail's block of entries ends before their lists pass this many positions:
+// unlike the other scans it is not resumed in the middle, and work is only
+// given away between blocks (32 entries with hub lists kept one warp busy for
+// 0.4 ms; a labeled power-law batch with such a tail 1.93 -> 1.07 ms; 1024 and
+// 16384 positions did the same).
+constexpr int kTailSpan = 4096;
 constexpr int kLookSteps = 32;         // 64-position steps of a scan between two looks at the idle mask
-constexpr int kCheckCycles = 16384;    // clocks between offers of work
 
 constexpr int kCntBytes = 7 * 32 * 4;
 constexpr int kRangeMin = 4;           // children of one parent given away as a range
@@ -340,7 +345,7 @@ struct Flat {
   // plans and do better without the mode's tests in the step (5-clique share
   // 21.4 against 25.1 ms).
   template <int FIXED>
-  __device__ __forceinline__ bool scan(const FlatStep &st, int L, int how, uint32_t *sizes) {
+  __device__ __forceinline__ bool scan(const FlatStep &st, int L, int how, uint32_t *sizes, int &width) {
     const int mode = FIXED >= 0 ? FIXED : how;
     FlatLevel &H = W.lev[L];
     const int first = H.next;
@@ -355,7 +360,12 @@ struct Flat {
       if (lane >= s) incl += t;
     }
     const uint32_t off = len > 0 ? incl - (uint32_t)len : ~0u;  // lanes without a list start nowhere
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    if (mode == 2) {
+      // a tail's block ends before its lists grow past kTailSpan positions
+      const unsigned fit = __ballot_sync(kFull, lane < width && incl <= (uint32_t)kTailSpan);
+      width = max(__popc(fit), 1);
+    }
+    const uint32_t total = __shfl_sync(kFull, incl, mode == 2 ? width - 1 : 31);
     const unsigned act = __ballot_sync(kFull, len > 0);
     if (len > 0) {
       const int rank = __popc(act & lanemask_lt());
@@ -561,15 +571,16 @@ struct Flat {
     FlatLevel &H = W.lev[L];
     const FlatPlan &F = W.plan;
     const bool leaf = L == F.s, tail = leaf && F.t > 1;
+    int width = 32;  // entries of this block
     if (!leaf && !filling) fill_begin(L);
     if (!LAB && !leaf) {
       while (H.next < H.end && W.lev[L + 1].n <= room(L + 1))
-        if (!scan<0>(F.step[L - 1], L, 0, nullptr)) return true;
+        if (!scan<0>(F.step[L - 1], L, 0, nullptr, width)) return true;
       fill_end(L);
       return false;
     }
     if (!LAB && F.t == 1 && !closed(F.term[0])) {
-      scan<1>(F.term[0], L, 1, nullptr);
+      scan<1>(F.term[0], L, 1, nullptr, width);
       return false;
     }
     const int p = H.next + lane;
@@ -589,8 +600,8 @@ struct Flat {
       } else {
         if (tail) cnt(u)[lane] = 0;
         __syncwarp();
-        if (LAB) scan<-1>(st, L, tail ? 2 : leaf ? 1 : 0, tail ? cnt(u) : nullptr);
-        else scan<2>(st, L, 2, cnt(u));
+        if (LAB) scan<-1>(st, L, tail ? 2 : leaf ? 1 : 0, tail ? cnt(u) : nullptr, width);
+        else scan<2>(st, L, 2, cnt(u), width);
         scanned = true;
       }
       __syncwarp();
@@ -600,11 +611,11 @@ struct Flat {
       fill_end(L);
       return false;
     }
-    if (tail && mine) count += tuples();
+    if (tail && mine && lane < width) count += tuples();
     __syncwarp();
     if (tail || !scanned) {  // the whole block is done (a scan of mode 1 keeps its own place)
       if (lane == 0) {
-        H.next = min(H.next + 32, H.end);
+        H.next = min(H.next + width, H.end);
         H.started = H.next;
       }
       __syncwarp();
@@ -945,7 +956,7 @@ struct Flat {
       if (inner && !more && W.lev[level + 1].n > 0) ++level;
       const long long c = clock64();
       int due = 0;
-      if (c - checked > kCheckCycles) {
+      if (c - checked > cfg.check) {
         checked = c;
         due = may_give();
       }

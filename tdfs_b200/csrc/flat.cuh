@@ -21,6 +21,7 @@ struct FlatCfg {
   int32_t warp_bytes;  // shared memory per warp
   int32_t idle_ms;     // bounded idle wait before a warp reports a timeout
   int32_t split_ns;    // work may be given away after this long on one base subtree
+  int32_t check;       // clocks between offers of work
   int32_t segments;    // 1: labeled plans read the label segments of rows (DevGraph::colidx_l)
   int32_t wide;        // 1: the 80-register build (3 CTAs of 256 threads per SM)
   int32_t share;       // 1: idle warps wait to be given work; 0: they leave
@@ -131,6 +132,16 @@ inline int flat_max_blocks(int warps_per_block) { return kFlatBoxes / warps_per_
 // in a launch of `edges` level-0 edges over all slots; skewed: on a graph with
 // hubs (kHubDegree); `edge_chunk` and `stride` as in tdfs_options.
 constexpr int32_t kHubDegree = 512;
+
+// How old a warp's base work must be before it gives some away, and the clocks
+// between its looks for idle warps.  Giving work away early costs more than it
+// gains where every warp has much of it, or the work is even (64-query ER burst
+// 0.154 ms at 60 us and 16384 clocks, 0.166 at 20 us and 4096; 7 power-law
+// queries 2.83 against 2.91).  A launch of fewer than kFewEdges level-0 edges
+// per warp on a graph with hubs is over when its few heavy edges are: they are
+// to be spread soon (4 labeled power-law queries 0.464 -> 0.373 ms).
+constexpr int kSplitNs = 60000, kCheckCycles = 16384;
+constexpr int kFewEdges = 16, kFewSplitNs = 20000, kFewCheckCycles = 4096;
 int flat_chunk(int64_t edges, int s, bool skewed, int stride, int warps, int edge_chunk);
 
 // Launch over the slots of `t` (on the device).

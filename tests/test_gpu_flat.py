@@ -175,3 +175,24 @@ def test_long_rows_are_split_over_a_block(T, po, nlabels):
                                                                 for i in range(5)]:
         P = T.PatternPreprocessor(text=text, labeled=labeled)
         assert T.count(dev, P).count == po.count(ora, po.Plan(text, labeled)), (text, labeled)
+
+
+@pytest.mark.parametrize("d", [127, 128, 129, 4095, 4097])
+def test_tail_blocks_end_at_a_span_of_lists(T, d):
+    """A block of a tail ends before its lists pass 4096 positions: 32 lists of
+    128 fill it, the 32nd of 129 starts the next, one of 4097 is a block."""
+    b = 12  # a clique of b vertices, each adjacent to all others: rows of d entries
+    n = d + 1
+    e = {(i, j) for i in range(b) for j in range(n) if i != j}
+    rowptr, colidx = csr(e | {(j, i) for i, j in e}, n)
+    labels = (np.arange(n) % 2).astype(np.int32)
+    dev = T.GraphPreprocessor(rowptr=rowptr, colidx=colidx, labels=labels, labeled=True)
+    edges = ("01 02 12 13 23 14 24", "01 02 03 04 12 13 14 23")
+    for es in edges:
+        for lab in ("11111", "01010", "11001"):
+            text = "".join(f"v {i} {l}\n" for i, l in enumerate(lab)) + "".join(
+                f"e {x[0]} {x[1]} 1\n" for x in es.split())
+            P = T.PatternPreprocessor(text=text, labeled=lab != "11111")
+            want = T.count(dev, P, T.default_options(steal=0)).count
+            assert T.count(dev, P).count == want
+            assert T.count(dev, P, T.default_options(split_after_us=-1)).count == want
