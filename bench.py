@@ -300,10 +300,10 @@ def reduce_over_ranks(dist, seconds_or_ms, counts, device="cuda"):
 
 
 def kernel_source_digest():
-    """SHA-256 (first 16 hex digits) of the match kernel's sources: an ncu
+    """SHA-256 (first 16 hex digits) of the counting kernels' sources: an ncu
     record of its traffic holds for the kernel it was captured on."""
     h = hashlib.sha256()
-    for f in ("match.cu", "match.cuh", "graph.h", "common.h"):
+    for f in ("flat.cu", "flat.cuh", "flat_plan.cpp", "match.cu", "match.cuh", "graph.h", "common.h"):
         with open(os.path.join(ROOT, "tdfs_b200", "csrc", f), "rb") as fh:
             h.update(fh.read())
     return h.hexdigest()[:16]
@@ -510,8 +510,9 @@ def run_tdfs(args, rank, world, dist):
                 "d2h_bytes_per_step": d2h,
                 "step": "tdfs_graph_from_csr from pinned host CSR (upload + derived arrays), pattern compiles, "
                         "tdfs_count_batch, count read-back, tdfs_graph_free"},
-        # per step and mode: the control reset and the match kernel
-        "gpu_launches": 2 * modes * args.steps,
+        # per step and mode one counting kernel (the flat one, or the DFS one, whose
+        # control reset is not counted)
+        "gpu_launches": modes * args.steps,
         "launch": launch,
         "parallelism": f"level-0 edge chunks dealt round-robin over {world} rank(s)",
         "clocks": clk,

@@ -228,7 +228,8 @@ int tdfs_server_destroy(tdfs_server *s); /* drains admitted queries, stops the k
 /* ---- counting without device allocation (no counterpart in the reference) --
  * For callers that cannot call cudaMalloc: a plugin whose host process hands
  * all device memory to its own allocator, or code that runs where allocating
- * is not allowed.  Same kernel and counts as tdfs_count; the graph is passed
+ * is not allowed.  Same kernels and counts as tdfs_count (the flat kernel while
+ * its row tables fit the array below, about 14*E + 37*n bytes); the graph is passed
  * as device pointers (not checked: the rules of tdfs_graph_from_csr; labels
  * int32, needed for a labeled pattern) and every working buffer lives in one fixed 48 MiB array inside the
  * library's device image, held on each GPU that uses the library until the

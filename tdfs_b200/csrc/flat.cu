@@ -47,9 +47,9 @@ struct FlatLevel {
 
 // Shared by a CTA's warps.
 struct FlatCta {
-  int32_t poll;    // 1: some idle warp of the CTA is watching SlotCtl::pending
+  int32_t poll;    // 1: some idle warp of the CTA is watching FlatCtl::pending
   int32_t done;    // 1: no work is left anywhere
-  int32_t active;  // busy warps; the CTA counts in SlotCtl::pending while there are any
+  int32_t active;  // busy warps; the CTA counts in FlatCtl::pending while there are any
   int32_t left;    // warps still in the kernel
   int32_t slot;    // slot whose counts are summed here first, -1 none
   unsigned long long sum, idle_ns, warp_ns;

@@ -6,7 +6,7 @@
 // so a step tests 32 candidates whatever the list lengths are (one DFS node at
 // a time leaves half of the lanes idle on lists of 16, and pays its set-up
 // per node).  Membership in the other backward neighbours' lists is one
-// 16-byte load of the row's hash table.
+// 32-byte load of a bucket of the row's hash table.
 #pragma once
 
 #include <cstdint>

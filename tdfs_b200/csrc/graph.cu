@@ -11,6 +11,8 @@
 //                             degree >= deg(pattern vertex 2)"
 //                             (src/gpu_match.cu:541-548) is one load
 //   label   uint8[n]          labeled graphs only (labels must be < 255)
+//   hash    int32[8 per bucket]  row membership tables (flat.cu), beside the
+//                             label index and label rows of labeled graphs
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -723,10 +725,10 @@ void build_label_arrays(int64_t n, int64_t nedges, const int64_t *rowptr, const 
 //   rowptr int64[n+1] | colidx int32[E + kColPad] | src int32[E] | maxnd int32[n]
 //   | label uint8[n] | lperm int32[E] | colidx_l int32[E + kColPad] | loff int32[n (nlab+1)]
 //   | scratch of the label index sort | row membership tables | self-loop flag and check result
-// The parts from `label` on are derived on the host into one pinned staging
-// block laid out the same way and uploaded with one copy.  The CSR copies and
-// the two preprocessing kernels are queued first, so the device works while
-// the host sorts; one synchronisation at the end.
+// The device derives everything but the narrowed labels; with more labels than
+// kSegLabels the host sorts the label index into a pinned staging block, laid
+// out the same way, while the copies and kernels queued before it run.  One
+// synchronisation at the end.
 int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx, const int32_t *labels,
                  int device, int32_t max_degree, bool check, tdfs_graph **out) {
   int ndev = 0;

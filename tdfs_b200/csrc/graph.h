@@ -99,8 +99,8 @@ namespace tdfs {
 
 // Launch workspace: what one persistent launch needs besides the graph --
 // the control block, the split ring, the slot table and its pinned host
-// staging copy.  About 12 MB of device memory and 1.7 MB of pinned host
-// memory, so it is pooled per device (graph.cu) instead of being allocated
+// staging copy.  Tens of MB of device memory (and 100 MB for `big`, on graphs
+// with hubs) and about 10 MB of pinned host memory, so it is pooled per device (graph.cu) instead of being allocated
 // with every graph: a graph takes one at its first launch and hands it back
 // when it is freed.
 struct Workspace {
