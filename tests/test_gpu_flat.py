@@ -181,7 +181,7 @@ def test_long_rows_are_split_over_a_block(T, po, nlabels):
 def test_tail_blocks_end_at_a_span_of_lists(T, d):
     """A block of a tail ends before its lists pass 4096 positions: 32 lists of
     128 fill it, the 32nd of 129 starts the next, one of 4097 is a block."""
-    b = 12  # a clique of b vertices, each adjacent to all others: rows of d entries
+    b = 8  # a clique of b vertices, each adjacent to all others: rows of d entries
     n = d + 1
     e = {(i, j) for i in range(b) for j in range(n) if i != j}
     rowptr, colidx = csr(e | {(j, i) for i, j in e}, n)
@@ -193,6 +193,6 @@ def test_tail_blocks_end_at_a_span_of_lists(T, d):
             text = "".join(f"v {i} {l}\n" for i, l in enumerate(lab)) + "".join(
                 f"e {x[0]} {x[1]} 1\n" for x in es.split())
             P = T.PatternPreprocessor(text=text, labeled=lab != "11111")
-            want = T.count(dev, P, T.default_options(steal=0)).count
+            want = T.count(dev, P, T.default_options(tail_count=1)).count  # a DFS kernel knob: that kernel
             assert T.count(dev, P).count == want
             assert T.count(dev, P, T.default_options(split_after_us=-1)).count == want
