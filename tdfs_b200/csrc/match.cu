@@ -378,7 +378,7 @@ struct Engine {
     LevelHdr &H = W.h[i];
     setup_into(H, i, false, a);
     if (H.send - H.spos > cfg.cap - 32) return false;
-    produce(i);
+    produce(i, false);
     if (lane == 0) {
       H.core = 1;
       H.complete = 0;  // not the candidate set of the current prefix: no reuse from it
@@ -530,7 +530,11 @@ struct Engine {
   }
 
   // Fill the level-i buffer with the next chunk of candidates and publish it.
-  __device__ void produce(int i) {
+  // offer = false: nothing is published yet.  A core set's items become
+  // claimable by publish_core only: had they been published here as well, a
+  // thief could take some between the two, and the second publication, which
+  // replaces the word, would hand them out again.
+  __device__ void produce(int i, bool offer = true) {
     LevelHdr &H = W.h[i];
     int32_t *out = buf(i);
     const int32_t *src = H.src;
@@ -569,9 +573,7 @@ struct Engine {
       } else {
         H.complete = 0;
       }
-      const unsigned long long gen = (W.word[i] >> 32) + 1;
-      __threadfence_block();
-      atomicExch(&W.word[i], (gen << 32) | (unsigned long long)n);
+      if (offer) publish(i, n);
     }
     __syncwarp();
   }
