@@ -431,9 +431,7 @@ void fill_flat(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_o
                int stride, Launch &L) {
   const FlatTable t = FlatTable::of(g->htab, n, nullptr, nullptr, nullptr);
   std::memset(static_cast<void *>(g->htab), 0, FlatTable::bytes(n) - (size_t)n * sizeof(FlatPlan));
-  t.ctl->ticket = (unsigned long long)L.warps();  // the first ones are dealt one per warp
-  t.ctl->pending = L.fl.blocks;
-  t.ctl->slots = n;
+  t.start(L.fl.blocks, L.fl.warps_per_block, L.fl.cfg.share != 0, n);
   int64_t edges = 0;
   for (int i = 0; i < n; ++i) {
     SlotInfo in;

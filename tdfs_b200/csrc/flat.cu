@@ -49,8 +49,10 @@ struct FlatLevel {
 struct FlatCta {
   int32_t poll;    // 1: some idle warp of the CTA is watching FlatCtl::pending
   int32_t done;    // 1: no work is left anywhere
-  int32_t active;  // busy warps; the CTA counts in FlatCtl::pending while there are any
+  int32_t all;     // 1: the whole grid has started
+  int32_t active;  // busy warps
   int32_t left;    // warps still in the kernel
+  long long first; // the CTA's first tickets: [first, first + warps)
   int32_t slot;    // slot whose counts are summed here first, -1 none
   unsigned long long sum, idle_ns, warp_ns;
 };
@@ -732,7 +734,7 @@ struct Flat {
   __device__ bool next_ticket(int &hint) {
     for (;;) {
       long long t = 0;
-      if (lane == 0) t = (long long)atomicAdd(&T.ctl->ticket, 1ull);
+      if (lane == 0) t = (long long)(atomicAdd(&T.ctl->ticket, 1ull) & (kCtaJoin - 1));
       t = __shfl_sync(kFull, t, 0);
       if (t >= T.ctl->tickets) return false;
       if (start_ticket(t, hint)) return true;
@@ -862,6 +864,27 @@ struct Flat {
     return l;
   }
 
+  // p: FlatCtl::pending as just read.  Is no CTA busy and no mailbox full?  The
+  // count of started CTAs is read after p, and it only grows: a sum of 0 means
+  // that when p was read every CTA started until then was idle.  A warp asks
+  // once it has seen the last ticket go, and the atomic that takes a CTA's
+  // tickets also counts it, so whoever took one is among them.  Once the whole
+  // grid has started, p alone tells.
+  __device__ __forceinline__ bool complete(int p) const {
+    const int grid = (int)gridDim.x;
+    if (p == -grid) return true;
+    if (*(volatile int32_t *)&C.all) return false;
+    __threadfence();
+    const int started = (int)(*(volatile unsigned long long *)&T.ctl->ticket >> kJoinShift);
+    if (started == grid) *(volatile int32_t *)&C.all = 1;
+    return p + started == 0;
+  }
+  // A warp has run dry (lane 0).  True when it was its CTA's last busy one and
+  // nothing is left anywhere.
+  __device__ __forceinline__ bool cta_idle() const {
+    return atomicSub(&C.active, 1) == 1 && complete(atomicSub(&T.ctl->pending, 1) - 1);
+  }
+
   // Wait until this warp is given work (returns its level, installed) or none
   // will come (0).  A waiting warp reads its own mailbox; one per CTA also
   // reads the count of what is pending.  Bounded: after cfg.idle_ms the
@@ -872,15 +895,15 @@ struct Flat {
     flush();
     if (!cfg.share) {
       // light, even work: nothing to wait for
-      if (lane == 0 && atomicSub(&C.active, 1) == 1 && atomicSub(&T.ctl->pending, 1) == 1) T.run->finished = 1;
+      if (lane == 0 && cta_idle()) T.run->finished = 1;
       __syncwarp();
       return 0;
     }
     if (lane == 0) {
       *(volatile int32_t *)&T.box[gid].full = 0;
-      __threadfence();
+      __threadfence();  // (the CTA's start comes before its idleness, too)
       atomicOr(&T.idle[gid >> 5], 1u << (gid & 31));
-      if (atomicSub(&C.active, 1) == 1 && atomicSub(&T.ctl->pending, 1) == 1) {
+      if (cta_idle()) {
         T.run->finished = 1;
         *(volatile int32_t *)&C.done = 1;
       }
@@ -892,7 +915,7 @@ struct Flat {
         if (*(volatile int32_t *)&T.box[gid].full) st = 1;
         else if (*(volatile int32_t *)&C.done) st = 2;
         else if (poller || (poller = atomicCAS(&C.poll, 0, 1) == 0)) {
-          if (*(volatile int32_t *)&T.ctl->pending <= 0) {
+          if (complete(*(volatile int32_t *)&T.ctl->pending)) {
             *(volatile int32_t *)&C.done = 1;
             st = 2;
           }
@@ -929,10 +952,10 @@ struct Flat {
     __syncwarp();
     int level = 0, base = 1, hint = 0;
     bool more = false;
-    bool dry = T.ctl->tickets <= (int)gridDim.x * (int)(blockDim.x >> 5);  // none besides the dealt ones
+    const long long mine = C.first + (threadIdx.x >> 5);
+    bool dry = C.first + (blockDim.x >> 5) >= T.ctl->tickets;  // none besides the CTA's first ones
     long long checked = clock64();
-    // the host dealt the first tickets, one per warp
-    if (gid < T.ctl->tickets && start_ticket(gid, hint)) level = 1;
+    if (mine < T.ctl->tickets && start_ticket(mine, hint)) level = 1;
     for (;;) {
       if (level < base) {
         level = 0;
@@ -1001,7 +1024,11 @@ __global__ void __launch_bounds__(256, MINB) flat_kernel(const __grid_constant__
   __shared__ FlatCta cta;
   if (threadIdx.x == 0) {
     cta.poll = cta.done = 0;
+    cta.all = !cfg.share;
     cta.active = cta.left = (int)(blockDim.x >> 5);
+    const unsigned warps = blockDim.x >> 5;
+    cta.first = cfg.share ? (long long)(atomicAdd(&T.ctl->ticket, kCtaJoin + warps) & (kCtaJoin - 1))
+                          : (long long)blockIdx.x * warps;
     cta.slot = 0;
     cta.sum = cta.idle_ns = cta.warp_ns = 0;
   }

@@ -51,10 +51,23 @@ int flat_blocks_per_sm(bool labeled, bool wide, bool big, int warps_per_block, s
 constexpr int kFlatBoxes = 8192;  // mailboxes, one per warp of the grid
 constexpr int kIdleWords = kFlatBoxes / 32;
 
+// A launch does not need its whole grid on the GPU at once: another kernel may
+// hold part of the SMs for as long as it likes.  Where warps wait for work, it
+// belongs to nobody before a running CTA takes it, and a CTA counts as busy
+// from when it starts, so the CTAs that run finish the launch and one that
+// starts later finds nothing.  One atomic does both: a CTA adds kCtaJoin + its
+// warps to `ticket`, which takes a ticket per warp and counts the CTA.  Where
+// warps leave when they run dry (FlatCfg::share 0), every CTA gets its turn:
+// there the host deals the first tickets and counts all CTAs (the atomics of
+// 592 CTAs on one word take 3.5 us, a tenth of a triangle count on the n=4096
+// ER graph).
+constexpr int kJoinShift = 50;  // tickets below, CTAs that have started above
+constexpr unsigned long long kCtaJoin = 1ull << kJoinShift;
 struct alignas(128) FlatCtl {
-  unsigned long long ticket;  // the next ticket; the host deals the first ones, one per warp
+  unsigned long long ticket;  // the next ticket; above kJoinShift, the CTAs that have started
   char pad0_[120];
-  int32_t pending;            // CTAs with busy warps + filled mailboxes; 0 = the launch is complete
+  int32_t pending;            // filled mailboxes - CTAs without a busy warp; the launch is complete when
+                              // no tickets are left and this plus the started CTAs is 0
   char pad1_[124];
   int32_t gone;               // CTAs that have left
   char pad3_[124];
@@ -123,10 +136,17 @@ struct FlatTable {
     t.host = host;
     return t;
   }
+  // The control block of a launch with this many CTAs, in a zeroed host image.
+  void start(int blocks, int warps_per_block, bool share, int n) const {
+    ctl->slots = n;
+    if (share) return;  // CTAs take their first tickets and count themselves
+    ctl->ticket = (unsigned long long)blocks * warps_per_block + kCtaJoin * blocks;
+  }
 };
 
 // The most CTAs of a launch (every warp has a mailbox).
 inline int flat_max_blocks(int warps_per_block) { return kFlatBoxes / warps_per_block; }
+static_assert((unsigned long long)kFlatBoxes < 1ull << (64 - kJoinShift), "a join count for every CTA");
 
 // Level-0 edges per ticket of a slot whose plan is enumerated down to level s,
 // in a launch of `edges` level-0 edges over all slots; skewed: on a graph with

@@ -193,9 +193,7 @@ extern "C" int tdfs_count_static(int device, int64_t n, int64_t nedges, const in
     constexpr size_t kImage = FlatTable::bytes(1);
     alignas(128) unsigned char image[kImage] = {};
     const FlatTable h = FlatTable::of(image, 1, nullptr, nullptr, nullptr);
-    h.ctl->ticket = (unsigned long long)fs.blocks * fs.warps_per_block;
-    h.ctl->pending = fs.blocks;
-    h.ctl->slots = 1;
+    h.start(fs.blocks, fs.warps_per_block, fs.cfg.share != 0, 1);
     FlatInfo &in = h.info[0];
     in.e_begin = eb;
     in.e_end = ee;
