@@ -1914,25 +1914,32 @@ void init_launch(RunCtl *ctl, QueueHdr *qh, cudaStream_t stream) {
 }
 
 int launch_match(bool labeled, const DevGraph &g, RunCtl *ctl, SlotTable *tab, SplitUnit *units, QueueHdr *qh,
-                 const KernelCfg &cfg, int blocks, int warps_per_block, cudaStream_t stream) {
+                 const KernelCfg &cfg, int blocks, int warps_per_block, cudaStream_t stream, bool leave_room) {
   const size_t smem = (size_t)cfg.warp_bytes * warps_per_block;
-  const dim3 grid(blocks), block(warps_per_block * 32);
+  cudaLaunchAttribute room;
+  room.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  room.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+  cudaLaunchConfig_t at{};
+  at.gridDim = dim3(blocks);
+  at.blockDim = dim3(warps_per_block * 32);
+  at.dynamicSmemBytes = smem;
+  at.stream = stream;
+  at.attrs = &room;
+  at.numAttrs = leave_room ? 1 : 0;
   cudaError_t a;
   if (labeled)
     a = cfg.wide_regs ? ensure_dynamic_smem<true, 3>(smem) : ensure_dynamic_smem<true, 4>(smem);
   else
     a = cfg.wide_regs ? ensure_dynamic_smem<false, 3>(smem) : ensure_dynamic_smem<false, 4>(smem);
   if (a != cudaSuccess) return fail(TDFS_ERR_CUDA, "match kernel shared memory: %s", cudaGetErrorString(a));
-  (void)cudaGetLastError();  // the check below must see this launch's error only
-  if (labeled) {
-    if (cfg.wide_regs) match_kernel<true, 3><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, units, qh);
-    else match_kernel<true, 4><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, units, qh);
-  } else {
-    if (cfg.wide_regs) match_kernel<false, 3><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, units, qh);
-    else match_kernel<false, 4><<<grid, block, smem, stream>>>(g, cfg, ctl, tab, units, qh);
+  (void)cudaGetLastError();  // a failure below must not find an older one
+  const auto kernel = labeled ? (cfg.wide_regs ? match_kernel<true, 3> : match_kernel<true, 4>)
+                              : (cfg.wide_regs ? match_kernel<false, 3> : match_kernel<false, 4>);
+  const cudaError_t e = cudaLaunchKernelEx(&at, kernel, g, cfg, ctl, tab, units, qh);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return fail(TDFS_ERR_CUDA, "match kernel launch: %s", cudaGetErrorString(e));
   }
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(TDFS_ERR_CUDA, "match kernel launch: %s", cudaGetErrorString(e));
   return TDFS_OK;
 }
 

@@ -98,7 +98,11 @@ int resident_blocks_per_sm(bool labeled, int warps_per_block, size_t smem, bool 
 void init_launch(RunCtl *ctl, QueueHdr *qh, cudaStream_t stream);
 
 // Launch the match kernel over the slot table `tab` (filled by the host).
+// leave_room: the launch's CTAs stay for long and are to share the SMs.  An SM
+// keeps the split between L1 and shared memory that the kernel on it started
+// with; chosen for the match kernel alone it kept every CTA of a count beside
+// it (57 KB) waiting until the kernel left.
 int launch_match(bool labeled, const DevGraph &g, RunCtl *ctl, SlotTable *tab, SplitUnit *units, QueueHdr *qh,
-                 const KernelCfg &cfg, int blocks, int warps_per_block, cudaStream_t stream);
+                 const KernelCfg &cfg, int blocks, int warps_per_block, cudaStream_t stream, bool leave_room = false);
 
 }  // namespace tdfs

@@ -130,7 +130,7 @@ int open_epoch(Server &S) {
 int launch_kernel(Server &S) {
   init_launch(S.g->ctl, queue_hdr(S.g), S.kstream);
   int rc = launch_match(S.labeled, graph_view(S.g), S.g->ctl, S.g->tab, S.g->queue, queue_hdr(S.g), S.shape.cfg,
-                        S.shape.blocks, S.shape.warps_per_block, S.kstream);
+                        S.shape.blocks, S.shape.warps_per_block, S.kstream, S.opt.launch.blocks_per_sm > 0);
   if (!rc) S.kernel_live = true;
   return rc;
 }

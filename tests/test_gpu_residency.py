@@ -3,7 +3,9 @@
 A server's idle kernel holds one CTA on every SM for a few seconds (it leaves
 by itself after idle_exit_ms); the counts beside it find room for part of
 their CTAs only.  Those finish the count: no count runs out of its own, much
-shorter, wait limit."""
+shorter, wait limit, and none waits for the server's kernel to leave."""
+import time
+
 import numpy as np
 import pytest
 
@@ -52,3 +54,16 @@ def test_counts_beside_a_resident_kernel(T, beside, shape):
             assert static(i, wait_limit_ms=500) == n
     assert run(0, 1, graph_capture=1, wait_limit_ms=500) == want[0, 1]
     srv.close()
+
+
+@pytest.mark.parametrize("shape", [{}, {"chunk_cap": 128}, {"warps_per_block": 1, "chunk_cap": 64}, {"blocks_per_sm": 2}])
+def test_a_limited_server_leaves_room_on_the_sm(T, beside, shape):
+    graph, triangle, run, static, want = beside
+    shape = {"blocks_per_sm": 1, **shape}
+    for i in range(4):
+        srv = T.Server(graph, max_inflight=4, idle_exit_ms=HOLD_MS, **shape)
+        assert srv.wait(srv.submit(triangle))[0] == want[0, 0]
+        t0 = time.monotonic()
+        assert run(0, i) == want[0, i] and static(1) == want[0, 1]
+        assert time.monotonic() - t0 < HOLD_MS / 2000, (shape, i)
+        srv.close()
