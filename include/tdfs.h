@@ -171,11 +171,13 @@ typedef struct {
 int tdfs_last_launch(const tdfs_graph *g, tdfs_launch_stats *st);
 
 /* ---- bounded device waits, shown to run out (no reference counterpart) ----
- * Launches the match kernel over a slot that can never complete (admitted,
- * no level-0 tickets, no work held), so every warp waits for work until its
- * wait_limit_ms bound runs out, then the kernel returns.  Returns the status
- * the launch reports -- TDFS_ERR_TIMEOUT when the bound works -- and the
- * kernel's duration in *kernel_ms.  The context stays usable afterwards. */
+ * Launches the DFS kernel over a slot that can never complete (admitted,
+ * no level-0 tickets, no work held), and, where the graph can run it, the flat
+ * kernel over work that nobody has, plainly and through a captured graph: every
+ * warp waits for work until its wait_limit_ms bound runs out, then the kernel
+ * returns.  Returns the status the launches report -- TDFS_ERR_TIMEOUT when
+ * the bound of each works -- and the longest kernel's duration in *kernel_ms.
+ * The context stays usable afterwards. */
 int tdfs_selftest_wait_limit(tdfs_graph *g, int wait_limit_ms, float *kernel_ms);
 
 /* ---- autotuner (no reference counterpart; the reference's shape is fixed at

@@ -396,9 +396,9 @@ def count_batch_status(graph: GraphPreprocessor, patterns, options: Options | No
 
 
 def selftest_wait_limit(graph: GraphPreprocessor, wait_limit_ms: int):
-    """Run the match kernel over a slot that can never complete; returns
-    (status code the launch reported, kernel ms).  TDFS_ERR_TIMEOUT (6) means
-    every warp's bounded wait ran out as designed."""
+    """Run both counting kernels over work that can never complete; returns
+    (status code the launches reported, longest kernel ms).  TDFS_ERR_TIMEOUT (6)
+    means every warp's bounded wait ran out as designed."""
     ms = C.c_float()
     rc = lib().tdfs_selftest_wait_limit(graph._h, wait_limit_ms, C.byref(ms))
     return rc, ms.value
