@@ -71,35 +71,45 @@ int check_csr_frame(int64_t n, int64_t nedges, const int64_t *rowptr) {
   return TDFS_OK;
 }
 
-int csr_fault(int kind, int64_t row) {
-  if (kind == 1) return fail(TDFS_ERR_FORMAT, "rowptr decreases at vertex %lld", (long long)row);
-  if (kind == 2) return fail(TDFS_ERR_FORMAT, "neighbour id out of range in row %lld", (long long)row);
-  return fail(TDFS_ERR_FORMAT, "row %lld not strictly increasing (unsorted or duplicate edge)", (long long)row);
-}
-
 int validate_csr(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx,
                  int32_t *max_degree) {
   if (const int rc = check_csr_frame(n, nedges, rowptr)) return rc;
-  std::atomic<int> bad{0};
-  std::atomic<int64_t> where{-1};
+  // the first row that breaks the rules, as 4 * row + what is wrong with it (1 its
+  // ends, 2 a neighbour id, 3 the order): rows before it are looked at whatever
+  // the threads beyond it have found, so the answer does not depend on them
+  std::atomic<int64_t> first{INT64_MAX};
   std::vector<int32_t> part_max(hw_threads() + 1, 0);
   std::atomic<int> slot{0};
   parallel_for(
       n, [&](int64_t b, int64_t e) {
     int32_t md = 0;
-    for (int64_t v = b; v < e && !bad.load(std::memory_order_relaxed); ++v) {
-      int64_t lo = rowptr[v], hi = rowptr[v + 1];
-      if (hi < lo || hi - lo > INT32_MAX) { bad = 1; where = v; break; }
-      md = std::max<int32_t>(md, (int32_t)(hi - lo));
-      for (int64_t j = lo; j < hi; ++j) {
-        int32_t c = colidx[j];
-        if (c < 0 || c >= n) { bad = 2; where = v; break; }
-        if (j + 1 < hi && c >= colidx[j + 1]) { bad = 3; where = v; break; }
+    for (int64_t v = b; v < e && 4 * v < first.load(std::memory_order_relaxed); ++v) {
+      const int64_t lo = rowptr[v], hi = rowptr[v + 1];
+      int kind = 0;
+      if (lo < 0 || hi > nedges || hi < lo || hi - lo > INT32_MAX) {
+        kind = 1;
+      } else {
+        md = std::max<int32_t>(md, (int32_t)(hi - lo));
+        for (int64_t j = lo; j < hi && !kind; ++j) {
+          const int32_t c = colidx[j];
+          if (c < 0 || c >= n) kind = 2;
+          else if (j + 1 < hi && c >= colidx[j + 1]) kind = 3;
+        }
+      }
+      if (kind) {
+        int64_t old = first.load();
+        while (4 * v + kind < old && !first.compare_exchange_weak(old, 4 * v + kind)) {}
+        break;
       }
     }
     part_max[slot++] = md;
   }, n + nedges);
-  if (bad) return csr_fault(bad, where.load());
+  if (const int64_t f = first.load(); f != INT64_MAX) {
+    const long long row = f / 4;
+    if (f % 4 == 1) return fail(TDFS_ERR_FORMAT, "rowptr decreases at vertex %lld", row);
+    if (f % 4 == 2) return fail(TDFS_ERR_FORMAT, "neighbour id out of range in row %lld", row);
+    return fail(TDFS_ERR_FORMAT, "row %lld not strictly increasing (unsorted or duplicate edge)", row);
+  }
   if (max_degree) *max_degree = *std::max_element(part_max.begin(), part_max.end());
   return TDFS_OK;
 }

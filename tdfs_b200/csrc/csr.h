@@ -41,10 +41,9 @@ inline uint64_t hash64(uint64_t seed, uint64_t i) {
 }
 
 // Check a CSR for the reference's invariants; returns TDFS_OK or error code.
-// check_csr_frame looks at the sizes and rowptr's ends only; csr_fault reports
-// a row that breaks the rules (kind 1 rowptr, 2 neighbour id, 3 order).
+// Of several faults the one in the lowest row is reported.  check_csr_frame
+// looks at the sizes and rowptr's ends only.
 int check_csr_frame(int64_t n, int64_t nedges, const int64_t *rowptr);
-int csr_fault(int kind, int64_t row);
 int validate_csr(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t *colidx,
                  int32_t *max_degree);
 

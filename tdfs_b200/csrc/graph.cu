@@ -66,41 +66,38 @@ constexpr int kBuildWarps = 8;    // warps per CTA of the build kernels
 
 // ---- the CSR's rules ------------------------------------------------------------
 struct CsrCheck {
-  int32_t kind;  // 0, or what is wrong: 1 rowptr, 2 a neighbour id, 3 a row's order (as validate_csr, csr.cpp)
+  int32_t bad;
   int32_t max_degree;
-  int64_t row;
 };
 
-// The rules of validate_csr on the device copy.  Reads inside the arrays
-// whatever they hold: a row's range is only compared, and a descending pair of
-// neighbours is looked up among the row starts.  6M edges take 0.10 ms; the
-// host's pass took 2.8 ms with 16 threads (the first of them had the hubs).
+// The rules of validate_csr (csr.cpp) on the device copy: a verdict only.  What
+// is wrong, and where, the host's pass then says, so the message is the same
+// wherever a CSR is checked.  Reads inside the arrays whatever they hold: a
+// row's range is only compared, and a descending pair of neighbours is looked
+// up among the row starts.  6M edges take 0.10 ms; the host's pass takes 2.8 ms
+// with 16 threads (the first of them has the hubs).
 __global__ void check_csr_kernel(const int64_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, int64_t n,
                                  int64_t nedges, CsrCheck *out) {
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  auto bad = [&](int kind, int64_t row) {
-    if (atomicCAS(&out->kind, 0, kind) == 0) out->row = row;
-  };
   int32_t md = 0;
   for (int64_t v = first; v < n; v += step) {
     const int64_t lo = rowptr[v], hi = rowptr[v + 1];
-    if (lo < 0 || hi > nedges || hi < lo || hi - lo > INT32_MAX) bad(1, v);
+    if (lo < 0 || hi > nedges || hi < lo || hi - lo > INT32_MAX) out->bad = 1;
     else md = max(md, (int32_t)(hi - lo));
   }
   md = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)md);
   if ((threadIdx.x & 31) == 0 && md > 0) atomicMax(&out->max_degree, md);
   for (int64_t j = first; j < nedges; j += step) {
     const int32_t c = colidx[j];
-    const bool range = c < 0 || c >= n, falls = j + 1 < nedges && c >= colidx[j + 1];
-    if (!range && !falls) continue;
+    if (c < 0 || c >= n) out->bad = 1;
+    if (j + 1 >= nedges || c < colidx[j + 1]) continue;
     int64_t a = 0, z = n;  // the first row that starts after j
     while (a < z) {
       const int64_t m = (a + z) >> 1;
       if (rowptr[m] <= j) a = m + 1; else z = m;
     }
-    if (range) bad(2, a - 1);
-    else if (rowptr[a] != j + 1) bad(3, a - 1);
+    if (rowptr[a] != j + 1) out->bad = 1;
   }
 }
 
@@ -755,7 +752,8 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     if (least < 0 || most > 254)
       return checked(fail(TDFS_ERR_FORMAT, "vertex labels must lie in [0, 254] for the device label array"));
     nl = most + 1;
-    if (nedges > INT32_MAX) return fail(TDFS_ERR_CAPACITY, "labeled graphs hold at most 2^31 - 1 directed edges");
+    if (nedges > INT32_MAX)
+      return checked(fail(TDFS_ERR_CAPACITY, "labeled graphs hold at most 2^31 - 1 directed edges"));
   }
   // label-partitioned rows for graphs with at most kSegLabels labels
   const int nlab = labels && nl <= kSegLabels ? nl : 0;
@@ -798,7 +796,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
                              &stage_bytes);
     if (e != cudaSuccess) {
       device_blocks().give(device, arrays, array_bytes);
-      return cuda_fail(e, "pinned staging for the label arrays");
+      return checked(cuda_fail(e, "pinned staging for the label arrays"));
     }
   }
   char *base = static_cast<char *>(arrays);
@@ -831,7 +829,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     e = cudaMemcpyAsync(g->colidx, colidx, sizeof(int32_t) * nedges, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(g->colidx + nedges, 0x7f, sizeof(int32_t) * kColPad, st);
   auto *lab8 = static_cast<uint8_t *>(stage);
-  CsrCheck ck{0, max_degree, 0};
+  CsrCheck ck{0, max_degree};
   if (e == cudaSuccess && check) {
     // nothing below may read rows that break the rules: wait for the verdict
     // (and narrow the labels meanwhile)
@@ -847,11 +845,12 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
       for (int64_t i = 0; i < n; ++i) lab8[i] = (uint8_t)labels[i];
     if (e == cudaSuccess) e = cudaMemcpyAsync(&ck, dck, sizeof ck, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess && ck.kind) {
+    if (e == cudaSuccess && ck.bad) {
       pinned_blocks().give(device, stage, stage_bytes);
       device_blocks().give(device, arrays, array_bytes);
       delete g;
-      return csr_fault(ck.kind, ck.row);
+      if (const int bad = validate_csr(n, nedges, rowptr, colidx, nullptr)) return bad;
+      return fail(TDFS_ERR_FORMAT, "the rows changed while they were read");
     }
     g->max_degree = ck.max_degree;
   } else if (labels) {
