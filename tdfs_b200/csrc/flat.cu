@@ -560,7 +560,14 @@ struct Flat {
       return u == kNoTerm ? 0ull : (unsigned long long)cnt(u)[lane];
     };
     const unsigned long long a = at(1);
-    if (F.form == 1) return F.t == 2 ? a * (a - 1) / 2 : a * (a - 1) / 2 * (a - 2) / 3;
+    if (F.form == 1) {
+      // subsets of two or three; counts are modulo 2^64, so 3 is divided out of a
+      // factor that holds it and not out of the product, which passes 2^64 from
+      // 3.3M candidates on
+      const unsigned long long pairs = a * (a - 1) / 2;
+      if (F.t == 2) return pairs;
+      return (uint32_t)a % 3 == 2 ? pairs * ((a - 2) / 3) : pairs / 3 * (a - 2);
+    }
     const unsigned long long b = at(2);
     if (F.t == 2) return a * b - at(3);
     const unsigned long long c = at(4);
