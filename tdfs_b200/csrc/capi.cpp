@@ -404,6 +404,14 @@ int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms,
   return collect(g, n, L.flat, raw, status);
 }
 
+// What a launch on g needs first, its device current and a workspace.  It comes
+// before the choice of the kernel: where memory is short g loses its tables.
+int workspace_of(tdfs_graph *g) {
+  const cudaError_t e = cudaSetDevice(g->device);
+  if (e != cudaSuccess) return cuda_err(e, "cudaSetDevice");
+  return acquire_workspace(g);
+}
+
 // The host image of the slot table for the DFS kernel.
 void fill_slots(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_options &o, int64_t eb, int64_t ee,
                 int stride, int warps) {
@@ -491,15 +499,12 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
     kmax = std::max(kmax, (int)plans[i]->dev.k);
   }
   if (labeled && !g->labeled) return fail(TDFS_ERR_ARG, "labeled pattern on a graph opened without labels");
-  cudaError_t e = cudaSetDevice(g->device);
-  if (e != cudaSuccess) return cuda_err(e, "cudaSetDevice");
   Launch L;
   std::memset(static_cast<void *>(&L), 0, sizeof L);
   L.flat = flat;
   LaunchShape shape;
   int rc = launch_shape(g, kmax, labeled, o, &shape);  // checks the options for either kernel
   if (rc) return rc;
-  if ((rc = acquire_workspace(g))) return rc;
   if (flat) {
     // with hubs of more than kSkewDegree neighbours, candidate sets outgrow
     // shared memory and long scans dominate
@@ -649,7 +654,10 @@ int tdfs_graph_info(const tdfs_graph *g, int64_t *n, int64_t *nedges, int32_t *m
   if (nedges) *nedges = g->nedges;
   if (max_degree) *max_degree = g->max_degree;
   if (labeled) *labeled = g->labeled;
-  if (device_bytes) *device_bytes = g->bytes;
+  if (device_bytes) {
+    std::lock_guard<std::mutex> lk(*g->tables_mu);
+    *device_bytes = g->bytes;
+  }
   return TDFS_OK;
 }
 
@@ -709,6 +717,8 @@ int tdfs_count(tdfs_graph *g, const tdfs_plan *p, const tdfs_options *opt, uint6
   tdfs_options o;
   if (opt) o = *opt; else tdfs_options_default(&o);
   unsigned long long raw = 0;
+  std::lock_guard<std::mutex> lk(*g->tables_mu);
+  if (const int rc = workspace_of(g)) return rc;
   int rc = run_batch(g, &p, 1, g->hash && p->has_flat && flat_options(o), o, &raw, nullptr, kernel_ms);
   if (rc) return rc;
   // cu_test.cu:100-105: the unlabeled total is multiplied by |Aut|
@@ -729,6 +739,8 @@ int tdfs_count_batch_status(tdfs_graph *g, const tdfs_plan *const *plans, int np
   float total = 0.f;
   for (int i = 0; i < nplans; ++i)
     if (!plans[i]) return fail(TDFS_ERR_ARG, "null plan %d", i);
+  std::lock_guard<std::mutex> lk(*g->tables_mu);
+  if (const int rc = workspace_of(g)) return rc;
   const bool flat_here = g->hash && flat_options(o);
   // one launch per mode (labeled or unlabeled) and kernel
   for (int launch = 0; launch < 4; ++launch) {
@@ -847,9 +859,8 @@ int tdfs_autotune(tdfs_graph *g, const tdfs_plan *const *plans, int nplans, cons
 
 int tdfs_selftest_wait_limit(tdfs_graph *g, int wait_limit_ms, float *kernel_ms) {
   if (!g || wait_limit_ms <= 0 || wait_limit_ms > 60000) return fail(TDFS_ERR_ARG, "wait_limit_ms must lie in [1, 60000]");
-  cudaError_t e = cudaSetDevice(g->device);
-  if (e != cudaSuccess) return cuda_err(e, "cudaSetDevice");
-  if (const int rc = acquire_workspace(g)) return rc;
+  std::lock_guard<std::mutex> lk(*g->tables_mu);
+  if (const int rc = workspace_of(g)) return rc;
   tdfs_options o;
   tdfs_options_default(&o);
   o.wait_limit_ms = wait_limit_ms;

@@ -442,6 +442,8 @@ void free_workspace(Workspace *w) {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+bool reclaim_memory(int device, tdfs_graph *self);
+
 }  // namespace
 
 int acquire_workspace(tdfs_graph *g) {
@@ -467,6 +469,10 @@ int acquire_workspace(tdfs_graph *g) {
     w->device = g->device;
     char *d = nullptr, *h = nullptr;
     cudaError_t e = cudaMalloc(&d, dev_bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      if (reclaim_memory(g->device, g)) e = cudaMalloc(&d, dev_bytes);
+    }
     if (e == cudaSuccess) {
       e = cudaMallocHost(&h, o_hctl + sizeof(RunCtl));
       if (e != cudaSuccess) cudaFree(d);
@@ -581,20 +587,8 @@ class BlockCache {
     for (void *x : out) release(x);
   }
 
- private:
-  struct Block {
-    int device;
-    size_t bytes;
-    void *p;
-  };
-  static constexpr size_t kGrain = size_t(1) << 20;  // sizes rounded to 1 MiB, so re-uploads fit exactly
-  static constexpr int kPerDevice = 4;
-
-  cudaError_t alloc(void **p, size_t bytes) { return pinned_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes); }
-  void release(void *p) {
-    if (pinned_) cudaFreeHost(p); else cudaFree(p);
-  }
-  void drop(int device) {
+  // Free this device's idle blocks; false when there were none.
+  bool drop(int device) {
     std::vector<Block> mine;
     {
       std::lock_guard<std::mutex> lk(mu_);
@@ -609,8 +603,22 @@ class BlockCache {
       }
     }
     for (const Block &b : mine) release(b.p);
+    return !mine.empty();
   }
 
+ private:
+  struct Block {
+    int device;
+    size_t bytes;
+    void *p;
+  };
+  static constexpr size_t kGrain = size_t(1) << 20;  // sizes rounded to 1 MiB, so re-uploads fit exactly
+  static constexpr int kPerDevice = 8;     // a graph's arrays and tables are a block each
+
+  cudaError_t alloc(void **p, size_t bytes) { return pinned_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes); }
+  void release(void *p) {
+    if (pinned_) cudaFreeHost(p); else cudaFree(p);
+  }
   std::mutex mu_;
   std::vector<Block> idle_;
   size_t idle_bytes_ = 0;
@@ -626,6 +634,45 @@ BlockCache &device_blocks() {
 BlockCache &pinned_blocks() {
   static BlockCache *c = new BlockCache(true, size_t(256) << 20);
   return *c;
+}
+
+// ---- memory that can be given up ---------------------------------------------
+std::mutex g_tables_mu;
+std::vector<tdfs_graph *> g_with_tables;  // every graph that holds row membership tables
+
+size_t table_bytes(int64_t n, int64_t nedges) { return 4 * kBucket * (size_t)row_table_buckets(n, nedges); }
+
+void forget_tables(tdfs_graph *g) {  // (with g_tables_mu)
+  const auto it = std::find(g_with_tables.begin(), g_with_tables.end(), g);
+  if (it != g_with_tables.end()) g_with_tables.erase(it);
+}
+
+// Device memory is short: free what only makes counts faster -- cached blocks,
+// idle workspaces' level-2 buffers and the row membership tables of graphs
+// that no launch is reading (and of `self`, whose tables_mu the caller holds).
+// True when there was any.
+bool reclaim_memory(int device, tdfs_graph *self) {
+  bool any = device_blocks().drop(device);
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    for (Workspace *w : g_pool)
+      if (w->device == device && w->big) {
+        cudaFree(w->big);
+        w->big = nullptr;
+        any = true;
+      }
+  }
+  std::lock_guard<std::mutex> lk(g_tables_mu);
+  for (tdfs_graph *g : std::vector<tdfs_graph *>(g_with_tables)) {
+    if (g->device != device || (g != self && !g->tables_mu->try_lock())) continue;
+    cudaFree(g->hash);
+    g->hash = nullptr;
+    g->bytes -= table_bytes(g->n, g->nedges);
+    forget_tables(g);
+    if (g != self) g->tables_mu->unlock();
+    any = true;
+  }
+  return any;
 }
 
 int host_threads() {
@@ -721,7 +768,8 @@ void build_label_arrays(int64_t n, int64_t nedges, const int64_t *rowptr, const 
 // 256-byte boundary:
 //   rowptr int64[n+1] | colidx int32[E + kColPad] | src int32[E] | maxnd int32[n]
 //   | label uint8[n] | lperm int32[E] | colidx_l int32[E + kColPad] | loff int32[n (nlab+1)]
-//   | scratch of the label index sort | row membership tables | self-loop flag and check result
+//   | scratch of the label index sort | self-loop flag and check result
+// and the row membership tables in another, which the graph can lose.
 // The device derives everything but the narrowed labels; with more labels than
 // kSegLabels the host sorts the label index into a pinned staging block, laid
 // out the same way, while the copies and kernels queued before it run.  One
@@ -778,24 +826,27 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   const size_t o_hist = o_loff + align256(sizeof(int32_t) * (nloff ? nloff : 1));
   const size_t o_goff = o_hist + align256(sizeof(int32_t) * (size_t)(dev_build && ntiles ? (int64_t)G * ntiles : 1));
   const size_t total = dev_build ? o_goff + align256(sizeof(int64_t) * (size_t)(G + 1)) : o_hist;
-  // the row membership tables, where the flat kernel can use them and the
-  // device has room; without them every plan runs on the DFS kernel
-  const int64_t buckets = row_table_buckets(n, nedges);
-  size_t hash_bytes = buckets <= (int64_t)UINT32_MAX ? 4 * kBucket * (size_t)buckets : 0;
-  void *arrays = nullptr, *stage = nullptr;
-  size_t array_bytes = 0, stage_bytes = 0;
-  e = device_blocks().take(device, total + hash_bytes + 256, &arrays, &array_bytes);
-  if (e == cudaErrorMemoryAllocation && hash_bytes) {
+  void *arrays = nullptr, *stage = nullptr, *hash = nullptr;
+  size_t array_bytes = 0, stage_bytes = 0, hash_bytes = 0;
+  e = device_blocks().take(device, total + 256, &arrays, &array_bytes);
+  if (e == cudaErrorMemoryAllocation) {
     (void)cudaGetLastError();
-    hash_bytes = 0;
-    e = device_blocks().take(device, total + 256, &arrays, &array_bytes);
+    if (reclaim_memory(device, nullptr)) e = device_blocks().take(device, total + 256, &arrays, &array_bytes);
   }
   if (e != cudaSuccess) return checked(cuda_fail(e, "graph arrays"));
+  // the row membership tables, where the flat kernel can use them and the
+  // device has room; without them every plan runs on the DFS kernel
+  if (row_table_buckets(n, nedges) <= (int64_t)UINT32_MAX &&
+      device_blocks().take(device, table_bytes(n, nedges), &hash, &hash_bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    hash = nullptr;
+  }
   if (labels) {
     e = pinned_blocks().take(device, dev_build ? (size_t)std::max<int64_t>(n, 1) : total - o_label, &stage,
                              &stage_bytes);
     if (e != cudaSuccess) {
       device_blocks().give(device, arrays, array_bytes);
+      device_blocks().give(device, hash, hash_bytes);
       return checked(cuda_fail(e, "pinned staging for the label arrays"));
     }
   }
@@ -820,9 +871,10 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   g->colidx_l = nlab ? reinterpret_cast<int32_t *>(base + o_coll) : nullptr;
   g->loff = nlab ? reinterpret_cast<int32_t *>(base + o_loff) : nullptr;
   g->nlab = nlab;
-  g->hash = hash_bytes ? reinterpret_cast<int32_t *>(base + total) : nullptr;
-  g->loops = hash_bytes ? reinterpret_cast<int32_t *>(base + total + hash_bytes) : nullptr;
-  g->bytes = (dev_build ? o_hist : total) + hash_bytes;  // the scratch is not part of the graph
+  g->hash = static_cast<int32_t *>(hash);
+  g->hash_bytes = hash_bytes;
+  g->loops = reinterpret_cast<int32_t *>(base + total);
+  g->bytes = (dev_build ? o_hist : total) + (hash ? table_bytes(n, nedges) : 0);  // the scratch is not part of the graph
   const cudaStream_t st = cudaStreamPerThread;
   e = cudaMemcpyAsync(g->rowptr, rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && nedges)
@@ -833,7 +885,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   if (e == cudaSuccess && check) {
     // nothing below may read rows that break the rules: wait for the verdict
     // (and narrow the labels meanwhile)
-    auto *dck = reinterpret_cast<CsrCheck *>(base + total + hash_bytes + 128);
+    auto *dck = reinterpret_cast<CsrCheck *>(base + total + 128);
     e = cudaMemsetAsync(dck, 0, sizeof *dck, st);
     if (e == cudaSuccess) {
       (void)cudaGetLastError();  // the check below must see this launch's error only
@@ -848,6 +900,7 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     if (e == cudaSuccess && ck.bad) {
       pinned_blocks().give(device, stage, stage_bytes);
       device_blocks().give(device, arrays, array_bytes);
+      device_blocks().give(device, hash, hash_bytes);
       delete g;
       if (const int bad = validate_csr(n, nedges, rowptr, colidx, nullptr)) return bad;
       return fail(TDFS_ERR_FORMAT, "the rows changed while they were read");
@@ -856,7 +909,11 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
   } else if (labels) {
     for (int64_t i = 0; i < n; ++i) lab8[i] = (uint8_t)labels[i];
   }
-  if (g->max_degree > kFlatMaxDegree) g->hash = nullptr;  // the flat kernel's positions would not fit 32 bits
+  if (g->max_degree > kFlatMaxDegree && g->hash) {  // the flat kernel's positions would not fit 32 bits
+    device_blocks().give(device, g->hash, g->hash_bytes);
+    g->hash = nullptr;
+    g->bytes -= table_bytes(n, nedges);
+  }
   Rows R{g->rowptr, g->colidx, (int32_t)n, g->src, g->maxnd, g->hash, g->loops, nullptr, 0, nullptr, nullptr};
   if (e == cudaSuccess && !nlab && run_rows(R, nedges, st) != TDFS_OK) e = cudaErrorUnknown;
   std::unique_ptr<LabelIndex> lindex;
@@ -909,10 +966,16 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
     cudaStreamSynchronize(st);
     pinned_blocks().give(device, stage, stage_bytes);
     device_blocks().give(device, arrays, array_bytes);
+    device_blocks().give(device, g->hash, g->hash_bytes);
     delete g;
     return rc;
   }
   g->lindex = lindex.release();
+  g->tables_mu = new std::mutex;
+  if (g->hash) {
+    std::lock_guard<std::mutex> lk(g_tables_mu);
+    g_with_tables.push_back(g);
+  }
   *out = g;
   return TDFS_OK;
 }
@@ -954,9 +1017,15 @@ void graph_release(tdfs_graph *g) {
   // the blocks go back to the caches, not to the driver: wait for anything
   // still reading them, as cudaFree would
   cudaDeviceSynchronize();
+  {
+    std::lock_guard<std::mutex> lk(g_tables_mu);
+    forget_tables(g);
+  }
   device_blocks().give(g->device, g->arrays, g->array_bytes);
+  device_blocks().give(g->device, g->hash, g->hash_bytes);
   pinned_blocks().give(g->device, g->staging, g->staging_bytes);
   delete g->lindex;
+  delete g->tables_mu;
   cudaSetDevice(cur);
   delete g;
 }

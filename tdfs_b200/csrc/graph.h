@@ -160,7 +160,13 @@ struct tdfs_graph {
   int32_t *colidx_l;      // label-partitioned rows (labeled graphs with <= kSegLabels labels)
   int32_t *loff;          //   and their segment starts per vertex and label
   int32_t nlab;
-  int32_t *hash;          // row membership tables, or nullptr when they did not fit in device memory
+  // The row membership tables, in a block of their own: memory that the graph
+  // can do without (its plans then run on the DFS kernel).  They are given up
+  // for good when a workspace or another graph's arrays find no room
+  // (reclaim_memory); a launch that reads them holds tables_mu meanwhile.
+  int32_t *hash;          // or nullptr
+  size_t hash_bytes;
+  std::mutex *tables_mu;
   int32_t *loops;         // with them: a flag, some row holds its own vertex
   tdfs::LabelIndex *lindex;  // its host copy and group offsets
   size_t array_bytes;     // size of the `arrays` block (cached for reuse when the graph is freed)
@@ -185,7 +191,8 @@ int graph_upload(int64_t n, int64_t nedges, const int64_t *rowptr, const int32_t
                  int device, int32_t max_degree, bool check, tdfs_graph **out);
 void graph_release(tdfs_graph *g);
 // Give g a launch workspace from its device's pool (allocating one when none
-// is idle); the device must be current.  Idempotent.
+// is idle); the device must be current and g's tables_mu held: where memory is
+// short g may lose its tables.  Idempotent.
 int acquire_workspace(tdfs_graph *g);
 void release_graphs(tdfs_graph *g);  // capi.cpp: destroys cached launch graphs
 DevGraph graph_view(const tdfs_graph *g);

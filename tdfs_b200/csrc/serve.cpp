@@ -128,6 +128,7 @@ int open_epoch(Server &S) {
 }
 
 int launch_kernel(Server &S) {
+  std::lock_guard<std::mutex> lk(*S.g->tables_mu);  // (graph_view reads the tables' address)
   init_launch(S.g->ctl, queue_hdr(S.g), S.kstream);
   int rc = launch_match(S.labeled, graph_view(S.g), S.g->ctl, S.g->tab, S.g->queue, queue_hdr(S.g), S.shape.cfg,
                         S.shape.blocks, S.shape.warps_per_block, S.kstream, S.opt.launch.blocks_per_sm > 0);
@@ -319,7 +320,10 @@ int server_create(tdfs_graph *g, const tdfs_server_options *o, Server **out) {
   tdfs_options lo = S->opt.launch;
   int rc = launch_shape(g, S->opt.max_k, S->labeled, lo, &S->shape);
   if (rc) return rc;
-  if ((rc = acquire_workspace(g))) return rc;
+  {
+    std::lock_guard<std::mutex> lk(*g->tables_mu);
+    if ((rc = acquire_workspace(g))) return rc;
+  }
   S->cap = S->shape.cfg.cap;
   if (S->opt.mem_budget == 0)
     S->opt.mem_budget = (size_t)S->opt.max_inflight * query_bytes(S->opt.max_k, S->cap, S->shape.warps_per_block);
