@@ -221,7 +221,7 @@ int64_t ticket_count(int64_t b, int64_t e, int stride, int phase, int chunk) {
 // One launch of either kernel.
 struct Launch {
   bool flat;
-  bool big;         // flat: level 2 of some plan is held in global memory
+  int32_t *big;     // flat: where level 2 of some plan is held in global memory, or nullptr
   LaunchShape dfs;  // !flat
   FlatShape fl;     // flat
   int warps() const { return flat ? fl.blocks * fl.warps_per_block : dfs.blocks * dfs.warps_per_block; }
@@ -265,9 +265,8 @@ std::vector<GraphEntry> &graph_cache(tdfs_graph *g) {
 // The workspace as a launch of the flat kernel uses it: its records where the
 // slot table is, the mailboxes in the split ring's memory.
 static_assert(kFlatBoxBytes <= sizeof(SplitUnit) * kQueueCap, "the mailboxes fit the split ring");
-FlatTable flat_table(const tdfs_graph *g, int n, bool big) {
-  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue),
-                       big ? static_cast<int32_t *>(g->ws->big) : nullptr, g->htab);
+FlatTable flat_table(const tdfs_graph *g, int n, int32_t *big) {
+  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue), big, g->htab);
 }
 
 // Upload, kernel (between the events k0 and k1, when given) and read-back.
@@ -404,6 +403,23 @@ int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms,
   return collect(g, n, L.flat, raw, status);
 }
 
+// The workspace's level-2 buffers for so many warps (43 MB for the grid of the
+// 80-register build, 24 warps on each of 148 SMs), or nullptr when there is no room.
+int32_t *level2_buffers(Workspace *w, int warps) {
+  const size_t need = kBigBytes * (size_t)warps;
+  if (w->big_bytes < need) {
+    cudaFree(w->big);
+    w->big_bytes = 0;
+    if (cudaMalloc(&w->big, need) != cudaSuccess) {
+      (void)cudaGetLastError();
+      w->big = nullptr;
+      return nullptr;
+    }
+    w->big_bytes = need;
+  }
+  return static_cast<int32_t *>(w->big);
+}
+
 // What a launch on g needs first, its device current and a workspace.  It comes
 // before the choice of the kernel: where memory is short g loses its tables.
 int workspace_of(tdfs_graph *g) {
@@ -510,25 +526,30 @@ int run_batch(tdfs_graph *g, const tdfs_plan *const *plans, int n, bool flat, co
     // shared memory and long scans dominate
     constexpr int32_t kSkewDegree = 4096;
     const bool skewed = g->max_degree > kSkewDegree;
-    L.big = false;
-    for (int i = 0; i < n; ++i) L.big |= skewed && plans[i]->flat.reuse2;
-    if (L.big && !g->ws->big && cudaMalloc(&g->ws->big, kBigBytes * kFlatBoxes) != cudaSuccess) {
-      (void)cudaGetLastError();  // no room: level 2 stays in shared memory
-      g->ws->big = nullptr;
-      L.big = false;
-    }
-    int levels = 0, tmax = 1, smax = 1;
+    int smax = 1, tmax = 1;
+    bool reuse = false;
     for (int i = 0; i < n; ++i) {
       const FlatPlan &f = plans[i]->flat;
       smax = std::max(smax, (int)f.s);
-      levels = std::max(levels, f.s - 1 - (L.big && f.reuse2 ? 1 : 0));
       tmax = std::max(tmax, (int)f.t);
+      reuse |= f.reuse2 != 0;
     }
     // counting at the edges of a graph without hubs is light and even: warps
     // that run out of tickets leave instead of waiting to be given work
     // (triangles of the n=4096 ER graph 25.7 -> 23.2 us)
     const bool share = smax > 1 || g->max_degree > kHubDegree;
-    if ((rc = flat_shape(g->device, levels, tmax, skewed, L.big, share, labeled, o, &L.fl))) return rc;
+    auto shape_with = [&](bool big) {
+      int levels = 0;
+      for (int i = 0; i < n; ++i) {
+        const FlatPlan &f = plans[i]->flat;
+        levels = std::max(levels, f.s - 1 - (big && f.reuse2 ? 1 : 0));
+      }
+      return flat_shape(g->device, levels, tmax, skewed, big, share, labeled, o, &L.fl);
+    };
+    const bool big = skewed && reuse;
+    if ((rc = shape_with(big))) return rc;
+    if (big && !(L.big = level2_buffers(g->ws, L.warps())))
+      if ((rc = shape_with(false))) return rc;  // no room: level 2 stays in shared memory
   } else {
     L.dfs = shape;
   }

@@ -659,6 +659,7 @@ bool reclaim_memory(int device, tdfs_graph *self) {
       if (w->device == device && w->big) {
         cudaFree(w->big);
         w->big = nullptr;
+        w->big_bytes = 0;
         any = true;
       }
   }

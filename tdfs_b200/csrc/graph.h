@@ -99,10 +99,10 @@ namespace tdfs {
 
 // Launch workspace: what one persistent launch needs besides the graph --
 // the control block, the split ring, the slot table and its pinned host
-// staging copy.  Tens of MB of device memory (and 100 MB for `big`, on graphs
-// with hubs) and about 10 MB of pinned host memory, so it is pooled per device (graph.cu) instead of being allocated
-// with every graph: a graph takes one at its first launch and hands it back
-// when it is freed.
+// staging copy.  Tens of MB of device memory (and 43 MB for `big`, on graphs
+// with hubs) and about 10 MB of pinned host memory, so it is pooled per device
+// (graph.cu) instead of being allocated with every graph: a graph takes one at
+// its first launch and hands it back when it is freed.
 struct Workspace {
   int device;
   RunCtl *ctl;
@@ -111,7 +111,8 @@ struct Workspace {
   SlotTable *htab;     // pinned
   RunCtl *hctl;        // pinned
   void *gstream;       // cudaStream_t for captured launches (created on first use)
-  void *big;           // the flat kernel's level-2 buffers (allocated on first use)
+  void *big;           // the flat kernel's level-2 buffers (allocated on first use) ...
+  size_t big_bytes;    // ... and their size
   void *ev[2];         // cudaEvent_t around the kernel of plain launches (created on first use)
 };
 

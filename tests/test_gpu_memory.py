@@ -7,7 +7,7 @@ import gc
 import numpy as np
 import pytest
 
-from tests.patterns import TRIANGLE
+from tests.patterns import TRIANGLE, clique
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +86,28 @@ def test_another_graph_finds_room_for_its_arrays(T, full):
     G.close()
     assert T.count(H, P).count == want
     H.close()
+
+
+def test_level_two_buffers_are_as_many_as_the_grid_has_warps(T, full):
+    import torch
+    csr = T.gen_chung_lu(30000, 90000, 2.1, 9000, 1)
+    G = T.GraphPreprocessor(csr=csr)
+    assert G.max_degree > 4096
+    P = T.PatternPreprocessor(text=clique(5))
+    part = dict(edge_end=400)
+
+    def count(**kw):
+        return T.count(G, P, T.default_options(**part, **kw)).count
+
+    want = count(tail_count=1)  # the DFS kernel: the workspace is there, the buffers are not
+    T.count(G, T.PatternPreprocessor(text=TRIANGLE))
+    free = torch.cuda.mem_get_info()[0]
+    assert want > 0 and count(blocks_per_sm=1) == want
+    few = free - torch.cuda.mem_get_info()[0]
+    assert count() == want
+    assert 0 < few < free - torch.cuda.mem_get_info()[0] < 56 * MB
+    # captured launches follow when the buffers grow and move
+    for shape in ({}, {}, {"warps_per_block": 1}, {}, {"warps_per_block": 1}, {"blocks_per_sm": 1}, {}):
+        for _ in range(3):
+            assert count(graph_capture=1, **shape) == want
+    G.close()
