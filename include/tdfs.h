@@ -60,8 +60,9 @@ typedef struct {
   int steal_min;        /* steal only levels with >= steal_min items left (0 auto = 2) */
   int merge_ratio;      /* merge a list whose length <= merge_ratio x the scanned span, else
                            search it (0 auto = 4) */
-  int graph_capture;    /* 1: launch through a cached CUDA graph (upload, reset, kernel,
-                           read-back captured at the second launch of a shape and batch size) */
+  int graph_capture;    /* 1: launch through a cached CUDA graph (upload, reset, kernel and
+                           read-back captured at the first launch of a shape and batch size, and
+                           kept for the next data graph when this one is freed) */
   int edge_chunk;       /* directed edges per level-0 ticket: 1, 2, 4, ..., 32 (0 auto; 32 whenever
                            edge_stride > 1, the chunk the round-robin dealing is defined on) */
   int fixed_stage;      /* last vertex: stage the intersection of its backward neighbours

@@ -228,39 +228,50 @@ struct Launch {
 };
 
 // Captured launches: one CUDA graph per (batch size, mode, launch shape), made
-// at the shape's second launch (exec is null until then),
-// holding the slot-table upload from the pinned staging copy, the control
-// reset, the kernel and the read-back; replays read the staging copy as it is
-// at replay time.
+// at a workspace's first launch of the shape and kept with the workspace.  It
+// holds the upload from the pinned staging copy, read as it is at replay time,
+// and the kernel; for the DFS kernel also the control reset and the read-back
+// (the flat kernel writes its results to the host itself).  All of these are
+// the workspace's own memory.  Of the data graph only the kernel's first
+// argument speaks, and it is exchanged when the workspace has come to another
+// one: capturing, instantiating and destroying a CUDA graph takes 280 us, more
+// than many a count, and a request that opens a data graph, counts and frees
+// it would pay that each time.
 struct GraphEntry {
   int n;
   bool labeled;
   Launch launch;
+  DevGraph view;        // the data graph that the kernel node's arguments name
+  cudaGraph_t graph;
   cudaGraphExec_t exec;
-  cudaEvent_t k0, k1;  // recorded inside the graph around the match kernel
+  cudaGraphNode_t kernel;
+  cudaEvent_t k0, k1;   // recorded inside the graph around the kernel
+  uint64_t used;        // the workspace's captured launches up to this one's last
 };
+constexpr size_t kGraphsKept = 64;  // per workspace; the ones unused for longest make room
+
+void destroy(GraphEntry &c) {
+  if (c.exec) cudaGraphExecDestroy(c.exec);
+  if (c.graph) cudaGraphDestroy(c.graph);
+  if (c.k0) cudaEventDestroy(c.k0);
+  if (c.k1) cudaEventDestroy(c.k1);
+}
 
 }  // namespace
 
-void release_graphs(tdfs_graph *g) {
-  if (!g->graphs) return;
-  auto *v = static_cast<std::vector<GraphEntry> *>(g->graphs);
-  for (auto &c : *v) {
-    if (!c.exec) continue;
-    cudaGraphExecDestroy(c.exec);
-    cudaEventDestroy(c.k0);
-    cudaEventDestroy(c.k1);
-  }
-  delete v;
-  g->graphs = nullptr;
+struct GraphCache {
+  std::vector<GraphEntry> entries;
+  uint64_t launches = 0;
+};
+
+void release_graphs(Workspace *w) {
+  if (!w->graphs) return;
+  for (GraphEntry &c : w->graphs->entries) destroy(c);
+  delete w->graphs;
+  w->graphs = nullptr;
 }
 
 namespace {
-
-std::vector<GraphEntry> &graph_cache(tdfs_graph *g) {
-  if (!g->graphs) g->graphs = new std::vector<GraphEntry>();
-  return *static_cast<std::vector<GraphEntry> *>(g->graphs);
-}
 
 // The workspace as a launch of the flat kernel uses it: its records where the
 // slot table is, the mailboxes in the split ring's memory.
@@ -271,9 +282,10 @@ FlatTable flat_table(const tdfs_graph *g, int n, int32_t *big) {
 
 // Upload, kernel (between the events k0 and k1, when given) and read-back.
 // Captured launches record the events as external ones, so that they time the
-// kernel when the graph replays (a plain record is only a join point).
+// kernel when the graph replays (a plain record is only a join point), and ask
+// for the kernel's node.
 int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStream_t st, cudaEvent_t k0,
-                   cudaEvent_t k1, unsigned flags) {
+                   cudaEvent_t k1, unsigned flags, cudaGraphNode_t *node) {
   SlotTable *h = g->htab, *d = g->tab;
   cudaError_t e;
   if (L.flat) {
@@ -293,6 +305,15 @@ int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStre
              : launch_match(labeled, graph_view(g), g->ctl, g->tab, g->queue, queue_hdr(g), L.dfs.cfg, L.dfs.blocks,
                             L.dfs.warps_per_block, st);
   if (rc) return rc;
+  if (node) {  // what was captured last
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t *last = nullptr;
+    size_t count = 0;
+    e = cudaStreamGetCaptureInfo(st, &status, nullptr, nullptr, &last, &count);
+    if (e != cudaSuccess) return cuda_err(e, "cudaStreamGetCaptureInfo");
+    if (count != 1) return fail(TDFS_ERR_CUDA, "the captured launch is not a chain");
+    *node = last[0];
+  }
   if (k1) e = cudaEventRecordWithFlags(k1, st, flags);
   if (e != cudaSuccess) return cuda_err(e, "kernel end event");
   if (!L.flat) {  // (the flat kernel writes its results to the host image itself)
@@ -345,59 +366,89 @@ int run_plain(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStream_t 
       }
   const cudaEvent_t k0 = ms ? static_cast<cudaEvent_t>(g->ws->ev[0]) : nullptr;
   const cudaEvent_t k1 = ms ? static_cast<cudaEvent_t>(g->ws->ev[1]) : nullptr;
-  if (const int rc = enqueue_launch(g, L, labeled, n, st, k0, k1, cudaEventRecordDefault)) return rc;
+  if (const int rc = enqueue_launch(g, L, labeled, n, st, k0, k1, cudaEventRecordDefault, nullptr)) return rc;
   e = cudaStreamSynchronize(st);
   if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, k0, k1);
   if (e != cudaSuccess) return cuda_err(e, "match kernel");
   return collect(g, n, L.flat, raw, status);
 }
 
+// Capture a launch on g as the entry c (its key set).
+int capture(tdfs_graph *g, cudaStream_t st, GraphEntry &c) {
+  cudaError_t e = cudaEventCreate(&c.k0);
+  if (e == cudaSuccess) e = cudaEventCreate(&c.k1);
+  if (e != cudaSuccess) return cuda_err(e, "cudaEventCreate");
+  e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return cuda_err(e, "cudaStreamBeginCapture");
+  const int rc = enqueue_launch(g, c.launch, c.labeled, c.n, st, c.k0, c.k1, cudaEventRecordExternal, &c.kernel);
+  e = cudaStreamEndCapture(st, &c.graph);
+  if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&c.exec, c.graph, 0);
+  if (rc || e != cudaSuccess) return rc ? rc : cuda_err(e, "capturing the launch");
+  return TDFS_OK;
+}
+
+// Let the entry's kernel read the data graph `view`: the first argument of
+// either kernel, the others staying as captured.
+cudaError_t point_to(GraphEntry &c, const DevGraph &view) {
+  cudaKernelNodeParams p{};
+  cudaError_t e = cudaGraphKernelNodeGetParams(c.kernel, &p);
+  if (e != cudaSuccess) return e;
+  DevGraph v = view;
+  void *args[6] = {&v};  // flat_kernel(G, cfg, T), match_kernel(G, cfg, ctl, tab, units, qh)
+  for (int i = 1; i < (c.launch.flat ? 3 : 6); ++i) args[i] = p.kernelParams[i];
+  p.kernelParams = args;
+  e = cudaGraphExecKernelNodeSetParams(c.exec, c.kernel, &p);
+  if (e == cudaSuccess) c.view = view;
+  return e;
+}
+
 int run_captured(tdfs_graph *g, const Launch &L, bool labeled, int n, float *ms, unsigned long long *raw,
                  int *status) {
   cudaError_t e;
-  if (!g->ws->gstream) {
-    cudaStream_t st;
-    e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e != cudaSuccess) return cuda_err(e, "capture stream");
-    g->ws->gstream = st;
+  Workspace &w = *g->ws;
+  if (!w.gstream) {
+    cudaStream_t s0;
+    e = cudaStreamCreateWithFlags(&s0, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return cuda_err(e, "cudaStreamCreate");
+    w.gstream = s0;
   }
-  cudaStream_t st = static_cast<cudaStream_t>(g->ws->gstream);
-  auto &cache = graph_cache(g);
-  GraphEntry *hit = nullptr;
-  for (auto &c : cache)
-    if (c.n == n && c.labeled == labeled && !std::memcmp(&c.launch, &L, sizeof L))
-      hit = &c;
-  if (!hit) {
-    // a shape's first launch on this graph runs without a capture: capturing,
-    // instantiating and destroying a graph costs 280 us, and a request that
-    // opens a graph, counts once and frees it would pay that for nothing
-    cache.push_back(GraphEntry{n, labeled, L, nullptr, nullptr, nullptr});
-    return run_plain(g, L, labeled, n, st, ms, raw, status);
+  cudaStream_t st = static_cast<cudaStream_t>(w.gstream);
+  if (!w.graphs) w.graphs = new GraphCache;
+  auto &cache = w.graphs->entries;
+  const DevGraph view = graph_view(g);
+  auto hit = std::find_if(cache.begin(), cache.end(), [&](const GraphEntry &c) {
+    return c.n == n && c.labeled == labeled && !std::memcmp(&c.launch, &L, sizeof L);
+  });
+  if (hit != cache.end() && std::memcmp(&hit->view, &view, sizeof view) && point_to(*hit, view) != cudaSuccess) {
+    (void)cudaGetLastError();  // capture it anew
+    destroy(*hit);
+    cache.erase(hit);
+    hit = cache.end();
   }
-  if (!hit->exec) {
-    GraphEntry ent = *hit;
-    e = cudaEventCreate(&ent.k0);
-    if (e == cudaSuccess) e = cudaEventCreate(&ent.k1);
-    if (e != cudaSuccess) return cuda_err(e, "cudaEventCreate");
-    cudaGraph_t graph;
-    e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return cuda_err(e, "cudaStreamBeginCapture");
-    int rc = enqueue_launch(g, L, labeled, n, st, ent.k0, ent.k1, cudaEventRecordExternal);
-    e = cudaStreamEndCapture(st, &graph);
-    if (!rc && e == cudaSuccess) {
-      e = cudaGraphInstantiate(&ent.exec, graph, 0);
-      cudaGraphDestroy(graph);
+  if (hit == cache.end()) {
+    GraphEntry c;
+    std::memset(static_cast<void *>(&c), 0, sizeof c);
+    c.n = n;
+    c.labeled = labeled;
+    std::memcpy(static_cast<void *>(&c.launch), &L, sizeof L);
+    std::memcpy(static_cast<void *>(&c.view), &view, sizeof view);
+    if (const int rc = capture(g, st, c)) {
+      destroy(c);
+      return rc;
     }
-    if (rc || e != cudaSuccess) {
-      cudaEventDestroy(ent.k0);
-      cudaEventDestroy(ent.k1);
-      return rc ? rc : cuda_err(e, "capturing the launch");
+    if (cache.size() >= kGraphsKept) {
+      const auto old = std::min_element(cache.begin(), cache.end(),
+                                        [](const GraphEntry &a, const GraphEntry &b) { return a.used < b.used; });
+      destroy(*old);
+      cache.erase(old);
     }
-    *hit = ent;
+    cache.push_back(c);
+    hit = cache.end() - 1;
   }
+  hit->used = ++w.graphs->launches;
   e = cudaGraphLaunch(hit->exec, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  // the match kernel's own time, from the event nodes around it in the graph
+  // the kernel's own time, from the event nodes around it in the graph
   if (e == cudaSuccess && ms) e = cudaEventElapsedTime(ms, hit->k0, hit->k1);
   if (e != cudaSuccess) return cuda_err(e, "graph launch");
   return collect(g, n, L.flat, raw, status);

@@ -431,6 +431,7 @@ std::vector<Workspace *> g_pool;        // idle workspaces (any device)
 constexpr int kIdlePerDevice = 4;       // idle workspaces kept per device; more are freed
 
 void free_workspace(Workspace *w) {
+  release_graphs(w);
   cudaFree(w->ctl);
   cudaFreeHost(w->htab);
   cudaFree(w->big);
@@ -1013,7 +1014,6 @@ void graph_release(tdfs_graph *g) {
   int cur = 0;
   cudaGetDevice(&cur);
   cudaSetDevice(g->device);
-  release_graphs(g);
   release_workspace(g);
   // the blocks go back to the caches, not to the driver: wait for anything
   // still reading them, as cudaFree would
@@ -1033,6 +1033,7 @@ void graph_release(tdfs_graph *g) {
 
 DevGraph graph_view(const tdfs_graph *g) {
   DevGraph v;
+  std::memset(static_cast<void *>(&v), 0, sizeof v);  // (views are compared as bytes)
   v.rowptr = g->rowptr;
   v.colidx = g->colidx;
   v.src = g->src;

@@ -111,6 +111,7 @@ struct Workspace {
   SlotTable *htab;     // pinned
   RunCtl *hctl;        // pinned
   void *gstream;       // cudaStream_t for captured launches (created on first use)
+  struct GraphCache *graphs;  // and these launches (capi.cpp)
   void *big;           // the flat kernel's level-2 buffers (allocated on first use) ...
   size_t big_bytes;    // ... and their size
   void *ev[2];         // cudaEvent_t around the kernel of plain launches (created on first use)
@@ -179,7 +180,6 @@ struct tdfs_graph {
   tdfs::SlotTable *tab;
   tdfs::SlotTable *htab;
   tdfs::RunCtl *hctl;
-  void *graphs;           // cache of instantiated launch graphs (capi.cpp)
   size_t bytes;
   int64_t last_warps;     // warps in the grid of the last count launch (diagnostics)
 };
@@ -195,7 +195,7 @@ void graph_release(tdfs_graph *g);
 // is idle); the device must be current and g's tables_mu held: where memory is
 // short g may lose its tables.  Idempotent.
 int acquire_workspace(tdfs_graph *g);
-void release_graphs(tdfs_graph *g);  // capi.cpp: destroys cached launch graphs
+void release_graphs(Workspace *w);  // capi.cpp: destroys captured launches
 DevGraph graph_view(const tdfs_graph *g);
 // hash (with loops) may be nullptr: no row membership tables.
 int prepare_graph_arrays(const int64_t *rowptr, const int32_t *colidx, int32_t n, int64_t nedges,
