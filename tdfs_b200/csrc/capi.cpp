@@ -277,7 +277,7 @@ namespace {
 // slot table is, the mailboxes in the split ring's memory.
 static_assert(kFlatBoxBytes <= sizeof(SplitUnit) * kQueueCap, "the mailboxes fit the split ring");
 FlatTable flat_table(const tdfs_graph *g, int n, int32_t *big) {
-  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue), big, g->htab);
+  return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue), big, n <= kHostSlots ? g->htab : nullptr);
 }
 
 // Upload, kernel (between the events k0 and k1, when given) and read-back.
@@ -316,7 +316,9 @@ int enqueue_launch(tdfs_graph *g, const Launch &L, bool labeled, int n, cudaStre
   }
   if (k1) e = cudaEventRecordWithFlags(k1, st, flags);
   if (e != cudaSuccess) return cuda_err(e, "kernel end event");
-  if (!L.flat) {  // (the flat kernel writes its results to the host image itself)
+  if (L.flat && n > kHostSlots) {  // (else the flat kernel writes its results to the host image itself)
+    e = cudaMemcpyAsync(h, d, FlatTable::readback(n), cudaMemcpyDeviceToHost, st);
+  } else if (!L.flat) {
     e = cudaMemcpyAsync(h->hot, d->hot, sizeof(SlotHot) * n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(g->hctl, g->ctl, sizeof(RunCtl), cudaMemcpyDeviceToHost, st);
   }

@@ -46,8 +46,11 @@ int flat_blocks_per_sm(bool labeled, bool wide, bool big, int warps_per_block, s
 // that the host fills and uploads with one copy:
 //   RunCtl | count[n] | FlatCtl | mask of idle warps | FlatInfo[n] | FlatPlan[n]
 // The first two come back with one copy, or, with FlatTable::host set, are
-// written to (pinned) host memory by the last CTA: a copy after the kernel
-// costs a small launch 4 us more.
+// written to (pinned) host memory by one warp of the last CTA.  The copy costs
+// a small launch 2 to 7 us more (a call over 1 slot 33.5 against 29.6 us, 128
+// slots 46.8 against 39.9), the one warp costs a large one more: 512 slots 90 us
+// either way, 1024 slots 141 against 127 with the copy, 16384 1.86 against 1.60 ms.
+constexpr int kHostSlots = 512;
 constexpr int kFlatBoxes = 8192;  // mailboxes, one per warp of the grid
 constexpr int kIdleWords = kFlatBoxes / 32;
 

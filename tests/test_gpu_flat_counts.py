@@ -1,7 +1,12 @@
-"""Counts of the flat kernel's closed forms far from the small graphs of the other
-tests: modulo 2^64, as the reference's unsigned 64-bit counters."""
+"""Counts of the flat kernel far from the small launches of the other tests: closed
+forms modulo 2^64, as the reference's unsigned 64-bit counters, and batches
+whose results are copied back instead of written by the kernel."""
+import random
+
 import numpy as np
 import pytest
+
+from tests.golden.make_golden import random_pattern
 
 pytestmark = pytest.mark.gpu
 
@@ -20,3 +25,16 @@ def test_triples_of_a_large_set(T, pages):
     P = T.PatternPreprocessor(text=BOOK)
     assert P.dump()["flat"]["t"] == 3 and P.dump()["flat"]["form"] == 1
     assert T.count(G, P).count == 12 * (pages * (pages - 1) * (pages - 2) // 6) % 2 ** 64
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 1500, 16384])
+def test_results_of_large_batches(T, n):
+    """Up to 512 slots the kernel writes the counts to the host, beyond they are copied."""
+    G = T.GraphPreprocessor(csr=T.gen_er(1000, 10.0, 0).set_labels(5, 2), labeled=True)
+    rng = random.Random(n)
+    base = [T.PatternPreprocessor(text=random_pattern(3 + i % 3, 0.5, 5, rng), labeled=True) for i in range(101)]
+    want = [T.count(G, p).count for p in base]
+    plans = [base[i % 101] for i in range(n)]
+    for opt in ({}, {"graph_capture": 1}, {"graph_capture": 1}):
+        assert T.count_batch(G, plans, T.default_options(**opt))[0] == [want[i % 101] for i in range(n)]
+        assert T.last_launch(G)["mean_warp_ms"] > 0
