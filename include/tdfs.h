@@ -70,7 +70,9 @@ typedef struct {
                            (0 auto = on, -1 off) */
   int split_after_us;   /* DFS kernel: a warp's subtree becomes stealable after this many microseconds
                            on it, donatable to the HBM ring after 4x (0 auto = 150, -1 = at once);
-                           flat kernel: a warp gives work to idle ones after this long (0 auto = 60) */
+                           flat kernel: a warp gives work to idle ones after this long on it
+                           (0 auto = 60, or 20 where a graph with vertices of more than 512
+                           neighbours has few level-0 edges per warp; -1 = at once) */
   int steal_first;      /* an idle warp first takes a level with >= steal_first items from a warp
                            of its CTA, then a unit of the split ring, and only then a level
                            with >= steal_min items (0 auto = 8) */

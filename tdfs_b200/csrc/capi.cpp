@@ -519,7 +519,7 @@ void fill_flat(tdfs_graph *g, const tdfs_plan *const *plans, int n, const tdfs_o
     edges += in.e_end - in.e_begin;
   }
   const bool hubs = g->max_degree > kHubDegree;
-  if (hubs && edges < (int64_t)kFewEdges * L.warps()) {
+  if (hubs && edges / stride < (int64_t)kFewEdges * L.warps()) {
     if (o.split_after_us == 0) L.fl.cfg.split_ns = kFewSplitNs;
     L.fl.cfg.check = kFewCheckCycles;
   }

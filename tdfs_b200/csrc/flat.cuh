@@ -151,20 +151,26 @@ struct FlatTable {
 inline int flat_max_blocks(int warps_per_block) { return kFlatBoxes / warps_per_block; }
 static_assert((unsigned long long)kFlatBoxes < 1ull << (64 - kJoinShift), "a join count for every CTA");
 
-// Level-0 edges per ticket of a slot whose plan is enumerated down to level s,
-// in a launch of `edges` level-0 edges over all slots; skewed: on a graph with
-// hubs (kHubDegree); `edge_chunk` and `stride` as in tdfs_options.
+// Hubs: vertices with more neighbours than this.
 constexpr int32_t kHubDegree = 512;
 
 // How old a warp's base work must be before it gives some away, and the clocks
 // between its looks for idle warps.  Giving work away early costs more than it
 // gains where every warp has much of it, or the work is even (64-query ER burst
-// 0.154 ms at 60 us and 16384 clocks, 0.166 at 20 us and 4096; 7 power-law
-// queries 2.83 against 2.91).  A launch of fewer than kFewEdges level-0 edges
-// per warp on a graph with hubs is over when its few heavy edges are: they are
-// to be spread soon (4 labeled power-law queries 0.464 -> 0.373 ms).
+// 0.154 ms at 60 us and 16384 clocks, 0.166 at 20 us and 4096, in a build of
+// then).  A launch with fewer than kFewEdges level-0 edges per warp in its share
+// of the range, on a graph with hubs, is over when its few heavy edges are: they
+// are to be spread soon.  Early against late over 216 batches of labeled random
+// queries, shares of them and unlabeled cliques on two power-law graphs, as
+// geometric means: 0.94 of the time below 8 edges per warp (0.87 to 1.03 by kind
+// and range), 0.97 from 8 to 16, 0.99 from 16 to 24; beyond, labeled batches take
+// 1.05 times as long, one of them 2.6.
 constexpr int kSplitNs = 60000, kCheckCycles = 16384;
 constexpr int kFewEdges = 16, kFewSplitNs = 20000, kFewCheckCycles = 4096;
+
+// Level-0 edges per ticket of a slot whose plan is enumerated down to level s,
+// in a launch of `edges` level-0 edges over all slots; skewed: on a graph with
+// hubs; `edge_chunk` and `stride` as in tdfs_options.
 int flat_chunk(int64_t edges, int s, bool skewed, int stride, int warps, int edge_chunk);
 
 // Launch over the slots of `t` (on the device).

@@ -28,11 +28,10 @@ void level0_range(const tdfs_graph *g, const DevPlan &p, int64_t eb, int64_t ee,
 const DevPlan &plan_device_table(const tdfs_plan *p);
 const FlatPlan *plan_flat_table(const tdfs_plan *p);
 
-// Launch shape of the flat kernel for plans enumerated down to level smax
-// (FlatPlan::s) with tails of up to tmax vertices, holding `levels` levels in
-// shared memory (big: and level 2 in global memory), on a skewed graph or not,
-// idle warps waiting to be given work (share) or leaving, from the options
-// launch_shape has accepted (capi.cpp).
+// Launch shape of the flat kernel for plans with tails of up to tmax vertices,
+// holding `levels` levels in shared memory (big: and level 2 of some plan in
+// global memory), on a skewed graph or not, idle warps waiting to be given work
+// (share) or leaving, from the options launch_shape has accepted (capi.cpp).
 struct FlatShape {
   int warps_per_block;
   int blocks;
