@@ -876,20 +876,22 @@ struct Flat {
   // that when p was read every CTA started until then was idle.  A warp asks
   // once it has seen the last ticket go, and the atomic that takes a CTA's
   // tickets also counts it, so whoever took one is among them.  Once the whole
-  // grid has started, p alone tells.
-  __device__ __forceinline__ bool complete(int p) const {
+  // grid has started, p alone tells.  (Out of line: the code of labeled launches
+  // is at the limit of the instruction cache; inlined in its three places it
+  // cost a batch of 4 power-law queries 7 %, 0.645 to 0.692 ms, here 1.7 %.)
+  __device__ __noinline__ static bool complete(int p, const FlatCtl *ctl, FlatCta &C) {
     const int grid = (int)gridDim.x;
     if (p == -grid) return true;
     if (*(volatile int32_t *)&C.all) return false;
     __threadfence();
-    const int started = (int)(*(volatile unsigned long long *)&T.ctl->ticket >> kJoinShift);
+    const int started = (int)(*(const volatile unsigned long long *)&ctl->ticket >> kJoinShift);
     if (started == grid) *(volatile int32_t *)&C.all = 1;
     return p + started == 0;
   }
   // A warp has run dry (lane 0).  True when it was its CTA's last busy one and
   // nothing is left anywhere.
   __device__ __forceinline__ bool cta_idle() const {
-    return atomicSub(&C.active, 1) == 1 && complete(atomicSub(&T.ctl->pending, 1) - 1);
+    return atomicSub(&C.active, 1) == 1 && complete(atomicSub(&T.ctl->pending, 1) - 1, T.ctl, C);
   }
 
   // Wait until this warp is given work (returns its level, installed) or none
@@ -922,7 +924,7 @@ struct Flat {
         if (*(volatile int32_t *)&T.box[gid].full) st = 1;
         else if (*(volatile int32_t *)&C.done) st = 2;
         else if (poller || (poller = atomicCAS(&C.poll, 0, 1) == 0)) {
-          if (complete(*(volatile int32_t *)&T.ctl->pending)) {
+          if (complete(*(volatile int32_t *)&T.ctl->pending, T.ctl, C)) {
             *(volatile int32_t *)&C.done = 1;
             st = 2;
           }
