@@ -276,6 +276,7 @@ namespace {
 // The workspace as a launch of the flat kernel uses it: its records where the
 // slot table is, the mailboxes in the split ring's memory.
 static_assert(kFlatBoxBytes <= sizeof(SplitUnit) * kQueueCap, "the mailboxes fit the split ring");
+static_assert(FlatTable::bytes(kMaxSlots) <= sizeof(SlotTable), "the records fit the slot table");
 FlatTable flat_table(const tdfs_graph *g, int n, int32_t *big) {
   return FlatTable::of(g->tab, n, reinterpret_cast<FlatBox *>(g->queue), big, n <= kHostSlots ? g->htab : nullptr);
 }
