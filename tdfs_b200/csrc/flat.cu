@@ -1024,7 +1024,7 @@ struct Flat {
 // 80 for 3, whose scan step has more loads in flight: on skewed graphs, where
 // long scans dominate, it is the faster one (R-MAT 4-clique share 17.0 against
 // 19.0 ms, house slice 38.5 against 40.4), on small uniform graphs the warps
-// count (64-query burst 0.243 against 0.219 ms).
+// count (64-query burst 1.11 times as long with 80).
 template <bool LAB, int MINB, bool BIG>
 __global__ void __launch_bounds__(256, MINB) flat_kernel(const __grid_constant__ DevGraph G,
                                                       const __grid_constant__ FlatCfg cfg,
@@ -1114,8 +1114,8 @@ int flat_chunk(int64_t edges, int s, bool skewed, int stride, int warps, int edg
   // Full lanes at the first levels against even shares.  A plan counted at its
   // edges has little work per edge and wants all 32 lanes (triangles of the
   // n=4096 ER graph: 87 us with 1 edge per ticket, 39 with 4, 25 with 32); each
-  // level more multiplies an edge's work (64-query burst, s up to 4: 0.50 ms
-  // with 1, 0.17 with 4, 0.17 with 8).  Where hubs make some edges thousands of
+  // level more multiplies an edge's work (64-query burst, s up to 4: 2.9 times as
+  // long with 1 as with 4 or 8).  Where hubs make some edges thousands of
   // times heavier than others, consecutive ones (a hub's) go to different
   // warps: power-law labeled batch 2.6 ms with 1, 3.0 with 4; triangles 0.16
   // with 4, 0.22 with 32.

@@ -157,8 +157,7 @@ constexpr int32_t kHubDegree = 512;
 // How old a warp's base work must be before it gives some away, and the clocks
 // between its looks for idle warps.  Giving work away early costs more than it
 // gains where every warp has much of it, or the work is even (64-query ER burst
-// 0.154 ms at 60 us and 16384 clocks, 0.166 at 20 us and 4096, in a build of
-// then).  A launch with fewer than kFewEdges level-0 edges per warp in its share
+// 1.08 times as long at 20 us and 4096 clocks).  A launch with fewer than kFewEdges level-0 edges per warp in its share
 // of the range, on a graph with hubs, is over when its few heavy edges are: they
 // are to be spread soon.  Early against late over 216 batches of labeled random
 // queries, shares of them and unlabeled cliques on two power-law graphs, as
