@@ -157,13 +157,13 @@ constexpr int32_t kHubDegree = 512;
 // How old a warp's base work must be before it gives some away, and the clocks
 // between its looks for idle warps.  Giving work away early costs more than it
 // gains where every warp has much of it, or the work is even (64-query ER burst
-// 1.08 times as long at 20 us and 4096 clocks).  A launch with fewer than kFewEdges level-0 edges per warp in its share
-// of the range, on a graph with hubs, is over when its few heavy edges are: they
-// are to be spread soon.  Early against late over 216 batches of labeled random
-// queries, shares of them and unlabeled cliques on two power-law graphs, as
-// geometric means: 0.94 of the time below 8 edges per warp (0.87 to 1.03 by kind
-// and range), 0.97 from 8 to 16, 0.99 from 16 to 24; beyond, labeled batches take
-// 1.05 times as long, one of them 2.6.
+// 1.08 times as long at 20 us and 4096 clocks).  A launch with fewer than
+// kFewEdges level-0 edges per warp in its share of the range, on a graph with
+// hubs, is over when its few heavy edges are: they are to be spread soon.  Early
+// against late over 216 batches of labeled random queries, shares of them and
+// unlabeled cliques on two power-law graphs, as geometric means: 0.94 of the time
+// below 8 edges per warp (0.87 to 1.03 by kind and range), 0.97 from 8 to 16, 0.99
+// from 16 to 24; beyond, labeled batches take 1.05 times as long, one of them 2.6.
 constexpr int kSplitNs = 60000, kCheckCycles = 16384;
 constexpr int kFewEdges = 16, kFewSplitNs = 20000, kFewCheckCycles = 4096;
 

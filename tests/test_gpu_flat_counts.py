@@ -38,3 +38,20 @@ def test_results_of_large_batches(T, n):
     for opt in ({}, {"graph_capture": 1}, {"graph_capture": 1}):
         assert T.count_batch(G, plans, T.default_options(**opt))[0] == [want[i % 101] for i in range(n)]
         assert T.last_launch(G)["mean_warp_ms"] > 0
+
+
+@pytest.mark.parametrize("warps", range(1, 9))
+@pytest.mark.parametrize("cap", [64, 1024, 4096, 8192])
+def test_the_deepest_buffers_that_are_accepted(T, warps, cap):
+    """A depth that one kernel accepts the other accepts: buffers up to all of an SM's shared memory."""
+    G = T.GraphPreprocessor(csr=T.gen_er(1000, 20.0, 0))
+    for text in (BOOK, "".join(f"v {i} 1\n" for i in range(4)) + "e 0 1 1\ne 0 2 1\ne 1 2 1\ne 0 3 1\ne 1 3 1\ne 2 3 1\n"):
+        P = T.PatternPreprocessor(text=text)
+        want = T.count(G, P).count
+        got = []
+        for kernel in ({}, {"tail_count": 1}):
+            try:
+                got.append(T.count(G, P, T.default_options(warps_per_block=warps, chunk_cap=cap, **kernel)).count)
+            except T.TdfsError as e:
+                got.append(e.code)
+        assert got in ([want, want], [5, 5]), (warps, cap)  # 5: TDFS_ERR_CAPACITY
